@@ -438,7 +438,6 @@ int fg_create(int width, int height, float density, float h, const fg_params* pa
   // the caller's current context or create the device's primary one.
   if (cudaFree(nullptr) != cudaSuccess) return bail(FG_ERR_CUDA);
   init_jacobi_tma();
-  init_lexsor_cluster();
   if (cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(FG_ERR_CUDA);
   for (int k = 0; k < 2; ++k) {
@@ -537,9 +536,7 @@ int fg_destroy(fg_fluid* f) {
   cudaFree(f->ectl);
   cudaFree(f->tile_done);
   if (f->image_pinned) cudaFreeHost(f->image_pinned);
-  for (float* q : f->skew) cudaFree(q);
-  cudaFree(f->skew_flags);
-  cudaFree(f->lex_scratch);
+  cudaFree(f->wave);
   for (int k = 0; k < 2; ++k) {
     cudaFreeHost(f->edit_pinned[k]);  // edit_dev / edit_off_dev map these
     cudaFreeHost(f->edit_off_pinned[k]);
@@ -670,34 +667,22 @@ int fg_synchronize(fg_fluid* f) {
 
 void* fg_stream(fg_fluid* f) { return f ? (void*)f->stream : nullptr; }
 
-// The diagonal-major copies of the wavefront SOR (LEXSOR and the multigrid
-// smoothers), allocated before the first step that uses them (outside any
-// capture); without them the row-major kernel runs.
-void ensure_skew(fg_fluid* f) {
-  if (f->skew[0] || f->batch || !(f->prm.scheme == FG_SCHEME_LEXSOR || multigrid(f))) return;
-  const int sp = (f->NX + 31) / 32 * 32;
-  const size_t n = (size_t)(f->NX + f->NY - 1) * sp;
-  // The wavefront kernels index the copies with 32-bit integers: a grid much
-  // wider than tall whose copies exceed that keeps the row-major kernel.
-  if (n > (size_t)INT_MAX) return;
-  float* a[3] = {};
-  uint8_t* fl = nullptr;
-  bool ok = true;
-  for (auto& q : a) ok = ok && dev_malloc((void**)&q, n * sizeof(float)) == cudaSuccess;
-  ok = ok && dev_malloc((void**)&fl, n) == cudaSuccess;
-  unsigned* lex = nullptr;
-  ok = ok && dev_malloc((void**)&lex, sizeof(unsigned) * lexsor_scratch_words()) == cudaSuccess;
-  if (!ok) {
-    for (auto& q : a) cudaFree(q);
-    cudaFree(fl);
-    cudaFree(lex);
+// The buffers of the serial schemes' pipeline (LEXSOR and UseMultigrid),
+// allocated before the first step that uses them (outside any capture);
+// without them the one-block wavefront runs.
+void ensure_wave(fg_fluid* f) {
+  if (f->wave || f->batch || !(f->prm.scheme == FG_SCHEME_LEXSOR || multigrid(f))) return;
+  if (dev_malloc(&f->wave, wave_bytes(f)) != cudaSuccess) {
+    f->wave = nullptr;
     cudaGetLastError();
     return;
   }
-  f->lex_scratch = lex;
-  for (int k = 0; k < 3; ++k) f->skew[k] = a[k];
-  f->skew_flags = fl;
-  f->skew_sp = sp;
+  if (wave_init(f) != cudaSuccess) {
+    cudaFree(f->wave);
+    f->wave = nullptr;
+    cudaGetLastError();
+    return;
+  }
   f->params_version++;  // captured steps run the other kernel sequence
 }
 
@@ -789,7 +774,7 @@ static int simulate_enqueue(fg_fluid* f, float dt) {
   int rc = flush(f);
   if (rc) return rc;
   f->step_mid = f->async_deferred;
-  ensure_skew(f);
+  ensure_wave(f);
   if ((rc = check_iters(f, f->prm.num_iters))) return rc;
   if ((rc = mg_prepare(f))) return rc;
   invalidate(f, kStepFields);
@@ -894,7 +879,7 @@ int fg_get_stats(fg_fluid* f, fg_stats* out) {
 int fg_make_incompressible(fg_fluid* f, int num_iters, float dt) {
   if (is_batch(f)) return batch_unsupported(f);
   STAGE_PROLOGUE(f);
-  ensure_skew(f);
+  ensure_wave(f);
   if ((rc = check_iters(f, num_iters))) return rc;
   if ((rc = mg_prepare(f))) return rc;
   invalidate(f, kStepFields);

@@ -338,10 +338,11 @@ struct fg_fluid {
   int* tile_done = nullptr;  // dataflow Jacobi kernel: per-tile phase flags + item counter
   int stall_tile = -1;       // fault injection: a tile the dataflow kernel never publishes
   int jacobi_kernel = 0;     // FG_JACOBI_KERNEL_* of the last main solve (fg_stats)
-  float* skew[3] = {};       // diagonal-major U, V, p of the wavefront SOR (or none)
-  uint8_t* skew_flags = nullptr;
-  int skew_sp = 0;           // their row stride (cells per diagonal)
-  unsigned* lex_scratch = nullptr;  // grid-wide wavefront: sweep maxima, barrier words
+  // The serial schemes' pipeline (k_lexsor.cu): control words, packets and
+  // the speculative pass's fields in one block (or none), and the blocks the
+  // device holds at once.
+  void* wave = nullptr;
+  int wave_blocks = 0;
   void* ectl = nullptr;   // control block of the FP64-residual correction solve
   int n_slots = 0;        // launch slots per control block
   float* copy_tmp = nullptr;        // fg_copy_border staging (2 fields)
@@ -468,14 +469,9 @@ cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb
 cudaError_t launch_mg_rebuild(fg_fluid* f);
 cudaError_t mg_kernel_setup();  // the bottom kernel's shared-memory limit (outside capture)
 void mg_free(fg_fluid* f);
-// solveMultigridVCycle (fluid.go:559-594) with the reference's serial
-// smoothers, bit for bit.
-cudaError_t launch_multigrid(fg_fluid* f, int num_iters, float dt);
 // K Jacobi sweeps of A x = b from x = 0 (no early exit); ctl->sel names the
 // buffer holding x.
 void init_jacobi_tma();
-void init_lexsor_cluster();
-int lexsor_scratch_words();
 int jacobi_tile_count(int NX, int NY);
 cudaError_t launch_jacobi_solve(fg_fluid* f, void* ctl, const float* b, const float* bw, float* x0,
                                 float* x1, int iters);
@@ -483,6 +479,16 @@ cudaError_t launch_jacobi_solve(fg_fluid* f, void* ctl, const float* b, const fl
 cudaError_t launch_store_phi(fg_fluid* f, float* dst);
 // Gradient subtract with a stored potential (a recorded step's replay).
 cudaError_t launch_grad_replay(fg_fluid* f, float dt, const float* phi, bool fuse_turb);
+// k_lexsor.cu
+// solveSingleGrid (fluid.go:157-234): the reference's serial SOR, bit for bit.
+cudaError_t launch_lexsor(fg_fluid* f, int num_iters, float dt);
+// solveMultigridVCycle (fluid.go:559-594) with the reference's serial
+// smoothers, bit for bit.
+cudaError_t launch_multigrid(fg_fluid* f, int num_iters, float dt);
+// The buffers both run in: their size, and the set-up of a fresh block
+// (f->wave; outside capture).
+size_t wave_bytes(const fg_fluid* f);
+cudaError_t wave_init(fg_fluid* f);
 // k_adjoint.cu
 constexpr int kTapeFields = 13;  // U2 V2 U4 V4 fwdU fwdV corrU corrV U5 V5 M1 fwdM corrM
 cudaError_t launch_add_forces(fg_fluid* f, const float* fu, const float* fv);

@@ -1,19 +1,6 @@
 // Pressure projection (pkg/fluid/fluid.go:144-234).
 //
-// Two schemes:
-//  * LEXSOR reproduces solveSingleGrid / pressureJacobiIteration exactly: the
-//    serial lexicographic SOR sweep in velocity form with the relaxation
-//    schedule 1.9 -> 1.2 and the early exit on max|div| < tolerance.  Cell
-//    (i, j) of a sweep depends on (i-1, j) and (i, j-1) of the same sweep and
-//    on (i+1, j), (i, j+1) of the previous one, so the sweep runs as a
-//    wavefront over anti-diagonals, with consecutive sweeps pipelined two
-//    diagonals apart.  Every face sees the same sequence of floating-point
-//    updates as in the serial loop, so the result is bit-identical.  The
-//    wavefront runs on one block (k_lexsor) or an 8-block cluster
-//    (k_lexsor_cl), on diagonal-major copies of the fields; the early exit
-//    either waits, step by step, for the previous sweep to be known not to
-//    exit, or runs speculatively (all sweeps, then an exact re-run of the
-//    sweeps the serial loop makes when one falls below the tolerance).
+// The parallel schemes (the reference's serial ones: k_lexsor.cu):
 //  * JACOBI relaxes the same masked Poisson system for the cell potential
 //    phi (the accumulated per-cell correction of the SOR loop):
 //        s_c phi_c - sum_n phi_n = -div_c,   phi = 0 off the active cells,
@@ -67,883 +54,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 constexpr int BX = 32, BY = 8;
 inline dim3 cell_grid(const fg_fluid* f) {
   return dim3((f->NY + BX - 1) / BX, (f->NX + BY - 1) / BY);
-}
-
-// q / n and q % n for 0 <= q < 2^24, n > 0, from a float reciprocal and one
-// correction step (exact: q and the candidate products are exact in float
-// range, and the float quotient is off by at most one).
-__device__ __forceinline__ int div_small(int q, int n, float inv_n, int& rem) {
-  int t = __float2int_rz((float)q * inv_n);
-  int r = q - t * n;
-  if (r < 0) {
-    --t;
-    r += n;
-  } else if (r >= n) {
-    ++t;
-    r -= n;
-  }
-  rem = r;
-  return t;
-}
-
-// ------------------------------------------------------------------ LEXSOR
-constexpr int LEX_THREADS = 1024;
-constexpr int LEX_RING = 4096;  // sweeps in flight (a new sweep waits while the ring is full)
-constexpr int LEX_CHUNK = 4;    // cells whose loads a thread issues together
-
-__global__ void __launch_bounds__(LEX_THREADS)
-    k_lexsor(float* U, float* V, float* p, const uint8_t* __restrict__ flags, Grid g,
-             int numIters, float relax0, float damping, float cp, float tol, int early_exit,
-             DevStats* st, float minRelax = 1.2f, const int* __restrict__ stop = nullptr,
-             int SP = 0, int* __restrict__ exit_out = nullptr,
-             const int* __restrict__ run_from = nullptr) {
-  __shared__ int s_start[LEX_RING];
-  __shared__ unsigned s_max[LEX_RING];
-  __shared__ uint8_t s_cont[LEX_RING];
-  __shared__ int s_lo, s_hi, s_done, s_exit, s_last;
-  const int P = g.P;
-  const int ni = g.NX - 2, nj = g.NY - 2;  // interior extent
-  const int D = ni + nj - 1;               // anti-diagonals d = i + j in [2, NX+NY-4]
-  // Row-major fields (SP = 0): cell (i, j) at i * P + j, its east face +P,
-  // its north face +1.  Diagonal-major copies (SP > 0): cell (i, j) at
-  // (i + j) * SP + i, east +SP+1, north +SP, so a step's accesses are
-  // contiguous along the diagonal.
-  const int offE = SP ? SP + 1 : P, offN = SP ? SP : 1;
-  const int L = ni < nj ? ni : nj;         // longest diagonal
-  if (threadIdx.x == 0) {
-    s_lo = 0;
-    s_hi = 0;
-    s_done = 0;
-    s_exit = 0;
-    s_last = -1;
-  }
-  __syncthreads();
-  if (numIters <= 0 || ni <= 0 || nj <= 0) return;
-  if (stop && *stop) return;  // a multigrid solve that already converged
-  // The cells of the W sweeps lo .. lo+W-1 that step tau reaches; sweep t is
-  // on diagonal 2 + delta_of(t) (out of range: not running) and its max
-  // |div| goes to s_max[r] (r = t mod LEX_RING).
-  auto step = [&](long long tau, int lo, int W, auto delta_of, int runIters, bool all) {
-      // Each warp takes 32 cells of one sweep's diagonal (the diagonal length
-      // padded to a multiple of 32), so the sweep's max |div| and its
-      // "cannot exit" mark are reduced in the warp and stored once per warp.
-      // The cells a step updates share no face or pressure value (cells of one
-      // diagonal are not neighbours; sweeps in flight are two diagonals
-      // apart), so a thread loads the inputs of LEX_CHUNK cells at once and
-      // then updates them: one memory round trip per chunk instead of one per
-      // cell.
-      const int Lp = (L + 31) & ~31;
-      const float invLp = 1.0f / (float)Lp;
-      const int items = W * Lp;
-      for (int base = 0; base < items; base += LEX_CHUNK * LEX_THREADS) {
-        int cc[LEX_CHUNK], rr[LEX_CHUNK], tt[LEX_CHUNK];
-        bool act[LEX_CHUNK] = {};
-        uint8_t fl[LEX_CHUNK];
-        float u0[LEX_CHUNK], u1[LEX_CHUNK], v0[LEX_CHUNK], v1[LEX_CHUNK], p0[LEX_CHUNK];
-#pragma unroll
-        for (int m = 0; m < LEX_CHUNK; ++m) {
-          if (base + m * LEX_THREADS >= items) break;  // (block-uniform)
-          const int q = base + m * LEX_THREADS + (int)threadIdx.x;
-          int k;
-          const int t = lo + (items < (1 << 24) ? div_small(q, Lp, invLp, k) : (k = q % Lp, q / Lp));
-          const int r = t & (LEX_RING - 1);
-          const int delta = q < items ? delta_of(t) : -1;
-          const int d = 2 + delta;
-          const int i_lo = max(1, d - nj), i_hi = min(ni, d - 1);
-          const int i = i_lo + k;
-          const bool in = delta >= 0 && delta < D && k < L && i <= i_hi;
-          const int c = in ? (SP ? d * SP + i : i * P + (d - i)) : 0;
-          cc[m] = c;
-          rr[m] = r;
-          tt[m] = t;
-          act[m] = in;
-          fl[m] = in ? flags[c] : 0;
-          u0[m] = in ? U[c] : 0.0f;
-          u1[m] = in ? U[c + offE] : 0.0f;
-          v0[m] = in ? V[c] : 0.0f;
-          v1[m] = in ? V[c + offN] : 0.0f;
-          p0[m] = in ? p[c] : 0.0f;
-        }
-#pragma unroll
-        for (int m = 0; m < LEX_CHUNK; ++m) {
-          if (base + m * LEX_THREADS >= items) break;  // (whole warps: items is a multiple of 32)
-          const uint8_t f = fl[m];
-          bool a = act[m] && (f & F_FLUID);
-          const float sx0 = fbit(f, F_W), sx1 = fbit(f, F_E), sy0 = fbit(f, F_S),
-                      sy1 = fbit(f, F_N);
-          const float s = sx0 + sx1 + sy0 + sy1;
-          a = a && s != 0.0f;
-          const float div = a ? u1[m] - u0[m] + v1[m] - v0[m] : 0.0f;
-          const float absDiv = fabsf(div);
-          const bool counted = a && !isnan(absDiv);
-          const unsigned mx = __reduce_max_sync(0xffffffffu, counted ? __float_as_uint(absDiv) : 0u);
-          const bool cont = __any_sync(0xffffffffu, counted && absDiv >= tol);
-          // (Without the early exit only the last sweep's max is reported,
-          // and more sweeps than ring slots may be in flight.)
-          if ((threadIdx.x & 31) == 0 && (early_exit || all || tt[m] == runIters - 1)) {
-            if (mx) atomicMax(&s_max[rr[m]], mx);
-            if (cont) s_cont[rr[m]] = 1;
-          }
-          if (!a) continue;
-          const int c = cc[m];
-          // Relaxation of sweep t (fluid.go:169-170).
-          float iterProgress = (float)tt[m] / (float)numIters;
-          float rel = relax0 - (relax0 - minRelax) * iterProgress;
-          float pp = -div / s;
-          pp *= rel;
-          pp *= damping;
-          p[c] = p0[m] + cp * pp;
-          U[c] = u0[m] - sx0 * pp;
-          U[c + offE] = u1[m] + sx1 * pp;
-          V[c] = v0[m] - sy0 * pp;
-          V[c + offN] = v1[m] + sy1 * pp;
-        }
-      }
-  };
-  if (!early_exit) {
-    // Without the early exit sweep t always starts at step 2t (two steps
-    // after the previous one, as the bookkeeping below would start it):
-    // sweep t covers steps 2t .. 2t + D - 1 and the steps need no
-    // bookkeeping between them, one barrier each.  With exit_out (the
-    // speculative pass of an early-exit solve) every sweep's max |div| is
-    // kept until the sweep retires and the first sweep below the tolerance
-    // is recorded; with run_from (the re-run) only sweeps 0 .. *run_from run,
-    // and nothing at all when no sweep was below it.
-    int runIters = numIters;
-    if (run_from) {
-      const int e = *run_from;
-      if (e < 0 || e >= numIters) return;
-      runIters = e + 1;
-    }
-    for (int r = threadIdx.x; r < LEX_RING; r += LEX_THREADS) s_max[r] = 0u;
-    __shared__ unsigned s_lastmax;
-    if (threadIdx.x == 0) s_lastmax = 0u;
-    __syncthreads();
-    const long long steps = (long long)D + 2LL * (runIters - 1);
-    for (long long tau = 0; tau < steps; ++tau) {
-      int t_lo = (int)((tau - D + 2) / 2);
-      if (t_lo < 0) t_lo = 0;
-      while (tau - 2LL * t_lo >= D) ++t_lo;
-      int t_hi = (int)(tau / 2);
-      if (t_hi > runIters - 1) t_hi = runIters - 1;
-      step(tau, t_lo, t_hi - t_lo + 1, [&](int t) { return (int)(tau - 2LL * t); }, runIters,
-           exit_out != nullptr);
-      __syncthreads();
-      // The sweep whose last diagonal ran in this step retires.
-      const long long rt = tau - (D - 1);
-      if (threadIdx.x == 0 && rt >= 0 && (rt & 1) == 0 && rt / 2 < runIters) {
-        const int t = (int)(rt / 2), r = t & (LEX_RING - 1);
-        const unsigned m = s_max[r];
-        if (exit_out && __uint_as_float(m) < tol) atomicMin(exit_out, t);
-        if (t == runIters - 1) s_lastmax = m;
-        s_max[r] = 0u;  // (slot reused by sweep t + LEX_RING, not yet started)
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      st->sweeps = runIters;
-      st->last_maxdiv = (double)__uint_as_float(s_lastmax);
-    }
-    return;
-  }
-  // Start sweep 0 at step 0.
-  if (threadIdx.x == 0) {
-    s_start[0] = 0;
-    s_max[0] = 0u;
-    s_cont[0] = 0;
-    s_hi = 1;
-  }
-  __syncthreads();
-  // Bounded: each sweep takes D steps and starts at most D + 2 steps after
-  // the previous one.
-  const long long max_steps = (long long)numIters * (D + 2) + D + 4;
-  for (long long tau = 0; tau < max_steps; ++tau) {
-    const int lo = s_lo, hi = s_hi;
-    step(tau, lo, hi - lo, [&](int t) { return (int)(tau - s_start[t & (LEX_RING - 1)]); },
-         numIters, false);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      // Retire sweeps whose last diagonal ran in this step.
-      while (s_lo < s_hi && tau - s_start[s_lo & (LEX_RING - 1)] >= D - 1) {
-        int r = s_lo & (LEX_RING - 1);
-        s_last = s_lo;
-        if (early_exit && __uint_as_float(s_max[r]) < tol) s_exit = 1;
-        ++s_lo;
-      }
-      // Start the next sweep if allowed.
-      int nxt = s_hi;
-      if (!s_exit && nxt < numIters) {
-        int pr = (nxt - 1) & (LEX_RING - 1);
-        bool prev_done = s_lo > nxt - 1;
-        bool gap_ok = prev_done || (tau + 1 - s_start[pr] >= 2);
-        bool safe = !early_exit || prev_done || s_cont[pr];
-        if (gap_ok && safe && nxt - s_lo < LEX_RING) {
-          int r = nxt & (LEX_RING - 1);
-          s_start[r] = (int)(tau + 1);
-          s_max[r] = 0u;
-          s_cont[r] = 0;
-          s_hi = nxt + 1;
-        }
-      }
-      if (s_lo == s_hi && (s_exit || s_hi >= numIters)) s_done = 1;
-    }
-    __syncthreads();
-    if (s_done) break;
-  }
-  if (threadIdx.x == 0) {
-    st->sweeps = s_hi;
-    st->last_maxdiv = s_last >= 0 ? (double)__uint_as_float(s_max[s_last & (LEX_RING - 1)]) : 0.0;
-  }
-}
-
-// ------------------------------------------------------------------ LEXSOR on a cluster
-// k_lexsor's schedule on a thread-block cluster of LEX_CLUSTER blocks (one
-// SM each): the cells of a step are spread over all of the cluster's
-// threads and every step ends with a cluster barrier (release / acquire, so
-// the steps' global stores are ordered for the whole cluster; the fields are
-// read past L1).  The sweep bookkeeping (start steps, maxima, "cannot exit"
-// marks, retire / start decisions) lives in the shared memory of block rank
-// 0; the other blocks read and update it through distributed shared memory.
-// With the early exit a step takes two cluster barriers (the step, then rank
-// 0's decisions); without it the closed-form schedule needs one.
-constexpr int LEX_CLUSTER = 8;
-
-__device__ __forceinline__ unsigned cl_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
-               ::: "memory");
-}
-// Shared-window address of `p` (a shared variable) in block `rank` of the cluster.
-__device__ __forceinline__ uint32_t cl_map(const void* p, unsigned rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ int cl_ld(uint32_t a) {
-  int v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cl_st8(uint32_t a, unsigned v) {
-  asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void cl_max(uint32_t a, unsigned v) {
-  asm volatile("red.shared::cluster.max.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
-
-__global__ void __launch_bounds__(LEX_THREADS)
-    k_lexsor_cl(float* U, float* V, float* p, const uint8_t* __restrict__ flags, Grid g,
-                int numIters, float relax0, float damping, float cp, float tol, int early_exit,
-                DevStats* st, float minRelax, const int* __restrict__ stop, int SP,
-                int* __restrict__ exit_out, const int* __restrict__ run_from) {
-  __shared__ int s_start[LEX_RING];
-  __shared__ unsigned s_max[LEX_RING];
-  __shared__ uint8_t s_cont[LEX_RING];
-  __shared__ int s_lo, s_hi, s_done, s_exit, s_last;
-  const unsigned rank = cl_rank();
-  const int P = g.P;
-  const int ni = g.NX - 2, nj = g.NY - 2;
-  const int D = ni + nj - 1;
-  const int offE = SP ? SP + 1 : P, offN = SP ? SP : 1;
-  const int L = ni < nj ? ni : nj;
-  // Rank 0's bookkeeping, as seen from this block.
-  const uint32_t a_start = cl_map(s_start, 0), a_max = cl_map(s_max, 0),
-                 a_cont = cl_map(s_cont, 0), a_lo = cl_map(&s_lo, 0), a_hi = cl_map(&s_hi, 0),
-                 a_done = cl_map(&s_done, 0);
-  if (rank == 0) {
-    for (int r = threadIdx.x; r < LEX_RING; r += LEX_THREADS) {
-      s_max[r] = 0u;
-      s_cont[r] = 0;
-    }
-    if (threadIdx.x == 0) {
-      s_start[0] = 0;
-      s_lo = 0;
-      s_hi = 1;
-      s_done = 0;
-      s_exit = 0;
-      s_last = -1;
-    }
-  }
-  cl_sync();
-  if (numIters <= 0 || ni <= 0 || nj <= 0) return;  // (the same in every block)
-  if (stop && *stop) return;
-  const int gt = (int)rank * LEX_THREADS + (int)threadIdx.x;
-  const int stride = LEX_CLUSTER * LEX_THREADS;
-  const int Lp = (L + 31) & ~31;
-  const float invLp = 1.0f / (float)Lp;
-  auto step = [&](long long tau, int lo, int W, auto delta_of, int runIters, bool all) {
-    const int items = W * Lp;
-    for (int base = 0; base < items; base += LEX_CHUNK * stride) {
-      int cc[LEX_CHUNK], rr[LEX_CHUNK], tt[LEX_CHUNK];
-      bool act[LEX_CHUNK] = {};
-      uint8_t fl[LEX_CHUNK];
-      float u0[LEX_CHUNK], u1[LEX_CHUNK], v0[LEX_CHUNK], v1[LEX_CHUNK], p0[LEX_CHUNK];
-#pragma unroll
-      for (int m = 0; m < LEX_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (uniform over the cluster)
-        const int q = base + m * stride + gt;
-        int k;
-        const int t = lo + (items < (1 << 24) ? div_small(q, Lp, invLp, k) : (k = q % Lp, q / Lp));
-        const int r = t & (LEX_RING - 1);
-        const int delta = q < items ? delta_of(t) : -1;
-        const int d = 2 + delta;
-        const int i_lo = max(1, d - nj), i_hi = min(ni, d - 1);
-        const int i = i_lo + k;
-        const bool in = delta >= 0 && delta < D && k < L && i <= i_hi;
-        const int c = in ? (SP ? d * SP + i : i * P + (d - i)) : 0;
-        cc[m] = c;
-        rr[m] = r;
-        tt[m] = t;
-        act[m] = in;
-        fl[m] = in ? __ldcg(flags + c) : 0;
-        u0[m] = in ? __ldcg(U + c) : 0.0f;
-        u1[m] = in ? __ldcg(U + c + offE) : 0.0f;
-        v0[m] = in ? __ldcg(V + c) : 0.0f;
-        v1[m] = in ? __ldcg(V + c + offN) : 0.0f;
-        p0[m] = in ? __ldcg(p + c) : 0.0f;
-      }
-#pragma unroll
-      for (int m = 0; m < LEX_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (whole warps: items is a multiple of 32)
-        const uint8_t f = fl[m];
-        bool a = act[m] && (f & F_FLUID);
-        const float sx0 = fbit(f, F_W), sx1 = fbit(f, F_E), sy0 = fbit(f, F_S),
-                    sy1 = fbit(f, F_N);
-        const float s = sx0 + sx1 + sy0 + sy1;
-        a = a && s != 0.0f;
-        const float div = a ? u1[m] - u0[m] + v1[m] - v0[m] : 0.0f;
-        const float absDiv = fabsf(div);
-        const bool counted = a && !isnan(absDiv);
-        const unsigned mx = __reduce_max_sync(0xffffffffu, counted ? __float_as_uint(absDiv) : 0u);
-        const bool cont = __any_sync(0xffffffffu, counted && absDiv >= tol);
-        if ((threadIdx.x & 31) == 0 && (early_exit || all || tt[m] == runIters - 1)) {
-          if (mx) cl_max(a_max + 4u * rr[m], mx);
-          if (cont) cl_st8(a_cont + (unsigned)rr[m], 1u);
-        }
-        if (!a) continue;
-        const int c = cc[m];
-        // Relaxation of sweep t (fluid.go:169-170).
-        float iterProgress = (float)tt[m] / (float)numIters;
-        float rel = relax0 - (relax0 - minRelax) * iterProgress;
-        float pp = -div / s;
-        pp *= rel;
-        pp *= damping;
-        p[c] = p0[m] + cp * pp;
-        U[c] = u0[m] - sx0 * pp;
-        U[c + offE] = u1[m] + sx1 * pp;
-        V[c] = v0[m] - sy0 * pp;
-        V[c + offN] = v1[m] + sy1 * pp;
-      }
-    }
-  };
-  if (!early_exit) {
-    // The closed-form schedule, as in k_lexsor (exit_out / run_from alike);
-    // rank 0's thread 0 retires the sweeps.
-    int runIters = numIters;
-    if (run_from) {
-      const int e = *run_from;
-      if (e < 0 || e >= numIters) {
-        cl_sync();
-        return;
-      }
-      runIters = e + 1;
-    }
-    const long long steps = (long long)D + 2LL * (runIters - 1);
-    for (long long tau = 0; tau < steps; ++tau) {
-      int t_lo = (int)((tau - D + 2) / 2);
-      if (t_lo < 0) t_lo = 0;
-      while (tau - 2LL * t_lo >= D) ++t_lo;
-      int t_hi = (int)(tau / 2);
-      if (t_hi > runIters - 1) t_hi = runIters - 1;
-      step(tau, t_lo, t_hi - t_lo + 1, [&](int t) { return (int)(tau - 2LL * t); }, runIters,
-           exit_out != nullptr);
-      cl_sync();
-      const long long rt = tau - (D - 1);
-      if (rank == 0 && threadIdx.x == 0 && rt >= 0 && (rt & 1) == 0 && rt / 2 < runIters) {
-        const int t = (int)(rt / 2), r = t & (LEX_RING - 1);
-        const unsigned m = s_max[r];
-        if (exit_out && __uint_as_float(m) < tol) atomicMin(exit_out, t);
-        if (t == runIters - 1) s_last = (int)m;
-        s_max[r] = 0u;  // (slot reused by sweep t + LEX_RING, not yet started)
-      }
-    }
-    cl_sync();
-    if (rank == 0 && threadIdx.x == 0) {
-      st->sweeps = runIters;
-      st->last_maxdiv = (double)__uint_as_float((unsigned)s_last);
-    }
-    cl_sync();  // (no block leaves while others may still address rank 0)
-    return;
-  }
-  const long long max_steps = (long long)numIters * (D + 2) + D + 4;
-  for (long long tau = 0; tau < max_steps; ++tau) {
-    const int lo = cl_ld(a_lo), hi = cl_ld(a_hi);
-    step(tau, lo, hi - lo,
-         [&](int t) { return (int)(tau - cl_ld(a_start + 4u * (t & (LEX_RING - 1)))); },
-         numIters, false);
-    cl_sync();
-    if (rank == 0 && threadIdx.x == 0) {
-      // Retire sweeps whose last diagonal ran in this step.
-      while (s_lo < s_hi && tau - s_start[s_lo & (LEX_RING - 1)] >= D - 1) {
-        int r = s_lo & (LEX_RING - 1);
-        s_last = s_lo;
-        if (__uint_as_float(s_max[r]) < tol) s_exit = 1;
-        ++s_lo;
-      }
-      // Start the next sweep if allowed.
-      int nxt = s_hi;
-      if (!s_exit && nxt < numIters) {
-        int pr = (nxt - 1) & (LEX_RING - 1);
-        bool prev_done = s_lo > nxt - 1;
-        bool gap_ok = prev_done || (tau + 1 - s_start[pr] >= 2);
-        bool safe = prev_done || s_cont[pr];
-        if (gap_ok && safe && nxt - s_lo < LEX_RING) {
-          int r = nxt & (LEX_RING - 1);
-          s_start[r] = (int)(tau + 1);
-          s_max[r] = 0u;
-          s_cont[r] = 0;
-          s_hi = nxt + 1;
-        }
-      }
-      if (s_lo == s_hi && (s_exit || s_hi >= numIters)) s_done = 1;
-    }
-    cl_sync();
-    if (cl_ld(a_done)) break;
-  }
-  if (rank == 0 && threadIdx.x == 0) {
-    st->sweeps = s_hi;
-    st->last_maxdiv = s_last >= 0 ? (double)__uint_as_float(s_max[s_last & (LEX_RING - 1)]) : 0.0;
-  }
-  cl_sync();
-}
-
-// ------------------------------------------------------------------ LEXSOR on the whole GPU
-// The closed-form schedule (no early exit, or the speculative early exit's
-// two passes) over every SM: a cooperative launch of one block per SM, a
-// grid barrier per step.  For solves with many sweeps in flight (a step
-// then holds hundreds of thousands of cells: the reference's 200-sweep
-// workload at 2048^2) the step is compute-bound and the cluster's 8 SMs are
-// too few.  Scratch (lex): [0, LEX_RING) the sweeps' maxima, then the
-// barrier's arrival count and generation, then its give-up flag.
-constexpr int LEX_GRID_SCRATCH = LEX_RING + 4;
-
-// A grid barrier: the block's last arrival advances the generation; the
-// others wait for it, for at most about a second (then *fail is set and
-// they go on; the solve's result is then not to be used).  Release / acquire
-// at GPU scope around it order the steps' stores.
-__device__ __forceinline__ void grid_barrier(unsigned* count, unsigned* gen, unsigned nblocks,
-                                             int* fail) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned g0;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(g0) : "l"(gen) : "memory");
-    __threadfence();
-    if (atomicAdd(count, 1u) == nblocks - 1) {
-      *count = 0u;
-      __threadfence();
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(gen) : "memory");
-    } else {
-      const unsigned long long t0 = global_ns();
-      for (int it = 0; it < MBAR_MAX_TRIES; ++it) {
-        unsigned gv;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(gv) : "l"(gen) : "memory");
-        if (gv != g0) break;
-        if (global_ns() - t0 > MBAR_WAIT_NS) {
-          atomicExch(fail, 1);
-          break;
-        }
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(LEX_THREADS)
-    k_lexsor_grid(float* U, float* V, float* p, const uint8_t* __restrict__ flags, Grid g,
-                  int numIters, float relax0, float damping, float cp, float tol, DevStats* st,
-                  float minRelax, int SP, int* __restrict__ exit_out,
-                  const int* __restrict__ run_from, unsigned* __restrict__ lex, int* err) {
-  const int P = g.P;
-  const int ni = g.NX - 2, nj = g.NY - 2;
-  const int D = ni + nj - 1;
-  const int offE = SP ? SP + 1 : P, offN = SP ? SP : 1;
-  const int L = ni < nj ? ni : nj;
-  unsigned* gmax = lex;
-  unsigned* bcount = lex + LEX_RING;
-  unsigned* bgen = lex + LEX_RING + 1;
-  int* bfail = reinterpret_cast<int*>(lex + LEX_RING + 2);
-  const unsigned nb = gridDim.x;
-  if (numIters <= 0 || ni <= 0 || nj <= 0) return;  // (the same in every block)
-  int runIters = numIters;
-  if (run_from) {
-    const int e = *run_from;
-    if (e < 0 || e >= numIters) return;
-    runIters = e + 1;
-  }
-  // (gmax and the barrier words were zeroed before the launch.)
-  const int gt = (int)blockIdx.x * LEX_THREADS + (int)threadIdx.x;
-  const int stride = (int)nb * LEX_THREADS;
-  const int Lp = (L + 31) & ~31;
-  const float invLp = 1.0f / (float)Lp;
-  const long long steps = (long long)D + 2LL * (runIters - 1);
-  for (long long tau = 0; tau < steps; ++tau) {
-    int t_lo = (int)((tau - D + 2) / 2);
-    if (t_lo < 0) t_lo = 0;
-    while (tau - 2LL * t_lo >= D) ++t_lo;
-    int t_hi = (int)(tau / 2);
-    if (t_hi > runIters - 1) t_hi = runIters - 1;
-    const int lo = t_lo, W = t_hi - t_lo + 1;
-    const int items = W * Lp;
-    for (int base = 0; base < items; base += LEX_CHUNK * stride) {
-      int cc[LEX_CHUNK], rr[LEX_CHUNK], tt[LEX_CHUNK];
-      bool act[LEX_CHUNK] = {};
-      uint8_t fl[LEX_CHUNK];
-      float u0[LEX_CHUNK], u1[LEX_CHUNK], v0[LEX_CHUNK], v1[LEX_CHUNK], p0[LEX_CHUNK];
-#pragma unroll
-      for (int m = 0; m < LEX_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (uniform over the grid)
-        const int q = base + m * stride + gt;
-        int k;
-        const int t = lo + (items < (1 << 24) ? div_small(q, Lp, invLp, k) : (k = q % Lp, q / Lp));
-        const int r = t & (LEX_RING - 1);
-        const int delta = q < items ? (int)(tau - 2LL * t) : -1;
-        const int d = 2 + delta;
-        const int i_lo = max(1, d - nj), i_hi = min(ni, d - 1);
-        const int i = i_lo + k;
-        const bool in = delta >= 0 && delta < D && k < L && i <= i_hi;
-        const int c = in ? (SP ? d * SP + i : i * P + (d - i)) : 0;
-        cc[m] = c;
-        rr[m] = r;
-        tt[m] = t;
-        act[m] = in;
-        fl[m] = in ? __ldcg(flags + c) : 0;
-        u0[m] = in ? __ldcg(U + c) : 0.0f;
-        u1[m] = in ? __ldcg(U + c + offE) : 0.0f;
-        v0[m] = in ? __ldcg(V + c) : 0.0f;
-        v1[m] = in ? __ldcg(V + c + offN) : 0.0f;
-        p0[m] = in ? __ldcg(p + c) : 0.0f;
-      }
-#pragma unroll
-      for (int m = 0; m < LEX_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (the slots the loads filled)
-        const uint8_t f = fl[m];
-        bool a = act[m] && (f & F_FLUID);
-        const float sx0 = fbit(f, F_W), sx1 = fbit(f, F_E), sy0 = fbit(f, F_S),
-                    sy1 = fbit(f, F_N);
-        const float s = sx0 + sx1 + sy0 + sy1;
-        a = a && s != 0.0f;
-        const float div = a ? u1[m] - u0[m] + v1[m] - v0[m] : 0.0f;
-        const float absDiv = fabsf(div);
-        const bool counted = a && !isnan(absDiv);
-        const unsigned mx = __reduce_max_sync(0xffffffffu, counted ? __float_as_uint(absDiv) : 0u);
-        if ((threadIdx.x & 31) == 0 && mx && (exit_out || tt[m] == runIters - 1))
-          atomicMax(&gmax[rr[m]], mx);
-        if (!a) continue;
-        const int c = cc[m];
-        // Relaxation of sweep t (fluid.go:169-170).
-        float iterProgress = (float)tt[m] / (float)numIters;
-        float rel = relax0 - (relax0 - minRelax) * iterProgress;
-        float pp = -div / s;
-        pp *= rel;
-        pp *= damping;
-        p[c] = p0[m] + cp * pp;
-        U[c] = u0[m] - sx0 * pp;
-        U[c + offE] = u1[m] + sx1 * pp;
-        V[c] = v0[m] - sy0 * pp;
-        V[c + offN] = v1[m] + sy1 * pp;
-      }
-    }
-    grid_barrier(bcount, bgen, nb, bfail);
-    // Block 0 retires the sweep whose last diagonal ran in this step (its
-    // slot is next used LEX_RING sweeps later).
-    const long long rt = tau - (D - 1);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && rt >= 0 && (rt & 1) == 0 && rt / 2 < runIters) {
-      const int t = (int)(rt / 2), r = t & (LEX_RING - 1);
-      const unsigned m = atomicExch(&gmax[r], 0u);
-      if (exit_out && __uint_as_float(m) < tol) atomicMin(exit_out, t);
-      if (t == runIters - 1) {
-        st->sweeps = runIters;
-        st->last_maxdiv = (double)__uint_as_float(m);
-      }
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && *bfail) atomicExch(err, 1);
-}
-
-// Copies of U, V, p and the flags into the diagonal-major layout of the
-// wavefront kernel (cell (i, j) at (i + j) * SP + i) and of U, V, p back.
-__global__ void k_skew_in(const float* __restrict__ U, const float* __restrict__ V,
-                          const float* __restrict__ p, const uint8_t* __restrict__ flags,
-                          float* __restrict__ sU, float* __restrict__ sV, float* __restrict__ sp,
-                          uint8_t* __restrict__ sf, Grid g, int SP,
-                          const int* __restrict__ only_if = nullptr, int limit = 0) {
-  if (only_if && *only_if >= limit) return;  // (the re-run copy: only when it runs)
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.NX || j >= g.NY) return;
-  const size_t c = (size_t)i * g.P + j, s = (size_t)(i + j) * SP + i;
-  sU[s] = U[c];
-  sV[s] = V[c];
-  sp[s] = p[c];
-  sf[s] = flags[c];
-}
-__global__ void k_skew_out(const float* __restrict__ sU, const float* __restrict__ sV,
-                           const float* __restrict__ sp, float* __restrict__ U,
-                           float* __restrict__ V, float* __restrict__ p, Grid g, int SP) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.NX || j >= g.NY) return;
-  const size_t c = (size_t)i * g.P + j, s = (size_t)(i + j) * SP + i;
-  U[c] = sU[s];
-  V[c] = sV[s];
-  p[c] = sp[s];
-}
-
-// ------------------------------------------------------------------ multigrid
-// solveMultigridVCycle (fluid.go:559-594) with its helpers (fluid.go:596-758,
-// 1122-1149): per iteration three SOR sweeps at relaxation 1.5 (k_lexsor),
-// the early exit on the last sweep's max |div|, the residual restricted by
-// full weighting to the (NX+1)/2 x (NY+1)/2 grid, 40 lexicographic
-// Gauss-Seidel sweeps there at relaxation 1.6, the bilinear prolongation
-// applied to p and the faces, three SOR sweeps at 1.2.  Every stage keeps
-// the reference's per-cell operation order; the serial loops become a
-// wavefront (the SOR sweeps, the coarse sweeps) or a per-face kernel that
-// applies a face's two updates in the loop's order (the correction).  Once
-// a solve exits early, *stop makes every later kernel of it return.
-
-// After the three pre-smoothing sweeps: count them and latch the exit when
-// the last one's max |div| is below the tolerance.
-__global__ void k_mg_check(const DevStats* __restrict__ sm, DevStats* st, int* stop, float tol,
-                           int post) {
-  if (*stop) return;
-  st->sweeps += 3;
-  if (post) return;
-  float maxDiv = (float)sm->last_maxdiv;
-  st->last_maxdiv = sm->last_maxdiv;
-  if (maxDiv < tol) *stop = 1;
-}
-
-// computePressureResidual (fluid.go:596-628): r = -div - laplacian(p) on
-// fluid interior cells, 0 elsewhere.
-__global__ void k_mg_residual(const float* __restrict__ U, const float* __restrict__ V,
-                              const float* __restrict__ p, const uint8_t* __restrict__ flags,
-                              float* __restrict__ r, const int* __restrict__ stop, Grid g) {
-  if (*stop) return;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.NX || j >= g.NY) return;
-  const int P = g.P;
-  int c = i * P + j;
-  uint8_t fl = flags[c];
-  float out = 0.0f;
-  if ((fl & (F_FLUID | F_INTERIOR)) == (F_FLUID | F_INTERIOR)) {
-    float div = U[c + P] - U[c] + V[c + 1] - V[c];
-    float sx0 = fbit(fl, F_W), sx1 = fbit(fl, F_E), sy0 = fbit(fl, F_S), sy1 = fbit(fl, F_N);
-    float lap = sx0 * (p[c - P] - p[c]) + sx1 * (p[c + P] - p[c]) + sy0 * (p[c - 1] - p[c]) +
-                sy1 * (p[c + 1] - p[c]);
-    out = -div - lap;
-  }
-  r[c] = out;
-}
-
-// restrictResidual (fluid.go:630-660) into the coarse grid (pitch cP = cNY).
-// Coarse-grid index of cell (i, j): row-major i * cNY + j (CSP = 0) or
-// diagonal-major (i + j) * CSP + i.
-__device__ __forceinline__ int cidx(int i, int j, int cNY, int CSP) {
-  return CSP ? (i + j) * CSP + i : i * cNY + j;
-}
-
-// The coarse solid mask: the fine cell (2i, 2j) (fluid.go:672-685).
-__device__ __forceinline__ float coarse_s(const uint8_t* __restrict__ flags, int i, int j,
-                                          const Grid& g) {
-  int fi = 2 * i, fj = 2 * j;
-  if (fi >= g.NX || fj >= g.NY) return 0.0f;
-  return (flags[fi * g.P + fj] & F_FLUID) ? 1.0f : 0.0f;
-}
-
-// restrictResidual (fluid.go:630-660) into cr at cidx; with CSP > 0 also the
-// coarse mask of every coarse cell into cmask (same layout).
-__global__ void k_mg_restrict(const float* __restrict__ r, float* __restrict__ cr,
-                              const int* __restrict__ stop, Grid g, int cNX, int cNY, int CSP,
-                              const uint8_t* __restrict__ flags, uint8_t* __restrict__ cmask) {
-  if (*stop) return;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= cNX || j >= cNY) return;
-  float out = 0.0f;
-  int fi = 2 * i, fj = 2 * j;
-  if (i >= 1 && i < cNX - 1 && j >= 1 && j < cNY - 1 && fi < g.NX - 1 && fj < g.NY - 1) {
-    const int P = g.P;
-    int c = fi * P + fj;
-    float center = r[c] * 0.25f;
-    float nb = (r[c - P] + r[c + P] + r[c - 1] + r[c + 1]) * 0.125f;
-    float cr4 = (r[c - P - 1] + r[c + P - 1] + r[c - P + 1] + r[c + P + 1]) * 0.0625f;
-    out = center + nb + cr4;
-  }
-  const int ci = cidx(i, j, cNY, CSP);
-  cr[ci] = out;
-  if (CSP) cmask[ci] = coarse_s(flags, i, j, g) != 0.0f ? 1 : 0;
-}
-
-// solveCoarseGrid (fluid.go:662-715): 40 lexicographic Gauss-Seidel sweeps
-// from zero, in one block.  Cell (i, j) of a sweep needs (i-1, j), (i, j-1)
-// of that sweep and (i+1, j), (i, j+1) of the previous one, so the sweeps
-// run as anti-diagonal wavefronts, each two diagonals behind the previous.
-constexpr int MG_THREADS = 1024;
-constexpr int MG_CHUNK = 4;  // cells whose loads a thread issues together
-// CLUSTER: the same schedule on a thread-block cluster of LEX_CLUSTER blocks
-// (a step's cells over all of its threads, a cluster barrier per step, the
-// solution read past L1), for coarse grids whose steps hold many cells.
-template <bool CLUSTER>
-__global__ void __launch_bounds__(MG_THREADS)
-    k_mg_coarse(const float* __restrict__ cr, float* __restrict__ cp_,
-                const uint8_t* __restrict__ flags, const int* __restrict__ stop, Grid g, int cNX,
-                int cNY, int sweeps, float relaxation, int CSP,
-                const uint8_t* __restrict__ cmask) {
-  if (*stop) return;  // (the same in every block)
-  const int ni = cNX - 2, nj = cNY - 2;
-  // Row-major (CSP = 0): neighbours at -cNY, +cNY, -1, +1.  Diagonal-major:
-  // west -(CSP+1), east +(CSP+1), south -CSP, north +CSP, and the cells of a
-  // step contiguous along their diagonal.
-  const int oW = CSP ? CSP + 1 : cNY, oS = CSP ? CSP : 1;
-  const int n0 = CSP ? (cNX + cNY - 1) * CSP : cNX * cNY;
-  const int gt = CLUSTER ? (int)cl_rank() * MG_THREADS + (int)threadIdx.x : (int)threadIdx.x;
-  const int stride = CLUSTER ? LEX_CLUSTER * MG_THREADS : MG_THREADS;
-  auto barrier = [] {
-    if (CLUSTER)
-      cl_sync();
-    else
-      __syncthreads();
-  };
-  for (int k = gt; k < n0; k += stride) cp_[k] = 0.0f;
-  barrier();
-  if (ni <= 0 || nj <= 0) return;
-  const int D = ni + nj - 1;
-  const int L = ni < nj ? ni : nj;
-  const float invL = 1.0f / (float)L;
-  const long long steps = (long long)D + 2LL * (sweeps - 1);
-  for (long long tau = 0; tau < steps; ++tau) {
-    // Sweeps t with 0 <= tau - 2t < D, each on diagonal d = tau - 2t + 2.
-    int t_lo = (int)((tau - D + 2) / 2);
-    if (t_lo < 0) t_lo = 0;
-    while (tau - 2LL * t_lo >= D) ++t_lo;
-    int t_hi = (int)(tau / 2);
-    if (t_hi > sweeps - 1) t_hi = sweeps - 1;
-    int nact = t_hi - t_lo + 1;
-    // The cells of a step are independent (one diagonal per sweep in flight,
-    // sweeps two diagonals apart, no cell reads another's value): a thread
-    // loads the inputs of MG_CHUNK cells at once, then updates them.
-    const int items = nact * L;
-    for (int base = 0; base < items; base += MG_CHUNK * stride) {
-      int cc[MG_CHUNK];
-      bool in[MG_CHUNK] = {};  // (slots past the step's cells stay out)
-      float s0[MG_CHUNK], s1[MG_CHUNK], s2[MG_CHUNK], s3[MG_CHUNK], sc[MG_CHUNK];
-      float pc[MG_CHUNK], pw[MG_CHUNK], pe[MG_CHUNK], ps[MG_CHUNK], pn[MG_CHUNK], rc[MG_CHUNK];
-#pragma unroll
-      for (int m = 0; m < MG_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (uniform over the block or cluster)
-        const int q = base + m * stride + gt;
-        int k;
-        const int t = t_lo + (items < (1 << 24) ? div_small(q, L, invL, k) : (k = q % L, q / L));
-        const int d = (int)(tau - 2LL * t) + 2;
-        const int i_lo = max(1, d - nj), i_hi = min(ni, d - 1);
-        const int i = i_lo + k;
-        const bool ok = q < items && i <= i_hi;
-        const int j = d - i;
-        const int c = ok ? cidx(i, j, cNY, CSP) : 0;
-        cc[m] = c;
-        in[m] = ok;
-        if (CSP) {
-          sc[m] = ok ? (float)cmask[c] : 0.0f;
-          s0[m] = ok ? (float)cmask[c - oW] : 0.0f;
-          s1[m] = ok ? (float)cmask[c + oW] : 0.0f;
-          s2[m] = ok ? (float)cmask[c - oS] : 0.0f;
-          s3[m] = ok ? (float)cmask[c + oS] : 0.0f;
-        } else {
-          sc[m] = ok ? coarse_s(flags, i, j, g) : 0.0f;
-          s0[m] = ok ? coarse_s(flags, i - 1, j, g) : 0.0f;
-          s1[m] = ok ? coarse_s(flags, i + 1, j, g) : 0.0f;
-          s2[m] = ok ? coarse_s(flags, i, j - 1, g) : 0.0f;
-          s3[m] = ok ? coarse_s(flags, i, j + 1, g) : 0.0f;
-        }
-        auto ld = [&](int a) { return CLUSTER ? __ldcg(cp_ + a) : cp_[a]; };
-        pc[m] = ok ? ld(c) : 0.0f;
-        pw[m] = ok ? ld(c - oW) : 0.0f;
-        pe[m] = ok ? ld(c + oW) : 0.0f;
-        ps[m] = ok ? ld(c - oS) : 0.0f;
-        pn[m] = ok ? ld(c + oS) : 0.0f;
-        rc[m] = ok ? cr[c] : 0.0f;
-      }
-#pragma unroll
-      for (int m = 0; m < MG_CHUNK; ++m) {
-        if (base + m * stride >= items) break;  // (the slots the loads filled)
-        if (!in[m] || sc[m] == 0.0f) continue;
-        const float sx0 = s0[m], sx1 = s1[m], sy0 = s2[m], sy1 = s3[m];
-        const float s = sx0 + sx1 + sy0 + sy1;
-        if (s == 0.0f) continue;
-        const float p0 = pc[m];
-        float lap = sx0 * (pw[m] - p0) + sx1 * (pe[m] - p0) + sy0 * (ps[m] - p0) +
-                    sy1 * (pn[m] - p0);
-        float residual = rc[m] - lap;
-        float correction = -residual / s * relaxation;
-        cp_[cc[m]] = p0 + correction;
-      }
-    }
-    barrier();
-  }
-}
-
-// prolongateCorrection (fluid.go:717-758) at fine cell (i, j).
-__device__ __forceinline__ float mg_corr(const float* __restrict__ cc, int i, int j, int cNX,
-                                         int cNY, int CSP) {
-  int ci = i / 2, cj = j / 2;
-  if (ci >= cNX - 1 || cj >= cNY - 1) return 0.0f;
-  float fI = (float)(i % 2) * 0.5f, fJ = (float)(j % 2) * 0.5f;
-  return (1.0f - fI) * (1.0f - fJ) * cc[cidx(ci, cj, cNY, CSP)] +
-         fI * (1.0f - fJ) * cc[cidx(ci + 1, cj, cNY, CSP)] +
-         (1.0f - fI) * fJ * cc[cidx(ci, cj + 1, cNY, CSP)] +
-         fI * fJ * cc[cidx(ci + 1, cj + 1, cNY, CSP)];
-}
-
-// applePressureCorrection (fluid.go:1122-1149): p += corr * cp on fluid
-// interior cells; face (i, j) of U first gets + S_i corr(i-1, j) from cell
-// (i-1, j), then - S_{i-1} corr(i, j) from cell (i, j), as the loop visits
-// them; V likewise along j.
-__global__ void k_mg_apply(float* __restrict__ U, float* __restrict__ V, float* __restrict__ p,
-                           const float* __restrict__ cc, const uint8_t* __restrict__ flags,
-                           const int* __restrict__ stop, float cp, Grid g, int cNX, int cNY,
-                           int CSP) {
-  if (*stop) return;
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.NX || j >= g.NY) return;
-  const int P = g.P;
-  int c = i * P + j;
-  auto fluid_int = [&](int a, int b) {
-    return a >= 1 && a <= g.NX - 2 && b >= 1 && b <= g.NY - 2 &&
-           (flags[a * P + b] & F_FLUID) != 0;
-  };
-  bool self = fluid_int(i, j);
-  float corr = self ? mg_corr(cc, i, j, cNX, cNY, CSP) : 0.0f;
-  if (self) p[c] += corr * cp;
-  uint8_t fl = flags[c];
-  if (i >= 1) {
-    float u = U[c];
-    if (fluid_int(i - 1, j)) u += fbit(fl, F_FLUID) * mg_corr(cc, i - 1, j, cNX, cNY, CSP);
-    if (self) u -= fbit(fl, F_W) * corr;
-    U[c] = u;
-  }
-  if (j >= 1) {
-    float v = V[c];
-    if (fluid_int(i, j - 1)) v += fbit(fl, F_FLUID) * mg_corr(cc, i, j - 1, cNX, cNY, CSP);
-    if (self) v -= fbit(fl, F_S) * corr;
-    V[c] = v;
-  }
 }
 
 // ------------------------------------------------------------------ parallel scheme
@@ -2628,201 +1738,6 @@ cudaError_t launch_jacobi_solve(fg_fluid* f, void* ctl, const float* b, const fl
   return jacobi_solve(f, (PCtl*)ctl, b, bw, x0, x1, iters, false);
 }
 
-// One k_lexsor solve on the handle's fields: on the diagonal-major copies
-// when the handle has them (copied in and back around the solve), else on
-// the row-major fields.
-// Blocks of the grid-wide wavefront the GPU holds at once (0: unavailable);
-// checked once per process by init_lexsor_cluster.
-static std::atomic<int> g_lex_grid_blocks{0};
-
-// Whether the cluster form of the wavefront can run on this device (checked
-// once per process, outside any capture: fg_create calls it).
-static std::atomic<int> g_lex_cluster{-1};
-void init_lexsor_cluster() {
-  if (g_lex_cluster.load() >= 0) return;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(LEX_CLUSTER);
-  cfg.blockDim = dim3(LEX_THREADS);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = LEX_CLUSTER;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  const bool ok = cudaOccupancyMaxActiveClusters(&n, k_lexsor_cl, &cfg) == cudaSuccess && n >= 1;
-  cudaGetLastError();
-  g_lex_cluster.store(ok ? 1 : 0);
-  int dev = 0, coop = 0, per = 0, sms = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lexsor_grid, LEX_THREADS, 0) ==
-          cudaSuccess &&
-      per >= 1)
-    g_lex_grid_blocks.store(per * sms);
-  cudaGetLastError();
-}
-
-int lexsor_scratch_words() { return LEX_GRID_SCRATCH; }
-
-// One wavefront solve: the cluster kernel when a step gives its threads work
-// (diagonals of at least 256 cells, at least 8 sweeps in the pipeline), else
-// one block (whose barrier is cheaper than the cluster's).
-static void lexsor_kernel(fg_fluid* f, float* U, float* V, float* p, const uint8_t* flags,
-                          int iters, float relax0, float cp, int early_exit, DevStats* st,
-                          float minRelax, const int* stop, int SP, int* exit_out = nullptr,
-                          const int* run_from = nullptr) {
-  const int L = std::min(f->NX - 2, f->NY - 2);
-  // Many sweeps in flight on long diagonals (the closed-form schedule only;
-  // no multigrid stop latch): every SM, a grid barrier per step.
-  const int nblk = g_lex_grid_blocks.load();
-  const int D = f->NX + f->NY - 5;  // (sweeps in flight must fit the maxima's ring)
-  if (!early_exit && !stop && f->lex_scratch && nblk > 0 && L >= 256 && iters >= 32 &&
-      D / 2 + 4 < LEX_RING) {
-    cudaMemsetAsync(f->lex_scratch, 0, sizeof(unsigned) * LEX_GRID_SCRATCH, f->stream);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nblk);
-    cfg.blockDim = dim3(LEX_THREADS);
-    cfg.stream = f->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_lexsor_grid, U, V, p, flags, f->g, iters, relax0,
-                           f->prm.pressure_damping, cp, f->prm.tolerance, st, minRelax, SP,
-                           exit_out, run_from, f->lex_scratch, &f->dstats->timeout) ==
-        cudaSuccess) {
-      count(f);
-      return;
-    }
-    cudaGetLastError();
-  }
-  if (L >= 256 && iters >= 8 && g_lex_cluster.load() == 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(LEX_CLUSTER);
-    cfg.blockDim = dim3(LEX_THREADS);
-    cfg.stream = f->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = LEX_CLUSTER;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_lexsor_cl, U, V, p, flags, f->g, iters, relax0,
-                           f->prm.pressure_damping, cp, f->prm.tolerance, early_exit, st,
-                           minRelax, stop, SP, exit_out, run_from) == cudaSuccess)
-      return;
-    cudaGetLastError();
-  }
-  k_lexsor<<<1, LEX_THREADS, 0, f->stream>>>(U, V, p, flags, f->g, iters, relax0,
-                                              f->prm.pressure_damping, cp, f->prm.tolerance,
-                                              early_exit, st, minRelax, stop, SP, exit_out,
-                                              run_from);
-}
-
-static void run_lexsor(fg_fluid* f, int iters, float relax0, float cp, int early_exit,
-                       DevStats* st, float minRelax, const int* stop, int* exit_slot) {
-  if (f->skew[0]) {
-    dim3 gr = cell_grid(f), bl(BX, BY);
-    const Grid& g = f->g;
-    k_skew_in<<<gr, bl, 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->d[FG_P], f->flags, f->skew[0],
-                                        f->skew[1], f->skew[2], f->skew_flags, g, f->skew_sp);
-    const int D = f->NX + f->NY - 5;  // anti-diagonals of the interior
-    if (early_exit && exit_slot && D / 2 + 4 < LEX_RING) {
-      // The early exit, speculatively: all sweeps on the closed-form
-      // schedule, recording the first sweep whose max |div| is below the
-      // tolerance; if there is one, the fields (untouched so far) are copied
-      // in again and exactly that many sweeps run.  Sweeps up to that one
-      // are the same in both runs, so this is the serial loop's result and
-      // the steps never wait for a "cannot exit" mark.
-      cudaMemsetAsync(exit_slot, 0x7f, sizeof(int), f->stream);
-      lexsor_kernel(f, f->skew[0], f->skew[1], f->skew[2], f->skew_flags, iters, relax0, cp, 0,
-                    st, minRelax, stop, f->skew_sp, exit_slot, nullptr);
-      k_skew_in<<<gr, bl, 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->d[FG_P], f->flags,
-                                          f->skew[0], f->skew[1], f->skew[2], f->skew_flags, g,
-                                          f->skew_sp, exit_slot, iters);
-      lexsor_kernel(f, f->skew[0], f->skew[1], f->skew[2], f->skew_flags, iters, relax0, cp, 0,
-                    st, minRelax, stop, f->skew_sp, nullptr, exit_slot);
-      count(f, 3);
-    } else {
-      lexsor_kernel(f, f->skew[0], f->skew[1], f->skew[2], f->skew_flags, iters, relax0, cp,
-                    early_exit, st, minRelax, stop, f->skew_sp);
-    }
-    k_skew_out<<<gr, bl, 0, f->stream>>>(f->skew[0], f->skew[1], f->skew[2], f->d[FG_U],
-                                         f->d[FG_V], f->d[FG_P], g, f->skew_sp);
-    count(f, 2);
-  } else {
-    lexsor_kernel(f, f->d[FG_U], f->d[FG_V], f->d[FG_P], f->flags, iters, relax0, cp, early_exit,
-                  st, minRelax, stop, 0);
-  }
-}
-
-// solveCoarseGrid's 40 sweeps: on the cluster when the coarse diagonals hold
-// at least 128 cells (a step then spans thousands), else on one block.
-static void launch_mg_coarse(fg_fluid* f, const int* stop, int cNX, int cNY, int CSP,
-                             const uint8_t* cmask) {
-  const int L = std::min(cNX - 2, cNY - 2);
-  if (CSP && L >= 128 && g_lex_cluster.load() == 1) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(LEX_CLUSTER);
-    cfg.blockDim = dim3(MG_THREADS);
-    cfg.stream = f->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = LEX_CLUSTER;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_mg_coarse<true>, (const float*)f->err, f->err2,
-                           (const uint8_t*)f->flags, stop, f->g, cNX, cNY, 40, 1.6f, CSP,
-                           cmask) == cudaSuccess)
-      return;
-    cudaGetLastError();
-  }
-  k_mg_coarse<false><<<1, MG_THREADS, 0, f->stream>>>(f->err, f->err2, f->flags, stop, f->g,
-                                                       cNX, cNY, 40, 1.6f, CSP, cmask);
-}
-
-cudaError_t launch_multigrid(fg_fluid* f, int num_iters, float dt) {
-  float cp = f->density * f->h / dt;  // fluid.go:560
-  const int cNX = (f->NX + 1) / 2, cNY = (f->NY + 1) / 2;
-  if ((size_t)cNX * cNY > (size_t)f->NX * f->P) return cudaErrorInvalidValue;
-  // Scratch: the fine residual in rhs, the coarse right-hand side and
-  // solution in err / err2, the stop latch and the smoothers' statistics in
-  // the correction solve's control block (unused by this scheme).
-  int* stop = reinterpret_cast<int*>(f->ectl);
-  DevStats* sm = reinterpret_cast<DevStats*>(reinterpret_cast<char*>(f->ectl) + 64);
-  cudaError_t e = cudaMemsetAsync(f->ectl, 0, 64 + sizeof(DevStats), f->stream);
-  if (e != cudaSuccess) return e;
-  dim3 gr = cell_grid(f), bl(BX, BY);
-  dim3 cg((cNY + BX - 1) / BX, (cNX + BY - 1) / BY);
-  // The coarse grid diagonal-major when it fits the scratch fields (err,
-  // err2; its mask in rhs_e) and the fine one is (the handle has the copies).
-  const int csp = (cNX + 31) / 32 * 32;
-  const int CSP = f->skew[0] && (size_t)(cNX + cNY - 1) * csp <= (size_t)f->NX * f->P ? csp : 0;
-  uint8_t* cmask = reinterpret_cast<uint8_t*>(f->rhs_e);
-  for (int it = 0; it < num_iters; ++it) {
-    count(f, 8);
-    run_lexsor(f, 3, 1.5f, cp, 0, sm, 1.5f, stop, nullptr);
-    k_mg_check<<<1, 1, 0, f->stream>>>(sm, f->dstats, stop, f->prm.tolerance, 0);
-    k_mg_residual<<<gr, bl, 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->d[FG_P], f->flags, f->rhs,
-                                            stop, f->g);
-    k_mg_restrict<<<cg, bl, 0, f->stream>>>(f->rhs, f->err, stop, f->g, cNX, cNY, CSP, f->flags,
-                                            cmask);
-    launch_mg_coarse(f, stop, cNX, cNY, CSP, cmask);
-    k_mg_apply<<<gr, bl, 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->d[FG_P], f->err2, f->flags,
-                                         stop, cp, f->g, cNX, cNY, CSP);
-    run_lexsor(f, 3, 1.2f, cp, 0, sm, 1.2f, stop, nullptr);
-    k_mg_check<<<1, 1, 0, f->stream>>>(sm, f->dstats, stop, f->prm.tolerance, 1);
-  }
-  return cudaGetLastError();
-}
-
 // ------------------------------------------------------------------ multigrid Jacobi
 // The MULTIGRID scheme: V(2,2) cycles on the masked Poisson system of the
 // Jacobi scheme.  A coarse cell covers up to 2 x 2 fine cells (the ghost
@@ -3204,14 +2119,7 @@ cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb
   float cp = f->density * f->h / dt;  // fluid.go:158
   cudaError_t e;
   f->jacobi_kernel = FG_JACOBI_KERNEL_NONE;
-  if (f->prm.scheme == FG_SCHEME_LEXSOR) {
-    count(f);
-    // (The correction solve's control block is free in this scheme: its
-    // first words hold the speculative early exit's sweep index.)
-    run_lexsor(f, num_iters, f->prm.relaxation, cp, f->prm.early_exit, f->dstats, 1.2f, nullptr,
-               reinterpret_cast<int*>(f->ectl));
-    return cudaGetLastError();
-  }
+  if (f->prm.scheme == FG_SCHEME_LEXSOR) return launch_lexsor(f, num_iters, dt);
   PCtl* ctl = (PCtl*)f->pctl;
   PCtl* ectl = (PCtl*)f->ectl;
   dim3 gr = cell_grid(f), bl(BX, BY);

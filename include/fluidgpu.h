@@ -410,7 +410,9 @@ const char* fg_last_error(const fg_fluid* f);
  * fg_debug_stall_tile(f, t): the dataflow Jacobi kernel never publishes tile
  * t of the handle's solves, so the tiles that read it wait until their
  * bounded waits (about a second) give up; the step's fg_get_stats returns
- * FG_ERR_TIMEOUT.  t < 0 disarms.  Changes the handle's captured graphs.
+ * FG_ERR_TIMEOUT.  With the reference's serial scheme, strip t of 32 rows
+ * sends nothing to the next one, with the same result.  t < 0 disarms.
+ * Changes the handle's captured graphs.
  * fg_debug_stall_tile(NULL, t): in later fg_project_noalloc calls, the
  * TMA-fed Jacobi kernel's copy barrier of tile t expects 16 bytes more than
  * its copies bring, so the block that sweeps tile t gives up after its
