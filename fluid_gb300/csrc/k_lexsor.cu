@@ -10,6 +10,7 @@
 // serial loop's sequence of operations, so the results are bit-identical.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "fg_internal.cuh"
 
@@ -31,10 +32,14 @@ inline dim3 cell_grid(const fg_fluid* f) {
 // w, which makes every dependency point to an earlier sweep or to the strip
 // below (smaller i), never back: a strip needs nothing of the strip above
 // within a group of G sweeps.  The strip's fields live in shared memory, a
-// ring of WV_W columns that a loader warp fills and a storer warp drains, so
-// the serial chain of a step is the shuffle and the arithmetic (about 50
-// cycles), where a wavefront through L2 with a barrier per anti-diagonal paid
-// a memory round trip and the barrier (2.4 us on one block, 2.4 us on eight).
+// ring of WV_W columns that a loader warp fills and a storer warp drains, so a
+// step costs the shuffle, the arithmetic and its own instructions (45 of them,
+// 50 ns), where a wavefront through L2 with a barrier per anti-diagonal paid
+// a memory round trip and the barrier (2.4 us, on one block or eight).
+// Chunks of 16 columns: a chunk's waits, packets and report take about 240
+// cycles, so 8 columns measured slower in a strip (20x2046, one sweep: 163
+// against 147 us) and 8 columns with 16 sweeps a block, whose ring then has
+// no slack, slower on large solves (2048^2, 200 sweeps: 2.56 against 2.35 ms).
 // Between strips the topmost lane hands each column's new values on as one
 // 16-byte packet {u, v, p, tag} in global memory, written and read whole, so
 // the receiving warp polls the data itself and no fence or flag stands
@@ -43,20 +48,32 @@ inline dim3 cell_grid(const fg_fluid* f) {
 // all of earlier tickets, so whatever number of blocks is resident the oldest
 // unfinished task can always proceed.
 //
+// Bound by the serial chain: NX + NY steps and a packet's flight per strip.
 // Measured on a GB300 against the wavefront through L2 that it replaced (one
 // block, an 8-block cluster or a grid barrier per anti-diagonal), whole
 // passes from the host: the app's 300x251 jet with 8 sweeps and the early
-// exit 1383 -> 329 us, two steps of a 128x128 jet with 40 sweeps 2891 -> 867
-// us, a 1024x768 box with BFECC 4471 -> 903 us, a 512x512 box with 8
-// reference V-cycles 45.7 -> 9.7 ms.
+// exit 1382 -> 178 us, two steps of a 128x128 jet with 40 sweeps 2890 -> 380
+// us, a 1024x768 box with BFECC 4439 -> 423 us, a 512x512 box with 8
+// reference V-cycles 45.5 -> 3.3 ms; 200 sweeps alone at 2048^2 2.35 ms.
 constexpr int WV_G = 8;            // sweeps per group (compute warps of a block)
-constexpr int WV_C = 8;            // columns per chunk
+constexpr int WV_C = 16;           // columns per chunk
 constexpr int WV_W = 256;          // ring columns
 constexpr int WV_M = WV_W - 1;
-constexpr int WV_FP = WV_W + 16;   // row pitch of the ring's flag bytes
+constexpr int WV_BEFORE = 64;      // columns before the row's start that the sweeps step through
+constexpr int WV_PAST = 96;        // columns past its end
 constexpr int WV_GROUPS = 256;     // groups per launch (slots of `fin` per strip)
 constexpr int WV_SWEEPS = WV_G * WV_GROUPS;
-constexpr int WV_A0 = 33 + WV_G, WV_A1 = 32 + WV_G;  // ring rows of the fields
+// The ring's rows: the first field's (U; the coarse solution), then V (the
+// coarse right-hand side), p (SOR only) and the cells' coefficient offsets.
+// Row q of each holds grid row i0 + q - WV_G, so a cell's values lie at
+// constant distances; 32 lanes on 32 rows and consecutive columns (a row is
+// a multiple of 32 words) never share a bank.
+constexpr int WV_A0 = 33 + WV_G, WV_A1 = 32 + WV_G;
+template <bool GS>
+struct WaveRing {
+  static constexpr int O1 = WV_A0 * WV_W, O2 = O1 + WV_A1 * WV_W,
+                       OF = GS ? O2 : O2 + WV_A1 * WV_W, WORDS = OF + WV_A1 * WV_W;
+};
 constexpr unsigned long long WV_WAIT_NS = 1000000000ull;  // a wait gives up after 1 s
 constexpr int WV_MAX_TRIES = 1 << 26;
 
@@ -79,7 +96,7 @@ struct WaveCtl {
 // have stopped before the last sweep, runs exactly its sweeps on the state
 // (sweeps up to that one are the same in both passes, so the result and the
 // count are the serial loop's).
-enum { WV_PLAIN = 0, WV_SPECULATE = 1, WV_FINISH = 2 };
+enum { WV_WLAIN = 0, WV_SPECULATE = 1, WV_FINISH = 2 };
 
 struct WaveArgs {
   // SOR: U, V, p.  Coarse Gauss-Seidel: the solution (zero before group 0)
@@ -160,9 +177,10 @@ __device__ __forceinline__ uint4 ld_pkt(const uint4* p) {
   return v;
 }
 __device__ __forceinline__ void st_pkt2(uint2* p, uint2 v) {
-  asm volatile("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], a;\n\t}" ::"l"(p),
-               "r"(v.x), "r"(v.y)
-               : "memory");
+  asm volatile(
+      "{\n\t.reg .b64 a;\n\tmov.b64 a, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], a;\n\t}" ::"l"(p),
+      "r"(v.x), "r"(v.y)
+      : "memory");
 }
 __device__ __forceinline__ uint2 ld_pkt2(const uint2* p) {
   uint2 v;
@@ -186,6 +204,7 @@ __device__ __forceinline__ bool wv_wait(const int* p, int need, WaveShared* sh) 
   if (__all_sync(0xffffffffu, ld_cta(p) >= need)) return true;
   const unsigned long long t0 = wv_ns();
   for (int it = 1; it < WV_MAX_TRIES; ++it) {
+    __nanosleep(20);  // (a polling warp takes issue slots from the sweeps)
     if (__all_sync(0xffffffffu, ld_cta(p) >= need)) return true;
     if ((it & 255) == 0 &&
         __any_sync(0xffffffffu, ld_cta(&sh->abort) != 0 || wv_ns() - t0 > WV_WAIT_NS))
@@ -195,44 +214,82 @@ __device__ __forceinline__ bool wv_wait(const int* p, int need, WaveShared* sh) 
   return false;
 }
 
-// x / n for the neighbour counts n = 1..4, correctly rounded: an exact
-// scaling for the powers of two, and for 3 the quotient by the rounded
-// reciprocal with Markstein's correction (IBM J. Res. Dev. 34, 1990), which
-// is correctly rounded where the remainder is exact -- |x| >= 2^-100 here;
-// compared with the division over every such float.  Smaller |x| divides.
-__device__ __forceinline__ float div_count(float x, int n) {
-  const float r = n == 4 ? 0.25f : n == 3 ? 1.0f / 3.0f : n == 2 ? 0.5f : 1.0f;
-  float q = x * r;
-  if (n == 3) {
-    const float t = fabsf(x);
-    const float q3 = __fmaf_rn(__fmaf_rn(-3.0f, q, x), r, q);
-    if (t >= 0x1p-100f && t <= 3.402823466e38f)
-      q = q3;
-    else if (t > 0.0f && t < 0x1p-100f)
-      q = x / 3.0f;
+// Per flag byte: the faces' fluid bits as floats, the neighbour count and its
+// rounded reciprocal (0 on cells the sweeps leave alone).  A step reads its
+// cell's entry a step ahead, so it has no branch and decodes nothing.
+struct __align__(16) WaveCoef {
+  float W, E, S, N, n, r, pad[2];
+};
+__device__ __forceinline__ void wv_fill_coef(WaveCoef* lut) {
+  for (int f = threadIdx.x - 1; f < 64; f += blockDim.x - 1) {  // (not by thread 0)
+    WaveCoef c = {};
+    if ((f & (F_FLUID | F_INTERIOR)) == (F_FLUID | F_INTERIOR) && (f & 15)) {
+      c.W = fbit(f, F_W);
+      c.E = fbit(f, F_E);
+      c.S = fbit(f, F_S);
+      c.N = fbit(f, F_N);
+      c.n = c.W + c.E + c.S + c.N;
+      c.r = 1.0f / c.n;
+    }
+    lut[f] = c;
   }
+}
+// x / n, n = 1..4, r = 1 / n rounded: the quotient by the reciprocal with
+// Markstein's correction (IBM J. Res. Dev. 34, 1990), whose remainder is
+// exact for every float and these n; the remainder is taken as n q - x so
+// that a zero keeps its sign, and an infinity keeps its first quotient.
+// Equal to the division for all 2^32 floats and each n (checked on the host).
+__device__ __forceinline__ float div_count(float x, float n, float r) {
+  float q = x * r;
+  const float e = __fmaf_rn(n, q, -x);
+  asm("{\n\t.reg .pred p;\n\t.reg .f32 a;\n\tabs.f32 a, %2;\n\tsetp.lt.f32 p, a, 0f7F800000;\n\t"
+      "@p fma.rn.f32 %0, %1, %3, %0;\n\t}"
+      : "+f"(q)
+      : "f"(e), "f"(x), "f"(-r));
   return q;
 }
-__device__ __forceinline__ float wv_bit(unsigned f, unsigned b) { return (f & b) ? 1.0f : 0.0f; }
-__device__ __forceinline__ bool wv_active(unsigned f) {
-  return (f & (F_FLUID | F_INTERIOR)) == (F_FLUID | F_INTERIOR) && (f & 15u) != 0;
+// x = fma(c, y, x), x = x + y, m = max(m, |y|) where r > 0, else unchanged (a
+// predicated instruction instead of a select behind it in the serial chain).
+__device__ __forceinline__ void fma_if(float& x, float c, float y, float r) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %3, 0f00000000;\n\t@p fma.rn.f32 %0, %1, %2, %0;\n\t}"
+      : "+f"(x)
+      : "f"(c), "f"(y), "f"(r));
 }
-constexpr unsigned WV_FULL = F_W | F_E | F_S | F_N | F_FLUID | F_INTERIOR;
+__device__ __forceinline__ void add_if(float& x, float y, float r) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %2, 0f00000000;\n\t@p add.rn.f32 %0, %0, %1;\n\t}"
+      : "+f"(x)
+      : "f"(y), "f"(r));
+}
+__device__ __forceinline__ void max_if(float& m, float y, float r) {
+  asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %2, 0f00000000;\n\t@p max.f32 %0, %0, %1;\n\t}"
+      : "+f"(m)
+      : "f"(fabsf(y)), "f"(r));
+}
+// The column that lane 0 of a strip would be at in step 0, but for the sweeps'
+// offsets (<= 0): lane 31 of the strip below is 31 columns behind its lane 0,
+// so this shift by b makes its chunks of columns the ones received here.
+__device__ __forceinline__ int wv_lead(int b) { return (b & (WV_C - 1)) - WV_C; }
 
 // One sweep (warp w of the block, sweep t of the solve) of task (b, g).
-// A0: U (SOR) or the solution; A1: V or the right-hand side; A2: p.  Ring row
-// q of a field holds grid row i0 + q - WV_G.
-template <bool GS>
-__device__ void wv_sweep(const WaveArgs& a, WaveShared* sh, float* A0, float* A1, float* A2,
-                         const uint8_t* F, int b, int g, int w, int Gt, int nchunks, unsigned tag) {
+// D1: the damping is 1 (its product is then the factor itself).
+//
+// Every step treats its cell alike, active or not, on the grid or off it:
+// predicates leave inactive cells as they are, the coefficients are 0 or 1 (so
+// each fused multiply-add rounds as the reference's product and sum), and the
+// ring holds zero coefficients in the columns before the first and past the
+// last, so lanes there change nothing.  A second body without coefficients
+// for chunks of full cells was measured slower than this one alone (chunks of
+// 8: 20x2046, one sweep, 199 against 163 us; 2048^2, 200 sweeps, 2.56 against
+// 2.49 ms): choosing costs more per chunk than it saves, and a strip's first
+// and last 33 columns, where the wave enters the next strip, are never full.
+template <bool GS, bool D1>
+__device__ __forceinline__ void wv_sweep(const WaveArgs& a, WaveShared* sh, const char* lut,
+                                         char* ring, int b, int g, int w, int Gt, int nchunks,
+                                         unsigned tag) {
+  using R = WaveRing<GS>;
+  constexpr int RB = 4 * WV_W;  // bytes of a ring row
   const int lane = threadIdx.x & 31;
-  const int q = WV_G - w + lane;
-  float* r0 = A0 + q * WV_W;       // own row
-  float* r0n = r0 + WV_W;          // row i + 1
-  float* r0s = r0 - WV_W;          // row i - 1 (GS, lane 0)
-  float* r1 = A1 + q * WV_W;
-  float* r2 = GS ? nullptr : A2 + q * WV_W;
-  const uint8_t* rf = F + q * WV_FP;
+  const int row = (WV_G - w + lane) * RB;
   const int t = a.t0 + g * a.G + w;
   const float prog_t = (float)t / (float)a.iters;
   const float rel = GS ? a.relax0 : a.relax0 - (a.relax0 - a.relax1) * prog_t;  // fluid.go:169-170
@@ -242,17 +299,26 @@ __device__ void wv_sweep(const WaveArgs& a, WaveShared* sh, float* A0, float* A1
   const size_t in_at = ((size_t)(b - 1) * 2 * a.G + slot) * a.P;
   const size_t out_at = ((size_t)b * 2 * a.G + slot) * a.P;
   const uint4* in4 = (const uint4*)a.pkt + in_at;
-  uint4* out4 = (uint4*)a.pkt + out_at;
   const uint2* in2 = (const uint2*)a.pkt + in_at;
-  uint2* out2 = (uint2*)a.pkt + out_at;
-  const bool recv = b > 0, send = b + 1 < a.B && b != a.stall && lane == 31;
+  const bool recv = b > 0, send = b + 1 < a.B && b != a.stall;
   float mx = 0.0f;
   // v0: V[i][j], updated by (i, j-1) (SOR); the old P[i][j] (GS).  ue: the
-  // east face after the last step (SOR); the last step's new P (GS).
-  float v0 = 0.0f, ue = 0.0f;
+  // last step's new P (GS).  shv: the lower lane's east face after the last
+  // step (SOR), its new P (GS).
+  float v0 = 0.0f, ue = 0.0f, shv = 0.0f;
   float n1 = 0.0f, n2 = 0.0f, n3 = 0.0f, west = 0.0f;  // the next step's inputs
-  unsigned nf = 0;
-  int s = -2 * (w + 1);  // the chunk's first step
+  float4 k4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);      // its coefficients
+  float2 k2 = make_float2(0.0f, 0.0f);
+  unsigned nf = 0;                     // the coefficient offset of the step after it
+  // The chunk's first step.  The first chunk is the one with step -1, in
+  // which lane 0 picks up V[i][0].
+  int s = wv_lead(b) - 2 * (w + 1);
+  const int n0 = (-1 - s) / WV_C;
+  s += n0 * WV_C;
+  int j4 = 4 * (s - lane);             // 4 x the step's column
+  // Byte offsets in the ring of the step's cell and of the next two columns'.
+  int at0 = row | (j4 & (RB - 4)), at1 = row | ((j4 + 4) & (RB - 4)), at2 = 0;
+  auto F = [&](int at) -> float& { return *reinterpret_cast<float*>(ring + at); };
   uint4 pk = make_uint4(0, 0, 0, tag - 1);
   auto poll = [&](int c) {
     if (GS) {
@@ -263,20 +329,24 @@ __device__ void wv_sweep(const WaveArgs& a, WaveShared* sh, float* A0, float* A1
       pk = ld_pkt(in4 + c);
     }
   };
-  auto fetch = [&](int j) {  // inputs of column j
-    const int c = j & WV_M, cn = (j + 1) & WV_M;
-    n1 = r0n[c];                       // U[i+1][j]; the old P[i+1][j]
-    n2 = GS ? r0[cn] : r1[cn];         // V[i][j+1]; the old P[i][j+1]
-    n3 = GS ? r1[c] : r2[c];           // p; the right-hand side
-    nf = rf[c];
+  // The inputs of the column at c, the next column at cn.
+  auto fetch = [&](int c, int cn) {
+    n1 = F(c + RB);                             // U[i+1][j]; the old P[i+1][j]
+    n2 = GS ? F(cn) : F(cn + 4 * R::O1);        // V[i][j+1]; the old P[i][j+1]
+    n3 = GS ? F(c + 4 * R::O1) : F(c + 4 * R::O2);  // p; the right-hand side
+  };
+  auto coef = [&] {
+    k4 = *reinterpret_cast<const float4*>(lut + nf);
+    k2 = *reinterpret_cast<const float2*>(lut + nf + 16);
   };
   if (recv && lane < WV_C && (unsigned)(s + lane) < (unsigned)NY) poll(s + lane);
-  for (int n = 0; n < nchunks; ++n, s += WV_C) {
-    if (w == 0) {
-      if (!wv_wait(&sh->loaded, min(s + WV_C + 2, a.P), sh)) return;
-    } else {
-      if (!wv_wait(&sh->prog[w - 1], n + 1, sh)) return;
-    }
+  // The progress of the sweep below (of the loader, for the first sweep) is
+  // read in the middle of a chunk for the next one.
+  const int* word = w ? &sh->prog[w - 1] : &sh->loaded;
+  int seen = 0;
+  for (int n = n0; n < nchunks; ++n, s += WV_C) {
+    const int need = w ? n + 1 : min(s + WV_C + 2, a.P + WV_PAST);
+    if (!__all_sync(0xffffffffu, seen >= need) && !wv_wait(word, need, sh)) return;
     if (recv) {
       // The chunk's packets from the strip below: the west values of this
       // sweep's lowest row, and that neighbour row's other values, which
@@ -302,91 +372,96 @@ __device__ void wv_sweep(const WaveArgs& a, WaveShared* sh, float* A0, float* A1
         }
       }
       if (mine) {
-        const int ql = (WV_G - w) * WV_W + (c & WV_M);
+        const int d = (WV_G - w) * RB | ((4 * c) & (RB - 4));
         if (GS) {
-          A0[ql - WV_W] = __uint_as_float(pk.x);
+          F(d - RB) = __uint_as_float(pk.x);
         } else {
-          A0[ql] = __uint_as_float(pk.x);
+          F(d) = __uint_as_float(pk.x);
           if (w + 1 < Gt) {
-            A1[ql - WV_W] = __uint_as_float(pk.y);
-            A2[ql - WV_W] = __uint_as_float(pk.z);
+            F(d + 4 * R::O1 - RB) = __uint_as_float(pk.y);
+            F(d + 4 * R::O2 - RB) = __uint_as_float(pk.z);
           }
         }
       }
+      west = __uint_as_float(pk.x);  // (lane 0's is the first step's)
       __syncwarp();
       if (lane < WV_C && (unsigned)(c + WV_C) < (unsigned)NY) poll(c + WV_C);
+    } else {
+      west = F(at0 - (GS ? RB : 0));
     }
-    if (n == 0) fetch(s - lane);
-    if (lane == 0) west = GS ? r0s[s & WV_M] : r0[s & WV_M];
-    auto step = [&](int k, bool edge) {
-      const int j = s + k - lane;
-      const bool in = !edge || (unsigned)j < (unsigned)NY;
-      float wv = __shfl_up_sync(0xffffffffu, ue, 1);
-      if (lane == 0) wv = west;
+    if (n == n0) {
+      fetch(at0, at1);
+      nf = __float_as_uint(F(at0 + 4 * R::OF));
+      coef();
+      nf = __float_as_uint(F(at1 + 4 * R::OF));
+    }
+#pragma unroll
+    for (int k = 0; k < WV_C; ++k) {
+      const float wv = lane == 0 ? west : shv;
       const float x1 = n1, x2 = n2, x3 = n3;
-      const unsigned fl = in ? nf : 0u;
-      fetch(j + 1);
-      if (lane == 0 && k + 1 < WV_C) west = (GS ? r0s : r0)[(j + 1) & WV_M];
-      const bool full = __all_sync(0xffffffffu, fl == WV_FULL);
-      const int c = j & WV_M;
+      const float4 c4 = k4;
+      const float2 c2 = k2;
+      at2 = row | ((j4 + 8) & (RB - 4));
+      fetch(at1, at2);
+      if (k + 1 < WV_C) west = F(at1 - (GS ? RB : 0));
+      coef();
+      nf = __float_as_uint(F(at2 + 4 * R::OF));
+      if (k == WV_C / 2) seen = ld_cta(word);
       if (GS) {
         float out = v0;
-        if (full) {
-          const float lap = (wv - v0) + (x1 - v0) + (ue - v0) + (x2 - v0);
-          out = v0 + -(x3 - lap) * 0.25f * rel;
-        } else if (wv_active(fl)) {
-          const float lap = wv_bit(fl, F_W) * (wv - v0) + wv_bit(fl, F_E) * (x1 - v0) +
-                            wv_bit(fl, F_S) * (ue - v0) + wv_bit(fl, F_N) * (x2 - v0);
-          out = v0 + div_count(-(x3 - lap), __popc(fl & 15u)) * rel;
-        }
-        if (in) r0[c] = out;
-        if (send && in) st_pkt2(out2 + j, make_uint2(__float_as_uint(out), tag));
+        const float lap =
+            c4.x * (wv - v0) + c4.y * (x1 - v0) + c4.z * (ue - v0) + c4.w * (x2 - v0);
+        add_if(out, div_count(-(x3 - lap), c2.x, c2.y) * rel, c2.y);
+        shv = __shfl_up_sync(0xffffffffu, out, 1);
+        F(at0) = out;
         ue = out;
         v0 = x2;
       } else {
         const float div = x1 - wv + x2 - v0;
         float un = wv, en = x1, vn = v0, tn = x2, pn = x3;
-        if (full) {
-          mx = fmaxf(mx, fabsf(div));
-          float pp = -div * 0.25f;
-          pp *= rel;
-          pp *= damping;
-          pn = x3 + cp * pp;
-          un = wv - pp;
-          en = x1 + pp;
-          vn = v0 - pp;
-          tn = x2 + pp;
-        } else if (wv_active(fl)) {
-          mx = fmaxf(mx, fabsf(div));
-          float pp = div_count(-div, __popc(fl & 15u));
-          pp *= rel;
-          pp *= damping;
-          pn = x3 + cp * pp;
-          un = wv - wv_bit(fl, F_W) * pp;
-          en = x1 + wv_bit(fl, F_E) * pp;
-          vn = v0 - wv_bit(fl, F_S) * pp;
-          tn = x2 + wv_bit(fl, F_N) * pp;
-        }
-        if (in) {
-          r0[c] = un;
-          r1[c] = vn;
-          r2[c] = pn;
-        }
-        if (send && in)
-          st_pkt(out4 + j, make_uint4(__float_as_uint(en), __float_as_uint(vn), __float_as_uint(pn), tag));
-        ue = en;
+        float pp = div_count(-div, c2.x, c2.y);
+        pp *= rel;
+        if (!D1) pp *= damping;
+        fma_if(en, c4.y, pp, c2.y);
+        // The next step's west value sets off before this step's stores.
+        shv = __shfl_up_sync(0xffffffffu, en, 1);
+        fma_if(tn, c4.w, pp, c2.y);
+        fma_if(un, -c4.x, pp, c2.y);
+        fma_if(vn, -c4.z, pp, c2.y);
+        add_if(pn, cp * pp, c2.y);
+        max_if(mx, div, c2.y);
+        F(at0) = un;
+        F(at0 + RB) = en;  // (the lane above stores its own value there one step later)
+        F(at0 + 4 * R::O1) = vn;
+        F(at0 + 4 * R::O2) = pn;
         v0 = tn;
       }
-    };
-    if (s - 31 >= 0 && s + WV_C <= NY) {
-#pragma unroll
-      for (int k = 0; k < WV_C; ++k) step(k, false);
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < WV_C; ++k) step(k, true);
+      at0 = at1;
+      at1 = at2;
+      j4 += 4;
+    }
+    __syncwarp();
+    // Lane 31's columns of this chunk go to the strip above (read before the
+    // chunk is reported, after which the ring may be refilled).
+    const int cs = s - 31 + lane;
+    const bool out = send && lane < WV_C && (unsigned)cs < (unsigned)NY;
+    uint4 x = make_uint4(0, 0, 0, tag);
+    if (out) {
+      const int d = (WV_G - w + 31) * RB | ((4 * cs) & (RB - 4));
+      x.x = __float_as_uint(F(d + (GS ? 0 : RB)));
+      if (!GS) {
+        x.y = __float_as_uint(F(d + 4 * R::O1));
+        x.z = __float_as_uint(F(d + 4 * R::O2));
+      }
     }
     __syncwarp();
     if (lane == 0) st_cta(&sh->prog[w], n + 1);
+    if (out) {
+      if (GS)
+        st_pkt2((uint2*)a.pkt + out_at + cs, make_uint2(x.x, tag));
+      else
+        st_pkt((uint4*)a.pkt + out_at + cs, x);
+    }
   }
   if (!GS) {
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
@@ -394,26 +469,27 @@ __device__ void wv_sweep(const WaveArgs& a, WaveShared* sh, float* A0, float* A1
   }
 }
 
-// Copies 32 ring columns (from column c) of the rows [q0, q1) of a field
-// whose ring row q is grid row i0 + q - WV_G; rows outside the grid, and
-// everything when !data, become zeros.
-template <typename T>
-__device__ __forceinline__ void wv_load_rows(T* ring, int pitch, const T* src, int q0, int q1, int i0,
+// Copies 32 columns (from column c) of grid rows [i, i + n) of a field to ring
+// row q on, 8 lanes a row; rows outside the grid, and everything when !data,
+// become zeros.
+__device__ __forceinline__ void wv_load_rows(float* ring, int q, const float* src, int i, int n,
                                              int c, int NX, int P, bool data) {
-  constexpr int PER = 16 / sizeof(T), SEG = 32 / PER;
-  const int lane = threadIdx.x & 31;
-  for (int it = lane; it < (q1 - q0) * SEG; it += 32) {
-    const int q = q0 + it / SEG, e = (it % SEG) * PER;
-    const int i = i0 + q - WV_G;
-    const bool in = data && i >= 0 && i < NX;
-    wv_copy16(ring + q * pitch + (c & WV_M) + e, in ? src + (size_t)i * P + c + e : src, in);
+  const int lane = threadIdx.x & 31, r0 = lane >> 3, e = c + (lane & 7) * 4;
+  float* d = ring + (q + r0) * WV_W + (e & WV_M);
+  const float* p = src + (ptrdiff_t)(i + r0) * P + e;
+  i += r0;
+#pragma unroll 4
+  for (int r = r0; r < n; r += 4, i += 4, d += 4 * WV_W, p += 4 * (ptrdiff_t)P) {
+    const bool in = data && (unsigned)i < (unsigned)NX;
+    wv_copy16(d, in ? p : src, in);
   }
 }
 
 // The loader warp: 32 columns at a time, as far ahead as the ring has room.
 template <bool GS>
-__device__ void wv_loader(const WaveArgs& a, WaveShared* sh, float* A0, float* A1, float* A2,
-                          uint8_t* F, int b, int g, unsigned tag) {
+__device__ void wv_loader(const WaveArgs& a, WaveShared* sh, float* ring, int b, int g, int Gt,
+                          int nchunks, unsigned tag) {
+  using R = WaveRing<GS>;
   const int lane = threadIdx.x & 31;
   const int i0 = 1 + 32 * b, lo = WV_G - (a.G - 1), hi = WV_G + 32;
   const float* s0 = g ? a.dst[0] : a.src[0];
@@ -436,20 +512,55 @@ __device__ void wv_loader(const WaveArgs& a, WaveShared* sh, float* A0, float* A
     __syncwarp();
     if (lane == 0) st_cta(&sh->loaded, cols);
   };
+  // Flag bytes of the next 32 columns (4 a lane), read a block ahead.
+  constexpr int NF = (WV_A1 * 8 + 31) / 32;
+  unsigned f[NF];
+  auto flags = [&](int c) {
+    const int r0 = lane >> 3, e = c + (lane & 7) * 4;
+    int i = i0 + lo - WV_G + r0;
+#pragma unroll
+    for (int m = 0; m < NF; ++m, i += 4)
+      f[m] = lo + r0 + 4 * m < hi && c < a.P && (unsigned)i < (unsigned)a.NX
+                 ? __ldg(reinterpret_cast<const unsigned*>(a.flags + (size_t)i * a.P + e))
+                 : 0u;
+  };
+  // Their coefficient offsets, into the ring.
+  auto offsets = [&](int c) {
+    const int r0 = lane >> 3;
+    float* d = ring + R::OF + (lo + r0) * WV_W + (c & WV_M) + (lane & 7) * 4;
+    constexpr unsigned SZ = sizeof(WaveCoef);
+#pragma unroll
+    for (int m = 0; m < NF; ++m, d += 4 * WV_W)
+      if (lo + r0 + 4 * m < hi)
+        *reinterpret_cast<uint4*>(d) =
+            make_uint4((f[m] & 63u) * SZ, (f[m] >> 8 & 63u) * SZ, (f[m] >> 16 & 63u) * SZ,
+                       (f[m] >> 24 & 63u) * SZ);
+  };
+  // Zero coefficients before column 0 (the ring's last blocks) and in the
+  // WV_PAST columns after the row.
+  flags(a.P);
+  for (int c = WV_W - WV_BEFORE; c < WV_W; c += 32) offsets(c);
+  flags(0);
+  // Chunks after which no lane of the last sweep is before column 0.
+  const int inside = (32 - wv_lead(b) + 2 * Gt + WV_C - 1) / WV_C;
   bool ok = true;
-  int pending = 0;  // columns copied but not yet published (0: none)
-  for (int c = 0; c < a.P && ok; c += 32) {
-    const int room = c + 32 - WV_W;
-    bool now = (room <= 0 || __all_sync(0xffffffffu, ld_cta(&sh->stored) >= room)) && ready(c);
+  int copied = 0, known = 0;  // columns issued, columns published
+  for (int c = 0; c < a.P + WV_PAST && ok; c += 32) {
+    // A block's ring columns are free once the storer has drained them; the
+    // last blocks' first columns once the sweeps have left them.
+    const bool first = c < WV_W;
+    const int* word = first ? &sh->prog[Gt - 1] : &sh->stored;
+    const int room = !first ? c + 32 - WV_W : c < WV_W - WV_BEFORE ? 0 : min(inside, nchunks);
+    const bool now = (room <= 0 || __all_sync(0xffffffffu, ld_cta(word) >= room)) &&
+                     (c >= a.P || ready(c));
     if (!now) {
-      if (pending) {
+      if (known < copied) {
         asm volatile("cp.async.wait_all;" ::: "memory");
-        publish(pending);
-        pending = 0;
+        publish(known = copied);
       }
-      if (room > 0) ok = wv_wait(&sh->stored, room, sh);
+      if (room > 0) ok = wv_wait(word, room, sh);
       const unsigned long long t0 = wv_ns();
-      for (int it = 1; ok && !ready(c); ++it)
+      for (int it = 1; ok && c < a.P && !ready(c); ++it)
         if ((it & 63) == 0 &&
             (it >= WV_MAX_TRIES ||
              __any_sync(0xffffffffu, ld_cta(&sh->abort) != 0 || wv_ns() - t0 > WV_WAIT_NS))) {
@@ -458,51 +569,55 @@ __device__ void wv_loader(const WaveArgs& a, WaveShared* sh, float* A0, float* A
         }
       if (!ok) break;
     }
-    if (GS) {
+    if (c >= a.P) {
+      // (no fields past the row)
+    } else if (GS) {
       // Row 0 and the rows below it hold zeros (strip 0); the right-hand side
       // and the flags reach down to the last sweep's rows.
-      wv_load_rows(A0, WV_W, s0, b ? WV_G : 0, hi + 1, i0, c, a.NX, a.P, g > 0);
-      wv_load_rows(A1, WV_W, s1, lo, hi, i0, c, a.NX, a.P, true);
+      const int q0 = b ? WV_G : WV_G - a.G;
+      wv_load_rows(ring, q0, s0, i0 + q0 - WV_G, hi + 1 - q0, c, a.NX, a.P, g > 0);
+      wv_load_rows(ring + R::O1, lo, s1, i0 + lo - WV_G, hi - lo, c, a.NX, a.P, true);
     } else {
-      wv_load_rows(A0, WV_W, s0, WV_G, hi + 1, i0, c, a.NX, a.P, true);
-      wv_load_rows(A1, WV_W, s1, WV_G, hi, i0, c, a.NX, a.P, true);
-      wv_load_rows(A2, WV_W, s2, WV_G, hi, i0, c, a.NX, a.P, true);
+      wv_load_rows(ring, WV_G, s0, i0, 33, c, a.NX, a.P, true);
+      wv_load_rows(ring + R::O1, WV_G, s1, i0, 32, c, a.NX, a.P, true);
+      wv_load_rows(ring + R::O2, WV_G, s2, i0, 32, c, a.NX, a.P, true);
     }
-    wv_load_rows(F, WV_FP, a.flags, lo, hi, i0, c, a.NX, a.P, true);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (pending) {
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-      publish(pending);
+    copied = c + 32;
+    offsets(c);
+    flags(c + 32);
+    if (copied - known > 64) {  // (up to three blocks in flight)
+      asm volatile("cp.async.wait_group 2;" ::: "memory");
+      publish(known = copied - 64);
     }
-    pending = c + 32;
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  if (pending) publish(pending);
+  if (known < copied) publish(copied);
 }
 
 // The storer warp: the group's final values, 32 columns at a time, once its
 // last sweep's topmost lane has passed them.
 template <bool GS>
-__device__ void wv_storer(const WaveArgs& a, WaveShared* sh, const float* A0, const float* A1,
-                          const float* A2, int b, int g, int Gt, int nchunks, unsigned tag,
-                          bool more) {
+__device__ void wv_storer(const WaveArgs& a, WaveShared* sh, const float* ring, int b, int g,
+                          int Gt, int nchunks, unsigned tag, bool more) {
+  using R = WaveRing<GS>;
   const int lane = threadIdx.x & 31;
   const int i0 = 1 + 32 * b;
   constexpr int NF = GS ? 1 : 3;
   const int first = GS ? 0 : 1;  // (GS: strip 0 also writes row 0's zeros)
   for (int c = 0; c < a.P; c += 32) {
     // Lane 31 passes column c + 31 in step c + 62.
-    const int need = min((c + 63 + 2 * Gt + WV_C - 1) / WV_C, nchunks);
+    const int need = min((c + 63 - wv_lead(b) + 2 * Gt + WV_C - 1) / WV_C, nchunks);
     if (!wv_wait(&sh->prog[Gt - 1], need, sh)) return;
 #pragma unroll
     for (int fd = 0; fd < NF; ++fd) {
-      const float* ring = fd == 0 ? A0 : fd == 1 ? A1 : A2;
+      const float* from = ring + (fd == 0 ? 0 : fd == 1 ? R::O1 : R::O2);
       float* dst = a.dst[fd];
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
         const int r = m * 4 + (lane >> 3), e = (lane & 7) * 4;
         const int q = WV_G - (Gt - 1) + r, i = i0 - (Gt - 1) + r, j = c + e;
-        const float4 v = *reinterpret_cast<const float4*>(ring + q * WV_W + (c & WV_M) + e);
+        const float4 v = *reinterpret_cast<const float4*>(from + q * WV_W + (c & WV_M) + e);
         if (i < first || i >= a.NX || j >= a.NY) continue;
         float* d = dst + (size_t)i * a.P + j;
         if (j + 4 <= a.NY) {
@@ -525,21 +640,20 @@ __device__ void wv_storer(const WaveArgs& a, WaveShared* sh, const float* A0, co
   }
 }
 
-template <bool GS>
-__global__ void __launch_bounds__((WV_G + 2) * 32) k_wave(WaveArgs a) {
-  extern __shared__ __align__(16) unsigned char wv_dyn[];
+template <bool GS, bool D1>
+__global__ void __launch_bounds__((WV_G + 2) * 32, 1) k_wave(WaveArgs a) {
+  extern __shared__ __align__(1024) unsigned char wv_dyn[];
   __shared__ WaveShared sh;
-  if (a.stop && *a.stop) return;  // (the same in every block)
-  float* A0 = reinterpret_cast<float*>(wv_dyn);
-  float* A1 = A0 + WV_A0 * WV_W;
-  float* A2 = A1 + WV_A1 * WV_W;
-  uint8_t* F = reinterpret_cast<uint8_t*>(GS ? A2 : A2 + WV_A1 * WV_W);
+  __shared__ WaveCoef lut[64];
+  float* ring = reinterpret_cast<float*>(wv_dyn);
   WaveCtl* ctl = a.ctl;
   const int warp = threadIdx.x >> 5;
+  // (Changed only after every block has left.)
   const unsigned epoch = ctl->epoch;
+  const int found = ctl->exit_sweep;
+  if (a.stop && *a.stop) return;  // (the same in every block)
   int nsw = a.nsweeps;
   bool copy = false;
-  const int found = ctl->exit_sweep;  // (changed only after every block has left)
   if (a.mode == WV_SPECULATE && a.t0 > 0 && found) nsw = 0;
   if (a.mode == WV_FINISH) {
     const bool rerun = found && found < a.iters;
@@ -549,11 +663,14 @@ __global__ void __launch_bounds__((WV_G + 2) * 32) k_wave(WaveArgs a) {
   const int ng = (nsw + a.G - 1) / a.G, ntasks = a.B * ng;
   if (threadIdx.x == 0) sh.abort = 0;
   int key = 0, before = 0;  // ticket decoding (thread 0): tasks with b + 2 g < key
-  for (;;) {
+  for (int turn = 0;; ++turn) {
     if (threadIdx.x == 0) {
       sh.b = -1;
-      const int tk = ntasks ? (int)atomicAdd(&ctl->ticket, 1u) : 0;
-      if (tk < ntasks && !sh.abort && !*(volatile int*)&ctl->fail) {
+      // (With a block per task, no block gets a second one.)
+      const int tk = ntasks && (turn == 0 || ntasks > (int)gridDim.x)
+                         ? (int)atomicAdd(&ctl->ticket, 1u)
+                         : ntasks;
+      if (tk < ntasks && !sh.abort && (turn == 0 || !*(volatile int*)&ctl->fail)) {
         for (;;) {
           const int g0 = max(0, (key - a.B + 2) / 2), g1 = min(ng - 1, key / 2);
           const int cnt = g1 - g0 + 1;
@@ -569,19 +686,22 @@ __global__ void __launch_bounds__((WV_G + 2) * 32) k_wave(WaveArgs a) {
       for (int w = 0; w < WV_G; ++w) sh.prog[w] = 0;
       sh.loaded = 0;
       sh.stored = 0;
+    } else if (turn == 0) {
+      wv_fill_coef(lut);
     }
     __syncthreads();
     const int b = sh.b, g = sh.g;
     if (b < 0) break;
     const int Gt = min(a.G, nsw - g * a.G);
-    const int nchunks = (a.NY + 31 + 2 * Gt + WV_C - 1) / WV_C;
+    const int nchunks = (a.NY + 31 - wv_lead(b) + 2 * Gt + WV_C - 1) / WV_C;
     const unsigned tag = epoch + 1u + (unsigned)g;
     if (warp == a.G)
-      wv_loader<GS>(a, &sh, A0, A1, A2, F, b, g, tag);
+      wv_loader<GS>(a, &sh, ring, b, g, Gt, nchunks, tag);
     else if (warp == a.G + 1)
-      wv_storer<GS>(a, &sh, A0, A1, A2, b, g, Gt, nchunks, tag, g + 1 < ng);
+      wv_storer<GS>(a, &sh, ring, b, g, Gt, nchunks, tag, g + 1 < ng);
     else if (warp < Gt)
-      wv_sweep<GS>(a, &sh, A0, A1, A2, F, b, g, warp, Gt, nchunks, tag);
+      wv_sweep<GS, D1>(a, &sh, reinterpret_cast<const char*>(lut),
+                       reinterpret_cast<char*>(wv_dyn), b, g, warp, Gt, nchunks, tag);
     __syncthreads();
   }
   if (copy) {
@@ -1038,26 +1158,34 @@ __global__ void k_mg_apply(float* __restrict__ U, float* __restrict__ V, float* 
 
 // ------------------------------------------------------------------ host side
 static size_t wave_smem(bool gs) {
-  return (size_t)WV_W * 4 * (WV_A0 + (gs ? 1 : 2) * WV_A1) + (size_t)WV_A1 * WV_FP;
+  return sizeof(float) * (gs ? WaveRing<true>::WORDS : WaveRing<false>::WORDS);
 }
 static int wave_strips(int NX, int G) { return (NX + G - 2 + 31) / 32; }
+
+// The kernel of a launch: the coarse solve, or the SOR with damping 1 or not.
+typedef void (*WaveKernel)(WaveArgs);
+static WaveKernel wave_kernel(bool gs, bool d1) {
+  return gs ? k_wave<true, true> : d1 ? k_wave<false, true> : k_wave<false, false>;
+}
 
 // Sets the pipeline kernels' shared-memory limit and counts the blocks the
 // current device holds at once (0: they cannot run).  Outside any capture.
 static int wave_blocks() {
-  int dev = 0, sms = 0, per[2] = {};
-  const int s0 = (int)wave_smem(false), s1 = (int)wave_smem(true), nt = (WV_G + 2) * 32;
-  const bool ok =
-      cudaGetDevice(&dev) == cudaSuccess &&
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-      cudaFuncSetAttribute(k_wave<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, s0) ==
-          cudaSuccess &&
-      cudaFuncSetAttribute(k_wave<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1) ==
-          cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0], k_wave<false>, nt, s0) == cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1], k_wave<true>, nt, s1) == cudaSuccess;
+  int dev = 0, sms = 0;
+  bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+  for (int k = 0; k < 3 && ok; ++k) {
+    const bool gs = k == 2;
+    WaveKernel fn = wave_kernel(gs, k == 1);
+    int per = 0;
+    ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)wave_smem(gs)) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, (WV_G + 2) * 32, wave_smem(gs)) ==
+             cudaSuccess &&
+         per > 0;
+  }
   cudaGetLastError();
-  return ok && per[0] > 0 && per[1] > 0 ? sms : 0;
+  return ok ? sms : 0;
 }
 
 // Bytes of the pipeline's buffers for an NX x NY grid (rows of P), and their
@@ -1116,10 +1244,7 @@ static void wave_launch(fg_fluid* f, WaveArgs a, bool gs, int t0, int n) {
   const long long tasks = (long long)a.B * ((n + a.G - 1) / a.G);
   const int blocks =
       a.mode == WV_FINISH ? f->wave_blocks : (int)std::min<long long>(tasks, f->wave_blocks);
-  if (gs)
-    k_wave<true><<<blocks, (a.G + 2) * 32, wave_smem(true), f->stream>>>(a);
-  else
-    k_wave<false><<<blocks, (a.G + 2) * 32, wave_smem(false), f->stream>>>(a);
+  wave_kernel(gs, a.damping == 1.0f)<<<blocks, (a.G + 2) * 32, wave_smem(gs), f->stream>>>(a);
   count(f);
 }
 
@@ -1163,7 +1288,7 @@ static void lexsor_solve(fg_fluid* f, int iters, float relax0, float relax1, flo
     pass(WV_SPECULATE);
     pass(WV_FINISH);
   } else {
-    pass(WV_PLAIN);
+    pass(WV_WLAIN);
   }
 }
 
@@ -1191,7 +1316,7 @@ static void launch_mg_coarse(fg_fluid* f, const int* stop, int cNX, int cNY, int
   a.P = cP;
   a.iters = 40;
   a.relax0 = 1.6f;
-  a.mode = WV_PLAIN;
+  a.mode = WV_WLAIN;
   a.stop = stop;
   a.stall = -1;
   wave_launch(f, a, true, 0, 40);
