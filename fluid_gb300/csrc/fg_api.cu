@@ -104,6 +104,14 @@ int alloc_dev(fg_fluid* f, float** p) {
   return FG_OK;
 }
 
+// The resident Jacobi solves' buffers (zeroed: no packet carries a live tag).
+int alloc_jres(fg_fluid* f, size_t n) {
+  if (!n) return FG_OK;
+  if (dev_malloc(&f->jres, n) != cudaSuccess) return FG_ERR_NOMEM;
+  CK(f, cudaMemsetAsync(f->jres, 0, n, f->stream), "jres");
+  return FG_OK;
+}
+
 int upload_field(fg_fluid* f, int k) {
   CK(f, cudaMemcpy2DAsync(f->d[k], sizeof(float) * f->P, f->hm[k], sizeof(float) * f->NY,
                           sizeof(float) * f->NY, f->NX, cudaMemcpyHostToDevice, f->stream),
@@ -474,6 +482,7 @@ int fg_create(int width, int height, float density, float h, const fg_params* pa
   if (dev_malloc((void**)&f->tile_done, sizeof(int) * ((size_t)jacobi_tile_count(f->NX, f->NY) + 1)) !=
       cudaSuccess)
     return bail(FG_ERR_NOMEM);
+  if ((rc = alloc_jres(f, jres_bytes_grid(f->NX, f->NY)))) return bail(rc);
   cudaMemsetAsync(f->pctl, 0, pctl_bytes(f->n_slots), f->stream);
   cudaMemsetAsync(f->ectl, 0, pctl_bytes(f->n_slots), f->stream);
   cudaMemsetAsync(f->dstats, 0, sizeof(DevStats), f->stream);
@@ -535,6 +544,7 @@ int fg_destroy(fg_fluid* f) {
   cudaFree(f->pctl);
   cudaFree(f->ectl);
   cudaFree(f->tile_done);
+  cudaFree(f->jres);
   if (f->image_pinned) cudaFreeHost(f->image_pinned);
   cudaFree(f->wave);
   for (int k = 0; k < 2; ++k) {
@@ -1878,6 +1888,7 @@ void batch_free(fg::BatchGeom* b) {
   cudaFree(b->cell_range);
   cudaFree(b->border_tiles);
   cudaFree(b->jac_tiles);
+  cudaFree(b->res_regions);
   cudaFree(b->src_scene);
   cudaFree(b->losses);
   delete b;
@@ -1953,6 +1964,74 @@ int batch_pack(fg_fluid* f) {
   }
   CK(f, cudaStreamSynchronize(f->stream), "batch pack");
   return FG_OK;
+}
+
+// Plans the batch's resident Jacobi solves: for each form, groups of whole
+// scenes (in the order jord: more sweeps first) whose regions fit the GPU at
+// once, evenly filled; the form whose groups' phases take least (measured per
+// phase, 3 us a launch), if that is less than the launches of 8 sweeps over
+// all started regions (2.4 us each and 6.2 us per 304 regions; 21 scenes of
+// 64^2-512^2: 8.7 us each).
+int batch_resident(fg_fluid* f, const std::vector<int>& jord) {
+  BatchGeom* b = f->batch;
+  JresForm forms[3];
+  jres_batch_forms(forms);
+  double best = 0.0;
+  for (int k = 0; k < (b->max_iters + kJacHalo - 1) / kJacHalo; ++k) {
+    int started = 0;
+    for (size_t s = 0; s < jord.size(); ++s)
+      if ((b->jac_iters[s] + kJacHalo - 1) / kJacHalo > k) started += b->jac_regions[s];
+    best += 2.4 + 6.2 * started / 304.0;
+  }
+  for (const JresForm& fm : forms) {
+    if (fm.cap <= 0) continue;
+    std::vector<int> size;
+    int total = 0, largest = 0;
+    for (int s : jord) {
+      const Grid& g = b->scenes[s].g;
+      size.push_back(span_count(g.NX, fm.rows) * span_count(g.NY, kJacRegionCols));
+      total += size.back();
+      largest = std::max(largest, size.back());
+    }
+    if (largest > fm.cap) continue;
+    const int n_groups = (total + fm.cap - 1) / fm.cap, want = (total + n_groups - 1) / n_groups;
+    std::vector<std::pair<int, int>> groups;
+    double us = 0.0;
+    int first = 0, held = 0;
+    for (size_t s = 0; s <= size.size(); ++s) {
+      if (s == size.size() || (held > 0 && (held + size[s] > fm.cap || held >= want))) {
+        groups.push_back({first, held});
+        first += held;
+        held = 0;
+        if (s == size.size()) break;
+      }
+      if (held == 0) us += 3.0 + fm.us * ((b->jac_iters[s] + kJacHalo - 1) / kJacHalo);
+      held += size[s];
+    }
+    if (us >= best) continue;
+    best = us;
+    b->res_form = fm.form;
+    b->res_groups = groups;
+    b->res_cap = 0;
+    for (const auto& gp : groups) b->res_cap = std::max(b->res_cap, gp.second);
+  }
+  if (!b->res_cap) return FG_OK;
+  int rows = 0;
+  for (const JresForm& fm : forms)
+    if (fm.form == b->res_form) rows = fm.rows;
+  std::vector<JRegion> rg;
+  for (int s : jord) {
+    const BScene& sc = b->scenes[s];
+    const int nty = span_count(sc.g.NX, rows), ntx = span_count(sc.g.NY, kJacRegionCols);
+    for (int ti = 0; ti < nty; ++ti)
+      for (int tj = 0; tj < ntx; ++tj)
+        rg.push_back(JRegion{sc.g.NX, sc.g.NY, sc.g.P, sc.iters, sc.off, ti * (rows - 2 * kJacHalo),
+                             tj * (kJacRegionCols - 2 * kJacHalo),
+                             span_own(ti, sc.g.NX, rows) | span_own(tj, sc.g.NY, kJacRegionCols) << 16,
+                             ntx, ti > 0, ti < nty - 1, tj > 0, tj < ntx - 1});
+  }
+  int rc = upload_table(f, &b->res_regions, rg);
+  return rc ? rc : alloc_jres(f, jres_bytes(0, b->res_cap, rows == 96 ? b->res_cap : 0));
 }
 
 int batch_check_member(fg_fluid* f, const fg_fluid* m, const fg_fluid* m0) {
@@ -2089,6 +2168,7 @@ int fg_batch_create(fg_fluid* const* scenes, int n, fg_fluid** out) {
     return bail(rc);
   b->n_border_tiles = (int)bt.size();
   b->n_jac_tiles = (int)jt.size();
+  if ((rc = batch_resident(f, jord))) return bail(rc);
   // Partial rows of the per-scene loss: one float pair per cell tile for the
   // block shape with the most tiles, plus the reserve partials_fit keeps.
   long long max_tiles = 0;

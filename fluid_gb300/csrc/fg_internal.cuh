@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/fluidgpu.h"
@@ -261,6 +262,20 @@ __host__ __device__ inline uint32_t span_own(int t, int n, int R) {
   return lo | hi << 8;
 }
 
+// A region of a batch: its scene's grid, place and sweeps, its window and
+// its neighbours (by their distance in the table).
+struct JRegion {
+  int NX, NY, P, iters;
+  long long off;  // element offset of the scene
+  int r0, c0;     // first row and column
+  uint32_t own;
+  int ntx;        // regions along the columns
+  int up, down, left, right;
+};
+
+// Regions a resident Jacobi solve's buffers are made for at most.
+constexpr int JRES_MAX_REGIONS = 512;
+
 struct BatchGeom {
   int n = 0;
   std::vector<BScene> scenes;
@@ -279,6 +294,11 @@ struct BatchGeom {
   // launch runs only the table's prefix of scenes that have started.
   std::vector<int> jac_iters, jac_regions;
   int max_iters = 0;
+  // Resident solves: every region, and groups (first region, regions) of
+  // whole scenes that are solved one after the other; res_cap the largest.
+  JRegion* res_regions = nullptr;
+  std::vector<std::pair<int, int>> res_groups;
+  int res_cap = 0, res_form = 0;
   int* src_scene = nullptr;  // device: scene of each source group
   double* losses = nullptr;  // device: per-scene loss of the last seed, then n floats 1 / L
 };
@@ -335,6 +355,7 @@ struct fg_fluid {
   int n_partials = 0;          // floats
   fg::DevStats* dstats = nullptr;
   void* pctl = nullptr;   // control block of the main Jacobi solve (k_pressure.cu PCtl)
+  void* jres = nullptr;  // resident Jacobi solves: epochs and packets (or none)
   int* tile_done = nullptr;  // dataflow Jacobi kernel: per-tile phase flags + item counter
   int stall_tile = -1;       // fault injection: a tile the dataflow kernel never publishes
   int jacobi_kernel = 0;     // FG_JACOBI_KERNEL_* of the last main solve (fg_stats)
@@ -473,6 +494,15 @@ void mg_free(fg_fluid* f);
 // buffer holding x.
 void init_jacobi_tma();
 int jacobi_tile_count(int NX, int NY);
+// Bytes of the resident solves' buffers for a grid, or for so many regions of
+// 4, 8 and 12 warps at once (0: none).
+size_t jres_bytes_grid(int NX, int NY);
+size_t jres_bytes(int regions4, int regions8, int regions12);
+struct JresForm {
+  int form, rows, cap;
+  float us;
+};
+void jres_batch_forms(JresForm (&out)[3]);
 cudaError_t launch_jacobi_solve(fg_fluid* f, void* ctl, const float* b, const float* bw, float* x0,
                                 float* x1, int iters);
 // Copies the last solve's potential to dst.

@@ -490,16 +490,16 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, unsigned parity) {
 // One sweep of a tile in registers, with the arithmetic of jacobi_tile;
 // buf alternates between consecutive sweeps (the row exchange is double
 // buffered, one barrier per sweep).
-template <bool OMEGA1>
+template <bool OMEGA1, int NW = NWARP>
 __device__ __forceinline__ void tile_sweep(float (&x)[RT][JT], const float (&w)[RT][JT],
                                            const float (&bw)[RT][JT], float om1,
-                                           float4 (&xch)[2][2][NWARP][32], int warp, int lane,
+                                           float4 (&xch)[2][2][NW][32], int warp, int lane,
                                            int buf) {
   xch[buf][0][warp][lane] = make_float4(x[0][0], x[0][1], x[0][2], x[0][3]);
   xch[buf][1][warp][lane] = make_float4(x[RT - 1][0], x[RT - 1][1], x[RT - 1][2], x[RT - 1][3]);
   __syncthreads();
   float4 u4 = warp > 0 ? xch[buf][1][warp - 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 d4 = warp < NWARP - 1 ? xch[buf][0][warp + 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 d4 = warp < NW - 1 ? xch[buf][0][warp + 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   float prev[JT] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
@@ -536,15 +536,15 @@ __device__ __forceinline__ void tile_sweep(float (&x)[RT][JT], const float (&w)[
 struct NoHook {
   __device__ __forceinline__ void operator()(int) const {}
 };
-template <bool OMEGA1, typename Hook = NoHook>
+template <bool OMEGA1, typename Hook = NoHook, int NW = NWARP>
 __device__ __forceinline__ void tile_sweeps(float (&x)[RT][JT], const float (&w)[RT][JT],
                                             const float (&bw)[RT][JT], float om1,
-                                            float4 (&xch)[2][2][NWARP][32], int warp, int lane,
+                                            float4 (&xch)[2][2][NW][32], int warp, int lane,
                                             Hook hook = Hook()) {
 #pragma unroll
   for (int sw = 0; sw < TMAX; ++sw) {
     hook(sw);
-    tile_sweep<OMEGA1>(x, w, bw, om1, xch, warp, lane, sw & 1);
+    tile_sweep<OMEGA1, NW>(x, w, bw, om1, xch, warp, lane, sw & 1);
   }
 }
 
@@ -1025,6 +1025,264 @@ __global__ void __launch_bounds__(TB_THREADS, 2)
   }
 }
 
+// ------------------------------------------------------------------ resident Jacobi
+// A whole fixed-count solve with every region in registers from the first
+// sweep to the last: one block per region (the placement of k_jacobi_rb:
+// span_count, span_own), all resident at once (a cooperative launch), 8
+// sweeps between exchanges.  Only the values that a neighbour's halo holds
+// leave a block: the 8 rows of its first and last owned warps and the 8
+// columns of lanes 2, 3 and 28, 29, written as 16-byte packets of three
+// values and a tag.  A packet is stored and read whole (one 128-bit access
+// each way) and its tag names the solve and the phase, so the receiver polls
+// the data itself: no fence, flag or grid barrier.  Two slots by phase
+// parity suffice: a neighbour writes phase p + 2 only after it has this
+// block's p + 1, sent after its p was read.  Same per-cell arithmetic as the
+// other kernels, the same bits.
+//
+// For grids whose regions fit the GPU at once.  Bound by the sweeps' own
+// latency (1.35 us per 8 sweeps for 4 warps, each alone on its scheduler:
+// 190 instructions a warp and sweep at half a one per cycle) and the packets'
+// flight (0.7 us).  With 8-warp regions the registers decide: 128 a thread
+// (two blocks an SM) spill and take 3.9 us, 190 take 3.0.  Barriers split
+// into arrive and wait around the inner rows measured slower (2.2 against
+// 1.35 us without exchange), as did the boundary rows computed first (1.41).
+constexpr int JP = (RT * JT + 2) / 3;        // packets of a thread's 8 x 4 cells
+constexpr int JROWS = 2 * JP * 32;           // a slot's row packets: first, last owned warp
+template <int NW>
+struct JSlot {
+  static constexpr int N = JROWS + 2 * NW * JP * 2;  // + the column packets: left, right lanes
+  static constexpr int PER = (N + 32 * NW - 1) / (32 * NW);  // a thread's share of the items
+};
+
+struct JResArgs {
+  float* x;                    // the solution
+  const float *W, *BW;
+  float om1;
+  int iters;
+  unsigned* epoch;             // per block: the tag its last solve ended on (all alike)
+  unsigned inc;                // the launch's phases (a batch: of its longest solve)
+  int count;                   // regions; the blocks past them only keep their epoch
+  uint4* pkt;                  // [region][parity][JSlot::N]
+  PCtl* ctl;
+  const JRegion* regions;      // batch: the launch's regions (nullptr: one grid)
+  Grid g;
+  int ntx, nty;
+  int last_launch;             // what ctl->last_launch reports
+  int* err;
+  int stall;                   // fault injection: a region that sends nothing
+};
+
+__device__ __forceinline__ void jst_pkt(uint4* p, float x, float y, float z, unsigned tag) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+      "mov.b128 t, {a, b};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "f"(x), "f"(y), "f"(z), "r"(tag)
+      : "memory");
+}
+__device__ __forceinline__ uint4 jld_pkt(const uint4* p) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.b128 t, [%4];\n\t"
+      "mov.b128 {a, b}, t;\n\tmov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
+}
+
+// MB: blocks per SM the registers are limited for.
+template <bool OMEGA1, int NW, bool BATCH, int MB>
+__global__ void __launch_bounds__(32 * NW, MB) k_jacobi_res(JResArgs a) {
+  using S = JSlot<NW>;
+  constexpr int NT = 32 * NW, R = NW * RT;
+  __shared__ float4 xch[2][2][NW][32];
+  __shared__ float stage[3 * S::N];
+  __shared__ int from[S::N];
+  __shared__ JRegion rg;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, id = blockIdx.x;
+  const unsigned epoch = a.epoch[id];
+  if (BATCH && id >= a.count) {
+    if (tid == 0) a.epoch[id] = epoch + a.inc;
+    return;
+  }
+  if (BATCH) {
+    if (tid == 0) rg = a.regions[id];
+  } else if (tid == 0) {
+    const int ty = id / a.ntx, tx = id - ty * a.ntx;
+    rg.NX = a.g.NX;
+    rg.NY = a.g.NY;
+    rg.P = a.g.P;
+    rg.iters = a.iters;
+    rg.off = 0;
+    rg.r0 = ty * (R - 2 * TMAX);
+    rg.c0 = tx * OJ;
+    rg.own = span_own(ty, a.g.NX, R) | span_own(tx, a.g.NY, RJ) << 16;
+    rg.ntx = a.ntx;
+    rg.up = ty > 0;
+    rg.down = ty < a.nty - 1;
+    rg.left = tx > 0;
+    rg.right = tx < a.ntx - 1;
+  }
+  __syncthreads();
+  const int gi0 = rg.r0 + warp * RT, gj = rg.c0 + lane * JT;
+  float x[RT][JT], w[RT][JT], bw[RT][JT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    float4 ww = make_float4(0.f, 0.f, 0.f, 0.f), bb = ww;
+    if (gi0 + r < rg.NX && gj < rg.P) {
+      const size_t c = (size_t)rg.off + (size_t)(gi0 + r) * rg.P + gj;
+      ww = *reinterpret_cast<const float4*>(a.W + c);
+      bb = *reinterpret_cast<const float4*>(a.BW + c);
+    }
+    w[r][0] = ww.x; w[r][1] = ww.y; w[r][2] = ww.z; w[r][3] = ww.w;
+    bw[r][0] = bb.x; bw[r][1] = bb.y; bw[r][2] = bb.z; bw[r][3] = bb.w;
+#pragma unroll
+    for (int q = 0; q < JT; ++q) {
+      x[r][q] = 0.0f;
+      if (gj + q >= rg.NY) {  // the pitch padding: outside the grid
+        w[r][q] = 0.0f;
+        bw[r][q] = 0.0f;
+      }
+    }
+  }
+  // Where each item the block receives lies, relative to its own slots
+  // (INT_MIN: not needed).  Items are numbered as a slot's packets: the rows
+  // above and below (all 32 lanes; the corners from the diagonal regions),
+  // then the columns left and right of the rows no halo covers.
+  for (int k = tid; k < S::N; k += NT) {
+    int at = INT_MIN;
+    if (k < JROWS) {
+      const int side = k / (JP * 32), rest = k - side * (JP * 32), l = rest & 31;
+      const int dx = l < 2 && rg.left ? -1 : l >= 30 && rg.right ? 1 : 0;
+      if (side ? rg.down : rg.up)
+        at = ((side ? rg.ntx : -rg.ntx) + dx) * 2 * S::N + (1 - side) * JP * 32 + rest - 28 * dx;
+    } else {
+      const int c = k - JROWS, side = c / (NW * JP * 2), wr = (c / (JP * 2)) % NW;
+      const bool covered = (wr == 0 && rg.up) || (wr == NW - 1 && rg.down);
+      if ((side ? rg.right : rg.left) && !covered)
+        at = (side ? 2 * S::N : -2 * S::N) + JROWS + (1 - side) * NW * JP * 2 +
+             (c - side * NW * JP * 2);
+    }
+    from[k] = at;
+  }
+  const bool up = rg.up, down = rg.down, left = rg.left, right = rg.right;
+  const int iters = rg.iters;
+  uint4* own_slot = a.pkt + (size_t)id * 2 * S::N;
+  const int nph = (iters + TMAX - 1) / TMAX;
+  bool fail = false;
+  for (int ph = 0; ph < nph; ++ph) {
+    const int ns = iters - ph * TMAX;
+    if (ns >= TMAX) {
+      tile_sweeps<OMEGA1, NoHook, NW>(x, w, bw, a.om1, xch, warp, lane);
+    } else {
+      for (int sw = 0; sw < ns; ++sw)
+        tile_sweep<OMEGA1, NW>(x, w, bw, a.om1, xch, warp, lane, sw & 1);
+    }
+    if (ph + 1 == nph) break;
+    const unsigned tag = epoch + 1u + (unsigned)ph;
+    uint4* slot = own_slot + (ph & 1) * S::N;
+    auto val = [&](int k) { return k < RT * JT ? x[k / JT][k % JT] : 0.0f; };
+    if (id != a.stall) {
+      // The rows of the first and last owned warps, for the regions above
+      // and below; the columns for those left and right.
+      if (warp == 1 && up) {
+#pragma unroll
+        for (int m = 0; m < JP; ++m)
+          jst_pkt(slot + m * 32 + lane, val(3 * m), val(3 * m + 1), val(3 * m + 2), tag);
+      }
+      if (warp == NW - 2 && down) {
+#pragma unroll
+        for (int m = 0; m < JP; ++m)
+          jst_pkt(slot + (JP + m) * 32 + lane, val(3 * m), val(3 * m + 1), val(3 * m + 2), tag);
+      }
+      const int cl = lane - 2, cr = lane - 28;  // 0, 1: a lane whose columns go left / right
+      const bool goes_l = (unsigned)cl < 2u && left, goes_r = (unsigned)cr < 2u && right;
+      if (goes_l || goes_r) {
+        uint4* d = slot + JROWS + ((goes_r ? NW : 0) + warp) * JP * 2 + (goes_r ? cr : cl);
+#pragma unroll
+        for (int m = 0; m < JP; ++m)
+          jst_pkt(d + m * 2, val(3 * m), val(3 * m + 1), val(3 * m + 2), tag);
+      }
+    }
+    // Receive: each thread polls its items into the staging area.
+    uint4 v[S::PER];
+    auto source = [&](int m) {
+      const int k = tid + NT * m;
+      return k < S::N ? from[k] : INT_MIN;
+    };
+    bool miss = false;
+#pragma unroll
+    for (int m = 0; m < S::PER; ++m) {
+      const int at = source(m);
+      v[m].w = tag;
+      if (at != INT_MIN) v[m] = jld_pkt(slot + at);
+    }
+#pragma unroll
+    for (int m = 0; m < S::PER; ++m) miss = miss || v[m].w != tag;
+    if (miss) {
+      const unsigned long long t0 = global_ns();
+      for (int it = 1; miss; ++it) {
+        miss = false;
+#pragma unroll
+        for (int m = 0; m < S::PER; ++m) {
+          if (v[m].w != tag) v[m] = jld_pkt(slot + source(m));
+          miss = miss || v[m].w != tag;
+        }
+        if ((it & 63) == 0 && (it >= MBAR_MAX_TRIES || global_ns() - t0 > MBAR_WAIT_NS)) break;
+      }
+      fail = miss;
+    }
+#pragma unroll
+    for (int m = 0; m < S::PER; ++m)
+      if (source(m) != INT_MIN) {
+        float* d = stage + 3 * (tid + NT * m);
+        d[0] = __uint_as_float(v[m].x);
+        d[1] = __uint_as_float(v[m].y);
+        d[2] = __uint_as_float(v[m].z);
+      }
+    if (__syncthreads_or(fail)) {
+      fail = true;
+      break;
+    }
+    const bool above = warp == 0 && up, below = warp == NW - 1 && down;
+    const bool lcol = lane < 2 && left, rcol = lane >= 30 && right;
+    if (above || below || lcol || rcol) {
+      const bool row = above || below;
+      const float* d =
+          stage + 3 * (row ? (below ? JP * 32 : 0) + lane
+                           : JROWS + ((rcol ? NW : 0) + warp) * JP * 2 + (rcol ? lane - 30 : lane));
+      const int step = 3 * (row ? 32 : 2);
+#pragma unroll
+      for (int k = 0; k < RT * JT; ++k) x[k / JT][k % JT] = d[(k / 3) * step + k % 3];
+    }
+  }
+  if (tid == 0) {
+    a.epoch[id] = epoch + a.inc;
+    if (fail) atomicExch(a.err, 1);
+    if (id == 0) {
+      a.ctl->sweeps = iters;
+      a.ctl->last_launch = a.last_launch;
+      a.ctl->sel = 0;
+    }
+  }
+  const int oi0 = rg.own & 255, oi1 = rg.own >> 8 & 255, oj0 = rg.own >> 16 & 255,
+            oj1 = rg.own >> 24;
+  if (lane * JT < oj0 || lane * JT >= oj1) return;
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    const int gi = gi0 + r;
+    if (warp * RT + r < oi0 || warp * RT + r >= oi1 || gi >= rg.NX || gj >= rg.NY) continue;
+    float* d = a.x + rg.off + (size_t)gi * rg.P + gj;
+    if (gj + JT <= rg.NY) {
+      *reinterpret_cast<float4*>(d) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < JT; ++q)
+        if (gj + q < rg.NY) d[q] = x[r][q];
+    }
+  }
+}
+
 // Final potential at cell c: the main iterate, plus the outer correction on
 // active cells when one ran (phi = phi + e, fluid.go's p accumulation aside).
 __device__ __forceinline__ float phi_final(const float* __restrict__ phi,
@@ -1358,6 +1616,7 @@ struct TmaDevice {
   int sms = 0;
   int flow_per_sm = 0;
   int batch_pf_per_sm = 0;  // blocks of kb_jacobi_pf per SM (0: the plain batch kernel runs)
+  int res_blocks[4] = {};   // blocks of k_jacobi_res's forms the device holds (0: none)
 };
 static TmaDevice g_tma_dev[kMaxContexts];
 static unsigned long long g_tma_key[kMaxContexts];
@@ -1419,6 +1678,22 @@ static bool encode_box_map(CUtensorMap* tm, const float* base, int rows, int pit
                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
+}
+
+// Forms of the resident solve: regions of 4, 8 and 12 warps, one to an SM (all
+// the registers they want), and of 8 warps two to an SM.
+enum { JRES_4 = 0, JRES_8 = 1, JRES_12 = 2, JRES_8X2 = 3 };
+static int res_warps(int form) { return form == JRES_4 ? 4 : form == JRES_12 ? 12 : 8; }
+typedef void (*ResKernel)(JResArgs);
+static ResKernel res_kernel(bool o1, bool batch, int form) {
+#define FG_RES1(NW, MB, B) (o1 ? k_jacobi_res<true, NW, B, MB> : k_jacobi_res<false, NW, B, MB>)
+#define FG_RES(NW, MB) (batch ? FG_RES1(NW, MB, true) : FG_RES1(NW, MB, false))
+  return form == JRES_4    ? FG_RES1(4, 2, false)  // (a batch has no use for it)
+         : form == JRES_8  ? FG_RES(8, 1)
+         : form == JRES_12 ? FG_RES(12, 1)
+                           : FG_RES(8, 2);
+#undef FG_RES
+#undef FG_RES1
 }
 
 // The current context's entry, or nullptr (no context identity, or more
@@ -1484,6 +1759,19 @@ void init_jacobi_tma() {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p2, kb_jacobi_pf<false>, TB_THREADS,
                                                       smem) == cudaSuccess)
       d->batch_pf_per_sm = p1 < p2 ? p1 : p2;
+    if (coop)
+      for (int form = 0; form < 4; ++form) {
+        int least = INT_MAX;
+        for (int v = 0; v < 4; ++v) {
+          int per = 0;
+          if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                  &per, res_kernel(v & 1, (v & 2) != 0, form), 32 * res_warps(form), 0) !=
+              cudaSuccess)
+            per = 0;
+          least = std::min(least, per);
+        }
+        d->res_blocks[form] = std::min(least, 2) * d->sms;
+      }
     cudaGetLastError();
     d->ready.store(true);
   });
@@ -1666,6 +1954,98 @@ static cudaError_t enqueue_jacobi(cudaStream_t st, const Grid& g, PCtl* ctl, con
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------- resident solves
+// Regions of a grid for the 4- and 8-warp forms.
+static int res_regions(int NX, int NY, int NW) {
+  const long long n = (long long)span_count(NX, NW * RT) * span_count(NY, RJ);
+  return n > JRES_MAX_REGIONS ? 0 : (int)n;
+}
+// Bytes of a handle's resident-solve buffers (epochs, then packets); 0 when
+// no form takes the grid.
+size_t jres_bytes(int regions4, int regions8, int regions12) {
+  const size_t n = 2 * std::max(std::max((size_t)regions4 * JSlot<4>::N, (size_t)regions8 * JSlot<8>::N),
+                                (size_t)regions12 * JSlot<12>::N);
+  return n ? JRES_MAX_REGIONS * sizeof(unsigned) + n * sizeof(uint4) : 0;
+}
+size_t jres_bytes_grid(int NX, int NY) {
+  return jres_bytes(res_regions(NX, NY, 4), res_regions(NX, NY, 8), res_regions(NX, NY, 12));
+}
+
+// The forms a batch may be solved in: rows of a region, regions at once, and
+// the measured time of 8 sweeps (us); 0 regions: unavailable.  (Outside any
+// capture.)
+void jres_batch_forms(JresForm (&out)[3]) {
+  init_jacobi_tma();
+  const TmaDevice* d = tma_device();
+  const bool ok = d && d->ready.load();
+  const int form[3] = {JRES_8, JRES_12, JRES_8X2};
+  const float us[3] = {3.0f, 4.1f, 6.2f};
+  for (int k = 0; k < 3; ++k) {
+    int cap = !ok ? 0 : form[k] == JRES_8X2 ? d->res_blocks[JRES_8X2]
+                                            : std::min(d->sms, d->res_blocks[form[k]]);
+    out[k] = JresForm{form[k], res_warps(form[k]) * RT, std::min(cap, JRES_MAX_REGIONS), us[k]};
+  }
+}
+
+static cudaError_t launch_res(cudaStream_t st, const JResArgs& a, bool o1, bool batch, int form,
+                              int blocks) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(32 * res_warps(form));
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, res_kernel(o1, batch, form), a);
+}
+
+// A fixed-count solve of one grid from x = 0 into x as one resident launch;
+// false (nothing launched) where its regions do not fit the GPU at once.
+static bool launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, const float* BW,
+                              float om1, int iters, int T, int stall) {
+  if (!f->jres) return false;
+  const TmaDevice* dv = tma_ready(f->stream);
+  if (!dv) return false;
+  int n[4];
+  for (int k = 0; k < 4; ++k) n[k] = res_regions(f->NX, f->NY, res_warps(k));
+  // 4 warps a region while each gets an SM of its own, else 8, one or two to
+  // an SM.
+  // The smallest regions that get an SM each; else two 8-warp regions an SM.
+  // Measured per 8 sweeps (us), against the launches or the dataflow kernel
+  // they replace: 4 warps 128^2 2.3 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
+  // 2.9 (4.4), 800^2 3.0 (6.6); 12 warps 1024x768 4.2 (7.4), 1200x800 4.1
+  // (9.4); 8 warps twice 1200^2 6.2 (11.0).  A larger form where a smaller
+  // one fits is slower (512x256: 2.4, 3.1, 4.2, 3.9).
+  int form = JRES_4;
+  while (form <= JRES_8X2 &&
+         !(n[form] > 0 && n[form] <= (form == JRES_8X2 ? dv->res_blocks[form]
+                                                       : std::min(dv->sms, dv->res_blocks[form]))))
+    ++form;
+  if (form > JRES_8X2) return false;
+  const int nw = res_warps(form);
+  JResArgs a = {};
+  a.x = x;
+  a.W = W;
+  a.BW = BW;
+  a.om1 = om1;
+  a.iters = iters;
+  a.inc = (unsigned)((iters + TMAX - 1) / TMAX);
+  a.epoch = static_cast<unsigned*>(f->jres);
+  a.pkt = reinterpret_cast<uint4*>(a.epoch + JRES_MAX_REGIONS);
+  a.ctl = ctl;
+  a.g = f->g;
+  a.ntx = span_count(f->NY, RJ);
+  a.nty = span_count(f->NX, nw * RT);
+  a.last_launch = (iters + T - 1) / T - 1;
+  a.err = &f->dstats->timeout;
+  a.stall = stall;
+  const bool ok = launch_res(f->stream, a, om1 == 0.0f, false, form, n[form]) == cudaSuccess;
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
 // A batch's solves: every scene runs its own sweep count, no early exit.
 static cudaError_t jacobi_solve_batch(fg_fluid* f, PCtl* ctl, const float* bw, float* x0,
                                       float* x1) {
@@ -1678,6 +2058,34 @@ static cudaError_t jacobi_solve_batch(fg_fluid* f, PCtl* ctl, const float* bw, f
   float om1 = 1.0f - om;
   const TmaDevice* dv = tma_ready(f->stream);
   const int pf_blocks = dv && dv->sms > 0 ? dv->batch_pf_per_sm * dv->sms : 0;
+  // Groups of scenes whose regions fit the GPU at once, each group's whole
+  // solve one resident launch.
+  if (f->jres && dv && bt->res_regions && bt->res_cap > 0 && dv->res_blocks[bt->res_form] >= bt->res_cap) {
+    JResArgs a = {};
+    a.x = x0;
+    a.W = f->wgt;
+    a.BW = bw;
+    a.om1 = om1;
+    a.ctl = ctl;
+    a.last_launch = L - 1;
+    a.err = &f->dstats->timeout;
+    a.stall = -1;
+    unsigned* epochs = static_cast<unsigned*>(f->jres);
+    uint4* pkts = reinterpret_cast<uint4*>(epochs + JRES_MAX_REGIONS);
+    bool ok = true;
+    for (const auto& gp : bt->res_groups) {  // (groups run in turn: they share the buffers)
+      a.regions = bt->res_regions + gp.first;
+      a.count = gp.second;
+      a.inc = (unsigned)((bt->max_iters + TMAX - 1) / TMAX);
+      a.epoch = epochs;
+      a.pkt = pkts;
+      ok = launch_res(f->stream, a, om1 == 0.0f, true, bt->res_form, bt->res_cap) == cudaSuccess;
+      if (!ok) break;
+      count(f);
+    }
+    if (ok) return cudaGetLastError();
+    cudaGetLastError();
+  }
   size_t sc = 0;  // scenes (in the table's order) started by launch k
   int n_act = 0;  // their regions: the prefix of the table launch k runs
   for (int k = 0; k < L; ++k) {
@@ -1715,7 +2123,20 @@ static cudaError_t jacobi_solve(fg_fluid* f, PCtl* ctl, const float* b, const fl
   const bool prof = f->profile && allow_exit;
   if (prof && (e = cudaEventRecord(f->prof_ev[0], f->stream)) != cudaSuccess) return e;
   int n = 0;
-  if (rinit)
+  const TmaDevice* dv = tma_ready(f->stream);
+  if (!rinit && !check && iters > 0 &&
+      launch_jacobi_res(f, ctl, x0, f->wgt, bw,
+                        1.0f - f->prm.jacobi_omega * f->prm.pressure_damping, iters, T,
+                        f->stall_tile)) {
+    // (Reported as the kernel that runs such a solve without the buffers.)
+    n = 1;
+    if (kind)
+      *kind = T < TMAX || iters < TMAX ? FG_JACOBI_KERNEL_SWEEP
+              : iters >= 2 * TMAX && jacobi_tile_count(f->NX, f->NY) >= dv->sms
+                  ? FG_JACOBI_KERNEL_DATAFLOW
+              : res_regions(f->NX, f->NY, 8) >= dv->sms ? FG_JACOBI_KERNEL_TMA
+                                                        : FG_JACOBI_KERNEL_SWEEP;
+  } else if (rinit)
     e = enqueue_jacobi(f->stream, f->g, ctl, b, bw, f->wgt, f->flags, x0, x1, iters, T,
                        f->prm.jacobi_omega * f->prm.pressure_damping, 0, f->prm.tolerance, &n,
                        f->phi, f->phi2, (const PCtl*)f->pctl, f->rhs_e, f->bwe);

@@ -118,7 +118,9 @@ typedef struct fg_stats {
  * tensor map); TMA the per-launch kernel fed by the tensor memory
  * accelerator; DATAFLOW the one cooperative launch that runs every full
  * 8-sweep phase (fixed sweep counts of at least 16 on grids of at least one
- * tile per SM). */
+ * tile per SM).  A fixed-count solve whose regions all fit the GPU at once
+ * runs as one launch that keeps them in registers, with the same result; it
+ * reports the value of its sweep count, depth and grid by the rules above. */
 #define FG_JACOBI_KERNEL_NONE 0
 #define FG_JACOBI_KERNEL_SWEEP 1
 #define FG_JACOBI_KERNEL_TMA 2
@@ -410,7 +412,8 @@ const char* fg_last_error(const fg_fluid* f);
  * fg_debug_stall_tile(f, t): the dataflow Jacobi kernel never publishes tile
  * t of the handle's solves, so the tiles that read it wait until their
  * bounded waits (about a second) give up; the step's fg_get_stats returns
- * FG_ERR_TIMEOUT.  With the reference's serial scheme, strip t of 32 rows
+ * FG_ERR_TIMEOUT; on smaller grids region t of the resident solve sends
+ * nothing to its neighbours.  With the reference's serial scheme, strip t of 32 rows
  * sends nothing to the next one, with the same result.  t < 0 disarms.
  * Changes the handle's captured graphs.
  * fg_debug_stall_tile(NULL, t): in later fg_project_noalloc calls, the
