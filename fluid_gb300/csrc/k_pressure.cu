@@ -490,14 +490,23 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, unsigned parity) {
 // One sweep of a tile in registers, with the arithmetic of jacobi_tile;
 // buf alternates between consecutive sweeps (the row exchange is double
 // buffered, one barrier per sweep).
-template <bool OMEGA1, int NW = NWARP>
+// The barrier of a tile's NW warps: the block's, or (OWN) a named one of
+// theirs alone in a block with other warps.
+template <int NW, bool OWN>
+__device__ __forceinline__ void tile_barrier() {
+  if (OWN)
+    asm volatile("barrier.cta.sync 1, %0;" ::"n"(32 * NW) : "memory");
+  else
+    __syncthreads();
+}
+template <bool OMEGA1, int NW = NWARP, bool OWN = false>
 __device__ __forceinline__ void tile_sweep(float (&x)[RT][JT], const float (&w)[RT][JT],
                                            const float (&bw)[RT][JT], float om1,
                                            float4 (&xch)[2][2][NW][32], int warp, int lane,
                                            int buf) {
   xch[buf][0][warp][lane] = make_float4(x[0][0], x[0][1], x[0][2], x[0][3]);
   xch[buf][1][warp][lane] = make_float4(x[RT - 1][0], x[RT - 1][1], x[RT - 1][2], x[RT - 1][3]);
-  __syncthreads();
+  tile_barrier<NW, OWN>();
   float4 u4 = warp > 0 ? xch[buf][1][warp - 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   float4 d4 = warp < NW - 1 ? xch[buf][0][warp + 1][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
   float prev[JT] = {u4.x, u4.y, u4.z, u4.w};
@@ -536,7 +545,7 @@ __device__ __forceinline__ void tile_sweep(float (&x)[RT][JT], const float (&w)[
 struct NoHook {
   __device__ __forceinline__ void operator()(int) const {}
 };
-template <bool OMEGA1, typename Hook = NoHook, int NW = NWARP>
+template <bool OMEGA1, typename Hook = NoHook, int NW = NWARP, bool OWN = false>
 __device__ __forceinline__ void tile_sweeps(float (&x)[RT][JT], const float (&w)[RT][JT],
                                             const float (&bw)[RT][JT], float om1,
                                             float4 (&xch)[2][2][NW][32], int warp, int lane,
@@ -544,7 +553,7 @@ __device__ __forceinline__ void tile_sweeps(float (&x)[RT][JT], const float (&w)
 #pragma unroll
   for (int sw = 0; sw < TMAX; ++sw) {
     hook(sw);
-    tile_sweep<OMEGA1, NW>(x, w, bw, om1, xch, warp, lane, sw & 1);
+    tile_sweep<OMEGA1, NW, OWN>(x, w, bw, om1, xch, warp, lane, sw & 1);
   }
 }
 
@@ -796,8 +805,8 @@ __global__ void __launch_bounds__(TB_THREADS, 2)
 // claims its next item while it sweeps the current one, so the tensor
 // memory accelerator copies the next boxes meanwhile.  Item (ph, t) starts
 // once the up to nine tiles whose owned cells its region reads have
-// finished phase ph - 1 (done[n] >= ph; done[t] = ph + 1 is published with
-// release semantics after the tile's stores).  That one wait covers both
+// finished phase ph - 1 (done[n] >= ph; done[t] = ph + 1 is published after
+// a fence that follows the tile's stores).  That one wait covers both
 // hazards of the ping-pong buffers: the neighbours' phase ph - 1 results
 // are in src(ph), and they no longer read src(ph - 1), which this item
 // overwrites.  Items are claimed in increasing order and depend only on
@@ -805,14 +814,11 @@ __global__ void __launch_bounds__(TB_THREADS, 2)
 // blocks are resident: cooperative launch).  No block idles at a launch
 // boundary or in a partial last wave.  Same per-cell arithmetic, same
 // results.
-__device__ __forceinline__ void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // Whether the tiles around t (3 x 3, clipped to the tile grid) finished
 // phase ph - 1.  All 32 lanes of a warp call it: lane l < 9 reads the flag
-// of neighbour (l / 3 - 1, l % 3 - 1) with a relaxed load followed by an
-// acquire fence.
+// of neighbour (l / 3 - 1, l % 3 - 1) with a relaxed load; an acquire fence
+// follows once all are set (one in every poll cost more than the poll).
 __device__ __forceinline__ bool flow_ready_warp(const int* done, int ph, int t, int ntx, int nty,
                                                 int lane) {
   bool ok = true;
@@ -824,204 +830,221 @@ __device__ __forceinline__ bool flow_ready_warp(const int* done, int ph, int t, 
       asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(done + y * ntx + x)
                    : "memory");
       ok = v >= ph;
-      asm volatile("fence.acq_rel.gpu;" ::: "memory");
     }
   }
-  return __all_sync(0xffffffffu, ok);
+  if (!__all_sync(0xffffffffu, ok)) return false;
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  return true;
+}
+
+// Tiles of 12 warps, one block an SM: 96 x 128 regions owning 80 x 112 cells
+// (73% of the swept cells; 66% with 8 warps and 48 x 112).  A thirteenth warp
+// does everything that waits: it claims the next item, starts its w and w*b
+// copies as soon as the sweeping warps have taken the present item into
+// registers, its phi copy once its neighbours' flags are set, and publishes
+// each tile once the warps have stored it; the sweeping warps meet only on a
+// barrier of their own.  (It belongs to a warpgroup whose registers go to the
+// other three: 12 x 32 x 152 + 4 x 32 x 40 = 63,488 of the 512 x 128 = 65,536
+// the block is launched with.)  Bound by the sweeps' instructions: of an item's
+// 8,000 cycles 5,430 are sweeps, 1,250 the fill from shared memory and 1,000
+// the stores; 48 MB of boxes a phase at 2048 x 2048 stay in L2.  Per 8 sweeps
+// (us), against two 8-warp blocks an SM whose own threads waited for boxes and
+// flags: 2048 x 2048 13.5 (16.9), 1300 x 1300 8.5 (10.7), 1500 x 1100 8.2
+// (10.5), 1700 x 1700 9.6 (12.5), 3000 x 2500 26.3 (32.2).  A fence in every
+// poll of the flags and the timer read on every turn held the phi copy back
+// 5,000 cycles an item (15.0 at 2048 x 2048).
+constexpr int FW = 12, FI = FW * RT, FO = FI - 2 * TMAX, FLOW_FLOATS = FI * RJ;
+constexpr int FLOW_THREADS = 32 * (FW + 4);
+
+// Whether phase `parity` has completed, without waiting (try_wait suspends).
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 template <bool OMEGA1>
-__global__ void __launch_bounds__(TB_THREADS, 2)
+__global__ void __launch_bounds__(FLOW_THREADS, 1)
     k_jacobi_flow(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
                   const __grid_constant__ CUtensorMap tmw, const __grid_constant__ CUtensorMap tmb,
                   float* __restrict__ x0, float* __restrict__ x1, float om1, PCtl* ctl,
                   int* __restrict__ done, int nphase, int zero_first, Grid g, int ntx, int nty,
                   int* err, int stall_tile) {
-  extern __shared__ __align__(128) float4 tbuf4[];  // [3][RI][RJ] floats: phi, w, w*b
+  extern __shared__ __align__(128) float4 tbuf4[];  // [3][FI][RJ] floats: phi, w, w*b
   float* tbuf = reinterpret_cast<float*>(tbuf4);
-  __shared__ float4 xch[2][2][NWARP][32];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ int s_item;
+  __shared__ float4 xch[2][2][FW][32];
+  // full: an item's boxes have landed (and s_item names it); empty: the
+  // sweeping warps hold it in registers; stored: they have stored it.
+  __shared__ __align__(8) uint64_t full, empty, stored;
+  __shared__ int s_item, s_lost;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntiles = ntx * nty, total = ntiles * nphase;
   int* counter = done + ntiles;
-  // Thread 0: copy item i's boxes (phi of its phase's source, w, w*b).
-  auto issue = [&](int i) {
-    const int ph = i / ntiles, t = i - ph * ntiles;
-    const int ty = t / ntx, tx = t - ty * ntx;
-    const int x = tx * OJ - TMAX, y = ty * OI - TMAX;  // x: a multiple of 4 floats (16 bytes)
-    const bool zi = zero_first && ph == 0;
-    // The neighbours' (generic) stores, acquired above, before the copy's
-    // reads; this block's earlier shared-memory reads before its writes.
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar, (zi ? 2u : 3u) * TILE_FLOATS * 4u);
-    if (!zi) tma_load_2d(tbuf, (ph & 1) ? &tm1 : &tm0, x, y, &bar);
-    tma_load_2d(tbuf + TILE_FLOATS, &tmw, x, y, &bar);
-    tma_load_2d(tbuf + 2 * TILE_FLOATS, &tmb, x, y, &bar);
-  };
-  // Warp 0 (all lanes): whether item i's inputs are final.
-  auto ready = [&](int i) {
-    const int ph = i / ntiles;
-    return flow_ready_warp(done, ph, i - ph * ntiles, ntx, nty, lane);
-  };
-  // Warp 0: bounded wait (about a second) for item i's inputs.
-  auto wait_ready = [&](int i) -> bool {
-    if (ready(i)) return true;
-    const unsigned long long t0 = global_ns();
-    for (int it = 0; it < MBAR_MAX_TRIES; ++it) {
-      if (ready(i)) return true;
-      if (global_ns() - t0 > MBAR_WAIT_NS) return false;
-    }
-    return false;
-  };
-  int fail = 0;            // thread 0: a wait gave up
-  bool in_flight = false;  // thread 0: a copy issued and not consumed
-  if (warp == 0) {
-    int i = 0;
-    if (lane == 0) {
-      mbar_init(&bar, 1);
-      i = atomicAdd(counter, 1);
-    }
-    i = __shfl_sync(0xffffffffu, i, 0);
-    const bool ok = i < total ? wait_ready(i) : true;
-    if (lane == 0) {
-      if (i < total) {
-        if (ok) {
-          issue(i);
-          in_flight = true;
-        } else {
-          fail = 1;
-        }
-      }
-      s_item = i;
-    }
+  if (tid == 0) {
+    mbar_init(&full, 1);
+    mbar_init(&empty, FW);
+    mbar_init(&stored, FW);
+    s_item = 0;
+    s_lost = 0;
   }
-  unsigned parity = 0;
-  const bool own_col = lane * JT >= TMAX && lane * JT < RJ - TMAX;
-  while (true) {
-    if (__syncthreads_or(fail)) break;
-    const int item = s_item;
-    if (item >= total) break;
-    const bool landed = mbar_wait_bounded(&bar, parity);
-    if (__syncthreads_or(!landed)) {
-      if (tid == 0) fail = 1;
-      break;
-    }
-    if (tid == 0) in_flight = false;
-    parity ^= 1u;
-    const int ph = item / ntiles, t = item - ph * ntiles;
-    const int ty = t / ntx, tx = t - ty * ntx;
-    const int gi0 = ty * OI - TMAX + warp * RT;
-    const int gj = tx * OJ - TMAX + lane * JT;
-    const bool zi = zero_first && ph == 0;
-    float x[RT][JT], w[RT][JT], bw[RT][JT];
-#pragma unroll
-    for (int r = 0; r < RT; ++r) {
-      const int o = (warp * RT + r) * RJ + lane * JT;
-      float4 a = zi ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(tbuf + o);
-      float4 ww = *reinterpret_cast<const float4*>(tbuf + TILE_FLOATS + o);
-      float4 bb = *reinterpret_cast<const float4*>(tbuf + 2 * TILE_FLOATS + o);
-      x[r][0] = a.x; x[r][1] = a.y; x[r][2] = a.z; x[r][3] = a.w;
-      w[r][0] = ww.x; w[r][1] = ww.y; w[r][2] = ww.z; w[r][3] = ww.w;
-      bw[r][0] = bb.x; bw[r][1] = bb.y; bw[r][2] = bb.z; bw[r][3] = bb.w;
-#pragma unroll
-      for (int q = 0; q < JT; ++q)
-        if (gj + q >= g.NY) {  // the pitch padding (outside the grid: zero-filled)
-          x[r][q] = 0.0f;
-          w[r][q] = 0.0f;
-          bw[r][q] = 0.0f;
-        }
-    }
-    __syncthreads();  // the boxes are in registers: the buffer takes the next item
-    // Warp 0 claims and prepares the next item while it sweeps this one:
-    // the claim is sent before sweep 0, the neighbours' flags are read
-    // before sweep 2 and looked at before sweep 4, where the copy of the
-    // next boxes starts if they are final (else after this tile).  No wait
-    // on an atomic or a flag sits in front of a sweep barrier.
-    int next = total, flag = 0;
-    bool pending = false;
-    auto hook = [&](int sw) {
-      if (warp != 0) return;
-      if (sw == 0) {
-        if (lane == 0) next = atomicAdd(counter, 1);
-      } else if (sw == 2) {
-        next = __shfl_sync(0xffffffffu, next, 0);
-        flag = INT_MAX;
-        const int nph = next / ntiles, nt = next - nph * ntiles;
-        if (next < total && nph > 0 && lane < 9) {
-          const int nty0 = nt / ntx, ntx0 = nt - nty0 * ntx;
-          const int y = nty0 + lane / 3 - 1, xx = ntx0 + lane % 3 - 1;
-          if (y >= 0 && y < nty && xx >= 0 && xx < ntx)
-            asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];"
-                         : "=r"(flag)
-                         : "l"(done + y * ntx + xx)
-                         : "memory");
-        }
-      } else if (sw == 4) {
-        const bool ok = __all_sync(0xffffffffu, flag >= next / ntiles);
-        if (next < total) {
-          if (ok) {
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");  // the flags acquired
-            __syncwarp();
-            if (lane == 0) {
-              issue(next);
-              in_flight = true;
+  __syncthreads();
+  bool fail = false;
+  if (warp >= FW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp > FW) return;
+    auto claim = [&] {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(counter, 1);
+      return __shfl_sync(0xffffffffu, i, 0);
+    };
+    // With two tiles or more for each block a neighbour's flag is set well
+    // before it is needed, and the next claim goes before the publication of
+    // the tile just stored (2048 x 2048, 494 tiles on 152 blocks: 13.5 us per
+    // phase against 14.4); with fewer the neighbours wait for that publication,
+    // and it goes first (1300 x 1300, 204 tiles: 8.5 us against 9.3).
+    const bool deep = ntiles >= 2 * (int)gridDim.x;
+    int cur_ph = 0, cur_t = -1, next = claim();
+    bool flight = false;
+    for (unsigned n = 0;; ++n) {
+      // Item `next` goes into the buffer when it is free; the item before it
+      // is swept meanwhile.  Everything about it that needs no buffer (its
+      // place, the neighbours' flags) is known by then.
+      const bool have = next < total;
+      const int ph = next / ntiles, t = next - ph * ntiles, ty = t / ntx, tx = t - ty * ntx;
+      const int x = tx * OJ - TMAX, y = ty * FO - TMAX;  // x: a multiple of 4 floats (16 bytes)
+      const bool zi = zero_first && ph == 0;  // phi starts from 0: not copied
+      int after = 0;
+      bool unused = n == 0, ready = !have, copied = !have, told = cur_t < 0;
+      bool taken = false;
+      unsigned long long t0 = 0;
+      for (int it = 0;; ++it) {
+        if (!taken && (unused || mbar_test(&empty, (n - 1) & 1))) {
+          taken = true;
+          flight = have;
+          if (lane == 0) {
+            s_item = next;
+            if (have) {
+              // The warps' earlier shared-memory reads before the copies' writes.
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              mbar_expect_tx(&full, (zi ? 2u : 3u) * FLOW_FLOATS * 4u);
+              tma_load_2d(tbuf + 2 * FLOW_FLOATS, &tmb, x, y, &full);
+              tma_load_2d(tbuf + FLOW_FLOATS, &tmw, x, y, &full);
+            } else {
+              mbar_arrive(&full);
             }
-          } else {
-            pending = true;  // issued after this tile, once its inputs are final
+          }
+        }
+        if (!ready) ready = flow_ready_warp(done, ph, t, ntx, nty, lane);
+        if (!copied && ready && taken) {
+          if (lane == 0 && !zi) {
+            // The neighbours' (generic) stores, acquired above, before the copy's reads.
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            tma_load_2d(tbuf, (ph & 1) ? &tm1 : &tm0, x, y, &full);
+          }
+          copied = true;
+        }
+        if (taken && !told && mbar_test(&stored, (n - 1) & 1)) {
+          if (deep) after = claim();
+          if (lane == 0 && cur_t != stall_tile) {  // (a stalled tile: fault injection)
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(done + cur_t), "r"(cur_ph + 1)
+                         : "memory");
+          }
+          told = true;
+        }
+        if (taken && copied && told) break;
+        if ((it & 63) == 63) {  // (the timer is slow to read)
+          const unsigned long long now = global_ns();
+          if (t0 == 0) t0 = now;
+          if (it >= MBAR_MAX_TRIES || now - t0 > MBAR_WAIT_NS) {
+            fail = true;
+            break;
           }
         }
       }
-    };
-    tile_sweeps<OMEGA1>(x, w, bw, om1, xch, warp, lane, hook);
-    float* dst = (ph & 1) ? x0 : x1;
-    if (own_col && warp >= TMAX / RT && warp < NWARP - TMAX / RT) {
+      if (fail || !have) break;
+      next = n == 0 || !deep ? claim() : after;
+      cur_ph = ph;
+      cur_t = t;
+    }
+    // A copy still landing when a wait gave up.
+    if (fail && flight && lane == 0) mbar_drain(&full, 0), mbar_drain(&full, 1);
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+    const bool own_col = lane * JT >= TMAX && lane * JT < RJ - TMAX;
+    for (unsigned n = 0;; ++n) {
+      const bool landed = mbar_wait_bounded(&full, n & 1);
+      const int item = s_item;
+      // (A wait that gave up: every warp leaves after this item's sweeps, whose
+      // barriers show it to all; the item named is then an earlier one.)
+      if (!landed) s_lost = 1;
+      if (item >= total) break;
+      const int ph = item / ntiles, t = item - ph * ntiles;
+      const int ty = t / ntx, tx = t - ty * ntx;
+      const int gi0 = ty * FO - TMAX + warp * RT;
+      const int gj = tx * OJ - TMAX + lane * JT;
+      const bool zi = zero_first && ph == 0;
+      float x[RT][JT], w[RT][JT], bw[RT][JT];
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
-        int gi = gi0 + r;
-        if (gi >= g.NX || gj >= g.NY) continue;
-        size_t c = (size_t)gi * g.P + gj;
-        if (gj + JT <= g.NY) {
-          *reinterpret_cast<float4*>(dst + c) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
-        } else {
+        const int o = (warp * RT + r) * RJ + lane * JT;
+        float4 a = zi ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(tbuf + o);
+        float4 ww = *reinterpret_cast<const float4*>(tbuf + FLOW_FLOATS + o);
+        float4 bb = *reinterpret_cast<const float4*>(tbuf + 2 * FLOW_FLOATS + o);
+        x[r][0] = a.x; x[r][1] = a.y; x[r][2] = a.z; x[r][3] = a.w;
+        w[r][0] = ww.x; w[r][1] = ww.y; w[r][2] = ww.z; w[r][3] = ww.w;
+        bw[r][0] = bb.x; bw[r][1] = bb.y; bw[r][2] = bb.z; bw[r][3] = bb.w;
 #pragma unroll
-          for (int q = 0; q < JT; ++q)
-            if (gj + q < g.NY) dst[c + q] = x[r][q];
-        }
+        for (int q = 0; q < JT; ++q)
+          if (gj + q >= g.NY) {  // the pitch padding (outside the grid: zero-filled)
+            x[r][q] = 0.0f;
+            w[r][q] = 0.0f;
+            bw[r][q] = 0.0f;
+          }
       }
-    }
-    __syncthreads();  // the tile's stores precede its publication
-    if (warp == 0) {
-      if (lane == 0 && t != stall_tile) {  // (a stalled tile: fault injection)
-        __threadfence();
-        st_release(done + t, ph + 1);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty);
+      tile_sweeps<OMEGA1, NoHook, FW, true>(x, w, bw, om1, xch, warp, lane);
+      if (*(volatile int*)&s_lost) {
+        fail = true;
+        break;
       }
-      if (pending) {
-        const bool ok = wait_ready(next);
-        if (lane == 0) {
-          if (ok) {
-            issue(next);
-            in_flight = true;
+      float* dst = (ph & 1) ? x0 : x1;
+      if (own_col && warp >= TMAX / RT && warp < FW - TMAX / RT) {
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          int gi = gi0 + r;
+          if (gi >= g.NX || gj >= g.NY) continue;
+          size_t c = (size_t)gi * g.P + gj;
+          if (gj + JT <= g.NY) {
+            *reinterpret_cast<float4*>(dst + c) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
           } else {
-            fail = 1;
+#pragma unroll
+            for (int q = 0; q < JT; ++q)
+              if (gj + q < g.NY) dst[c + q] = x[r][q];
           }
         }
       }
-      if (lane == 0) s_item = next;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&stored);
     }
   }
-  if (tid == 0) {
-    if (fail) {
-      atomicExch(&ctl->pad[0], 1);
-      if (err) atomicExch(err, 1);
-    }
-    if (in_flight) mbar_drain(&bar, parity);  // a copy still landing
-    if (blockIdx.x == 0 && nphase > 0) {
-      ctl->sweeps = nphase * TMAX;
-      ctl->last_launch = nphase - 1;
-      ctl->sel = ((nphase - 1) & 1) ? 0 : 1;
-    }
+  if (fail && lane == 0) {
+    atomicExch(&ctl->pad[0], 1);
+    if (err) atomicExch(err, 1);
+  }
+  if (tid == 0 && blockIdx.x == 0 && nphase > 0) {
+    ctl->sweeps = nphase * TMAX;
+    ctl->last_launch = nphase - 1;
+    ctl->sel = ((nphase - 1) & 1) ? 0 : 1;
   }
 }
 
@@ -1667,11 +1690,12 @@ unsigned long long context_key() {
   return (1ull << 63) | (unsigned long long)dev;
 }
 
-static bool encode_box_map(CUtensorMap* tm, const float* base, int rows, int pitch) {
+static bool encode_box_map(CUtensorMap* tm, const float* base, int rows, int pitch,
+                           int box_rows = RI) {
   if (!g_encode || (reinterpret_cast<uintptr_t>(base) & 15) || (pitch % 4) != 0) return false;
   cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(float)};
-  cuuint32_t box[2] = {(cuuint32_t)RJ, (cuuint32_t)RI};
+  cuuint32_t box[2] = {(cuuint32_t)RJ, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims,
                         strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1737,14 +1761,15 @@ void init_jacobi_tma() {
       d->sms = 0;
     // Blocks of the dataflow kernel that fit on one SM (co-residency bound).
     int b1 = 0, b2 = 0;
+    const int fsmem = 3 * FLOW_FLOATS * (int)sizeof(float);
     if (cudaFuncSetAttribute(k_jacobi_flow<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) == cudaSuccess &&
+                             fsmem) == cudaSuccess &&
         cudaFuncSetAttribute(k_jacobi_flow<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_jacobi_flow<true>, TB_THREADS,
-                                                      smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_jacobi_flow<false>, TB_THREADS,
-                                                      smem) == cudaSuccess)
+                             fsmem) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_jacobi_flow<true>, FLOW_THREADS, fsmem) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, k_jacobi_flow<false>, FLOW_THREADS, fsmem) ==
+            cudaSuccess)
       d->flow_per_sm = b1 < b2 ? b1 : b2;
     int coop = 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
@@ -1842,15 +1867,14 @@ static bool launch_jacobi_flow(cudaStream_t st, const Grid& g, PCtl* ctl, float*
   if (!done || nphase < 2) return false;
   const TmaDevice* dv = tma_ready(st);
   if (!dv || dv->flow_per_sm <= 0 || dv->sms <= 0) return false;
-  const int ntx = (g.NY + OJ - 1) / OJ, nty = (g.NX + OI - 1) / OI;
+  // Grids of fewer 48 x 112 tiles than SMs stay with the per-launch kernels
+  // (which run there only without the resident solve's buffers).
+  if (jacobi_tile_count(g.NX, g.NY) < dv->sms) return false;
+  const int ntx = (g.NY + OJ - 1) / OJ, nty = (g.NX + FO - 1) / FO;
   const int ntiles = ntx * nty;
-  // Below one tile per SM the per-launch kernels were measured faster
-  // (128^2 jet 68.3 against 64.6 us per step, 512x256 Karman street 138.5
-  // against 121.7 us).
-  if (ntiles < dv->sms) return false;
   CUtensorMap tm0, tm1, tmw, tmb;
-  if (!encode_box_map(&tm0, x0, g.NX, g.P) || !encode_box_map(&tm1, x1, g.NX, g.P) ||
-      !encode_box_map(&tmw, W, g.NX, g.P) || !encode_box_map(&tmb, BW, g.NX, g.P))
+  if (!encode_box_map(&tm0, x0, g.NX, g.P, FI) || !encode_box_map(&tm1, x1, g.NX, g.P, FI) ||
+      !encode_box_map(&tmw, W, g.NX, g.P, FI) || !encode_box_map(&tmb, BW, g.NX, g.P, FI))
     return false;
   // The tile flags and the item counter.
   if (cudaMemsetAsync(done, 0, sizeof(int) * ((size_t)ntiles + 1), st) != cudaSuccess) return false;
@@ -1858,8 +1882,8 @@ static bool launch_jacobi_flow(cudaStream_t st, const Grid& g, PCtl* ctl, float*
   const int grid = ntiles < cap ? ntiles : cap;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(TB_THREADS);
-  cfg.dynamicSmemBytes = 3 * (size_t)TILE_FLOATS * sizeof(float);
+  cfg.blockDim = dim3(FLOW_THREADS);
+  cfg.dynamicSmemBytes = 3 * (size_t)FLOW_FLOATS * sizeof(float);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;
