@@ -1243,7 +1243,7 @@ __global__ void __launch_bounds__(32 * NW, MB) k_jacobi_res(JResArgs a) {
 #pragma unroll
     for (int m = 0; m < S::PER; ++m) miss = miss || v[m].w != tag;
     if (miss) {
-      const unsigned long long t0 = global_ns();
+      unsigned long long t0 = 0;
       for (int it = 1; miss; ++it) {
         miss = false;
 #pragma unroll
@@ -1251,7 +1251,11 @@ __global__ void __launch_bounds__(32 * NW, MB) k_jacobi_res(JResArgs a) {
           if (v[m].w != tag) v[m] = jld_pkt(slot + source(m));
           miss = miss || v[m].w != tag;
         }
-        if ((it & 63) == 0 && (it >= MBAR_MAX_TRIES || global_ns() - t0 > MBAR_WAIT_NS)) break;
+        if ((it & 63) == 0) {  // (the timer is slow to read)
+          const unsigned long long now = global_ns();
+          if (t0 == 0) t0 = now;
+          if (it >= MBAR_MAX_TRIES || now - t0 > MBAR_WAIT_NS) break;
+        }
       }
       fail = miss;
     }
@@ -2038,9 +2042,9 @@ static bool launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, 
   // an SM.
   // The smallest regions that get an SM each; else two 8-warp regions an SM.
   // Measured per 8 sweeps (us), against the launches or the dataflow kernel
-  // they replace: 4 warps 128^2 2.3 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
+  // they replace: 4 warps 128^2 2.2 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
   // 2.9 (4.4), 800^2 3.0 (6.6); 12 warps 1024x768 4.2 (7.4), 1200x800 4.1
-  // (9.4); 8 warps twice 1200^2 6.2 (11.0).  A larger form where a smaller
+  // (9.4); 8 warps twice 1200^2 6.0 (11.0).  A larger form where a smaller
   // one fits is slower (512x256: 2.4, 3.1, 4.2, 3.9).
   int form = JRES_4;
   while (form <= JRES_8X2 &&
