@@ -552,6 +552,19 @@ cudaError_t launch_particles_advect(fg_fluid* f, float dt, int n_upper, const fl
 cudaError_t launch_render(fg_fluid* f, const float* field, const float* dev_minmax, int diverging,
                           uint32_t* img);
 // Device-to-device copy of an NX x NY field between two row pitches.
+// One copy between rows x width floats stored linearly and the same rows at a
+// pitch (both 16-byte aligned; rows * width < 2^31); a launch takes a list.
+struct CopyItem {
+  float* linear;
+  float* pitched;
+  unsigned rows, width, pitch;
+};
+struct CopyList {
+  CopyItem it[120];
+  int n = 0;
+  bool full() const { return n == 120; }
+};
+cudaError_t launch_copy_list(fg_fluid* f, const CopyList& l, bool to_linear);
 cudaError_t launch_repitch(fg_fluid* f, float* dst, const float* src, int dpitch, int spitch);
 
 // Grid of the reduction kernels: 32 x 8 threads per block over (j, i), at
