@@ -1,5 +1,7 @@
 // C ABI of libfluidgpu: handle lifetime, host mirrors, tool edits, the step
 // sequence and the views.  The kernels live in k_*.cu.
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <climits>
@@ -139,6 +141,31 @@ int copy_mirrors(fg_fluid* f, unsigned mask, bool down) {
                               cudaMemcpyHostToDevice, f->stream), "upload");
   }
   return FG_OK;
+}
+
+enum class Where { Pageable, Pinned, Device };
+Where where_is(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return Where::Pageable;
+  }
+  return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged ? Where::Device
+         : a.type == cudaMemoryTypeHost                                    ? Where::Pinned
+                                                                           : Where::Pageable;
+}
+
+// Before a copy into pageable memory that it overwrites whole: writes one byte
+// of every page, so the pages are mapped.  Where the GPU reads the host's page
+// tables the copy engine writes such memory at the link's rate (3.2 MB in 26
+// us, 195 through a pinned buffer and a memcpy), but pages that nobody has
+// written yet fault one row at a time (2.8 ms).
+void map_pages(void* p, size_t n) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  if (!n || where_is(p) != Where::Pageable) return;
+  volatile char* b = (volatile char*)p;
+  for (size_t k = 0; k < n; k += page) b[k] = 0;
+  b[n - 1] = 0;
 }
 
 int check_mask(fg_fluid* f) {
@@ -558,7 +585,7 @@ int fg_destroy(fg_fluid* f) {
   cudaFree(f->ectl);
   cudaFree(f->tile_done);
   cudaFree(f->jres);
-  if (f->image_pinned) cudaFreeHost(f->image_pinned);
+  if (f->parts.stage) cudaFreeHost(f->parts.stage);
   cudaFree(f->wave);
   for (int k = 0; k < 2; ++k) {
     cudaFreeHost(f->edit_pinned[k]);  // edit_dev / edit_off_dev map these
@@ -1203,22 +1230,17 @@ int fg_max_divergence(fg_fluid* f, float* out) {
   if (is_batch(f)) return batch_unsupported(f);
   STAGE_PROLOGUE(f);
   if (!out) return FG_ERR_INVALID;
-  float* slot = dev_scalar_slot(f);
-  CK(f, launch_max_divergence(f, slot), "maxdiv");
-  CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, sizeof(float), cudaMemcpyDeviceToHost, f->stream),
-     "maxdiv");
+  CK(f, launch_max_divergence(f, f->scalar_pinned), "maxdiv");
   if ((rc = read_scalars(f, 1))) return rc;
   *out = f->scalar_pinned[0];
   return FG_OK;
 }
 
 static int view_common(fg_fluid* f, int kind, float* out_host, float* mn, float* mx) {
-  float* slot = dev_scalar_slot(f);
-  CK(f, launch_view(f, kind, slot), "view");
-  CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, 2 * sizeof(float), cudaMemcpyDeviceToHost,
-                        f->stream), "view");
+  CK(f, launch_view(f, kind, f->scalar_pinned), "view");
   if (out_host) {
     size_t hp = sizeof(float) * f->NY, dp = sizeof(float) * f->P;
+    map_pages(out_host, hp * f->NX);
     CK(f, cudaMemcpy2DAsync(out_host, hp, f->view, dp, hp, f->NX, cudaMemcpyDeviceToHost,
                             f->stream), "view");
   }
@@ -1245,10 +1267,7 @@ int fg_field_min_max(fg_fluid* f, int field, float* mn, float* mx) {
   if (is_batch(f)) return batch_unsupported(f);
   STAGE_PROLOGUE(f);
   if (field < 0 || field >= FG_NUM_FIELDS) return fail(f, FG_ERR_INVALID, "bad field");
-  float* slot = dev_scalar_slot(f);
-  CK(f, launch_field_minmax(f, field, slot), "minmax");
-  CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, 2 * sizeof(float), cudaMemcpyDeviceToHost,
-                        f->stream), "minmax");
+  CK(f, launch_field_minmax(f, field, f->scalar_pinned), "minmax");
   if ((rc = read_scalars(f, 2))) return rc;
   if (mn) *mn = f->scalar_pinned[0];
   if (mx) *mx = f->scalar_pinned[1];
@@ -1258,10 +1277,7 @@ int fg_field_min_max(fg_fluid* f, int field, float* mn, float* mx) {
 int fg_sample_velocity(fg_fluid* f, float x, float y, float* u, float* v) {
   if (is_batch(f)) return batch_unsupported(f);
   STAGE_PROLOGUE(f);
-  float* slot = dev_scalar_slot(f);
-  CK(f, launch_sample_velocity(f, x, y, slot), "sample");
-  CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, 2 * sizeof(float), cudaMemcpyDeviceToHost,
-                        f->stream), "sample");
+  CK(f, launch_sample_velocity(f, x, y, f->scalar_pinned), "sample");
   if ((rc = read_scalars(f, 2))) return rc;
   if (u) *u = f->scalar_pinned[0];
   if (v) *v = f->scalar_pinned[1];
@@ -1272,10 +1288,7 @@ int fg_adaptive_time_step(fg_fluid* f, float basedt, float* out) {
   if (is_batch(f)) return batch_unsupported(f);
   STAGE_PROLOGUE(f);
   if (!out) return FG_ERR_INVALID;
-  float* slot = dev_scalar_slot(f);
-  CK(f, launch_max_speed(f, slot), "max speed");
-  CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, sizeof(float), cudaMemcpyDeviceToHost, f->stream),
-     "max speed");
+  CK(f, launch_max_speed(f, f->scalar_pinned), "max speed");
   if ((rc = read_scalars(f, 1))) return rc;
   float maxVel = f->scalar_pinned[0];
   if (maxVel == 0.0f) {
@@ -1443,16 +1456,8 @@ int load_state(fg_fluid* f, const float* src) {
 
 // Copies a field in the Go slice layout (host or device memory) to a
 // pitched device field, or back.
-bool on_device(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
-}
 int put_field(fg_fluid* f, float* dev, const float* src) {
-  if (on_device(src)) {
+  if (where_is(src) == Where::Device) {
     CK(f, launch_repitch(f, dev, src, f->P, f->NY), "upload");
     return FG_OK;
   }
@@ -1461,11 +1466,12 @@ int put_field(fg_fluid* f, float* dev, const float* src) {
   return FG_OK;
 }
 int get_field(fg_fluid* f, float* dst, const float* dev) {
-  if (on_device(dst)) {
+  if (where_is(dst) == Where::Device) {
     CK(f, launch_repitch(f, dst, dev, f->NY, f->P), "download");
     return FG_OK;
   }
   size_t hp = sizeof(float) * f->NY, dp = sizeof(float) * f->P;
+  map_pages(dst, hp * f->NX);
   CK(f, cudaMemcpy2DAsync(dst, hp, dev, dp, hp, f->NX, cudaMemcpyDefault, f->stream), "download");
   return FG_OK;
 }
@@ -2336,6 +2342,8 @@ int fg_batch_grad(fg_fluid* f, int s, float* dU, float* dV, float* dM) {
   const int src[3] = {fg_fluid::A_U, fg_fluid::A_V, fg_fluid::A_M};
   size_t hp = sizeof(float) * sc.g.NY, dp = sizeof(float) * sc.g.P;
   for (int k = 0; k < 3; ++k)
+    if (out[k]) map_pages(out[k], hp * sc.g.NX);
+  for (int k = 0; k < 3; ++k)
     if (out[k])
       CK(f, cudaMemcpy2DAsync(out[k], hp, f->adj[src[k]] + sc.off, dp, hp, sc.g.NX,
                               cudaMemcpyDefault, f->stream), "grad");
@@ -2423,9 +2431,39 @@ namespace {
 
 constexpr int kParticleBlock = 1024;
 
+// Up to this many particles go through one pinned buffer and one launch (five
+// copies to or from pageable memory cost 10 us each); more, and calls with
+// device pointers, are copied directly.
+constexpr int kStageParticles = 16384;
+
+// The pinned buffer: x, y, age, max age, rgb of kStageParticles, the count.
+uint32_t* particle_stage(fg_fluid* f) {
+  if (!f->parts.stage &&
+      host_malloc((void**)&f->parts.stage, sizeof(uint32_t) * (5 * kStageParticles + 4)) !=
+          cudaSuccess) {
+    f->parts.stage = nullptr;
+    cudaGetLastError();
+  }
+  return f->parts.stage;
+}
+
+// The staged copies of n particles at index `at`, and the count's.
+CopyList particle_list(fg_fluid* f, int n, int at) {
+  auto& P = f->parts;
+  CopyList l;
+  auto add = [&](int slot, void* dev, unsigned words) {
+    l.it[l.n++] = {(float*)(P.stage + (size_t)slot * kStageParticles), (float*)dev, 1u, words,
+                   words};
+  };
+  for (int q = 0; q < 4; ++q) add(q, P.a[P.cur][q] + at, n);
+  add(4, P.rgb[P.cur] + at, n);
+  add(5, P.count, 1);
+  return l;
+}
+
 int particles_read_count(fg_fluid* f, int* out) {
   auto& P = f->parts;
-  if (!P.count) {
+  if (!P.count || P.n_upper == 0) {
     *out = 0;
     return FG_OK;
   }
@@ -2435,6 +2473,14 @@ int particles_read_count(fg_fluid* f, int* out) {
   memcpy(out, f->scalar_pinned, sizeof(int));
   P.n_upper = *out;
   return FG_OK;
+}
+
+void unpack_rgb(unsigned char* rgb, const uint32_t* packed, int n) {
+  for (int k = 0; rgb && k < n; ++k) {
+    rgb[3 * k] = (unsigned char)(packed[k] & 0xff);
+    rgb[3 * k + 1] = (unsigned char)((packed[k] >> 8) & 0xff);
+    rgb[3 * k + 2] = (unsigned char)((packed[k] >> 16) & 0xff);
+  }
 }
 
 // Grows the particle buffers to hold `need` particles, keeping the first n.
@@ -2447,6 +2493,7 @@ int particles_reserve(fg_fluid* f, int need, int n) {
   Q.cap = cap;
   Q.cur = 0;
   Q.n_upper = P.n_upper;
+  Q.stage = P.stage;
   cudaError_t e = cudaSuccess;
   for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
     for (int q = 0; q < 4 && e == cudaSuccess; ++q)
@@ -2505,6 +2552,24 @@ int fg_particles_add(fg_fluid* f, int n, const float* x, const float* y, const f
   if (n == 0) return FG_OK;
   if ((rc = particles_reserve(f, have + n, have))) return rc;
   auto& P = f->parts;
+  const int total = have + n;
+  if (n <= kStageParticles && particle_stage(f) && where_is(x) != Where::Device &&
+      where_is(y) != Where::Device && where_is(max_age) != Where::Device) {
+    uint32_t* st = P.stage;
+    memcpy(st, x, sizeof(float) * n);
+    memcpy(st + kStageParticles, y, sizeof(float) * n);
+    memset(st + 2 * kStageParticles, 0, sizeof(float) * n);
+    memcpy(st + 3 * kStageParticles, max_age, sizeof(float) * n);
+    uint32_t* c = st + 4 * kStageParticles;
+    for (int k = 0; k < n; ++k)
+      c[k] = (uint32_t)rgb[3 * k] | ((uint32_t)rgb[3 * k + 1] << 8) |
+             ((uint32_t)rgb[3 * k + 2] << 16);
+    st[5 * kStageParticles] = (uint32_t)total;
+    CK(f, launch_copy_list(f, particle_list(f, n, have), false), "particle upload");
+    CK(f, cudaStreamSynchronize(f->stream), "particle upload");
+    P.n_upper = total;
+    return FG_OK;
+  }
   std::vector<float> age(n, 0.0f);
   std::vector<uint32_t> packed(n);
   for (int k = 0; k < n; ++k)
@@ -2516,7 +2581,6 @@ int fg_particles_add(fg_fluid* f, int n, const float* x, const float* y, const f
                           f->stream), "particle upload");
   CK(f, cudaMemcpyAsync(P.rgb[P.cur] + have, packed.data(), sizeof(uint32_t) * n,
                         cudaMemcpyHostToDevice, f->stream), "particle upload");
-  int total = have + n;
   CK(f, cudaMemcpyAsync(P.count, &total, sizeof(int), cudaMemcpyHostToDevice, f->stream),
      "particle count");
   CK(f, cudaStreamSynchronize(f->stream), "particle upload");
@@ -2554,11 +2618,22 @@ int fg_particles_get(fg_fluid* f, float* x, float* y, float* age, float* max_age
   if (!f) return FG_ERR_INVALID;
   int rc = bind(f);
   if (rc) return rc;
-  int n = 0;
-  if ((rc = particles_read_count(f, &n))) return rc;
-  if (n == 0) return FG_OK;
   auto& P = f->parts;
   float* dst[4] = {x, y, age, max_age};
+  int n = P.count ? P.n_upper : 0;
+  bool stage = n <= kStageParticles;
+  for (float* d : dst) stage = stage && !(d && where_is(d) == Where::Device);
+  if (n && stage && particle_stage(f)) {
+    CK(f, launch_copy_list(f, particle_list(f, n, 0), true), "particle download");
+    CK(f, cudaStreamSynchronize(f->stream), "particle download");
+    P.n_upper = n = (int)P.stage[5 * kStageParticles];
+    for (int q = 0; q < 4; ++q)
+      if (dst[q]) memcpy(dst[q], P.stage + (size_t)q * kStageParticles, sizeof(float) * n);
+    unpack_rgb(rgb, P.stage + 4 * kStageParticles, n);
+    return FG_OK;
+  }
+  if ((rc = particles_read_count(f, &n))) return rc;
+  if (n == 0) return FG_OK;
   for (int q = 0; q < 4; ++q)
     if (dst[q])
       CK(f, cudaMemcpyAsync(dst[q], P.a[P.cur][q], sizeof(float) * n, cudaMemcpyDefault,
@@ -2568,11 +2643,7 @@ int fg_particles_get(fg_fluid* f, float* x, float* y, float* age, float* max_age
     CK(f, cudaMemcpyAsync(packed.data(), P.rgb[P.cur], sizeof(uint32_t) * n,
                           cudaMemcpyDeviceToHost, f->stream), "particle download");
   CK(f, cudaStreamSynchronize(f->stream), "particle download");
-  for (int k = 0; rgb && k < n; ++k) {
-    rgb[3 * k] = (unsigned char)(packed[k] & 0xff);
-    rgb[3 * k + 1] = (unsigned char)((packed[k] >> 8) & 0xff);
-    rgb[3 * k + 2] = (unsigned char)((packed[k] >> 16) & 0xff);
-  }
+  unpack_rgb(rgb, packed.data(), n);
   return FG_OK;
 }
 
@@ -2605,25 +2676,7 @@ int fg_render(fg_fluid* f, int kind, void* rgba) {
     field = f->view;
   }
   CK(f, launch_render(f, field, mm, kind == FG_RENDER_VORTICITY ? 1 : 0, f->image), "render");
-  // Pageable host memory (an app's image buffer) gets the frame through a
-  // pinned staging copy: the device copy into pageable memory runs at a
-  // fraction of the link's rate.
-  cudaPointerAttributes pa{};
-  const bool pageable = cudaPointerGetAttributes(&pa, rgba) == cudaSuccess
-                            ? pa.type == cudaMemoryTypeUnregistered
-                            : (cudaGetLastError(), true);
-  if (pageable && !f->image_pinned &&
-      host_malloc((void**)&f->image_pinned, bytes) != cudaSuccess) {
-    f->image_pinned = nullptr;
-    cudaGetLastError();
-  }
-  if (pageable && f->image_pinned) {
-    CK(f, cudaMemcpyAsync(f->image_pinned, f->image, bytes, cudaMemcpyDeviceToHost, f->stream),
-       "render");
-    CK(f, cudaStreamSynchronize(f->stream), "render");
-    memcpy(rgba, f->image_pinned, bytes);
-    return FG_OK;
-  }
+  map_pages(rgba, bytes);
   CK(f, cudaMemcpyAsync(rgba, f->image, bytes, cudaMemcpyDefault, f->stream), "render");
   CK(f, cudaStreamSynchronize(f->stream), "render");
   return FG_OK;

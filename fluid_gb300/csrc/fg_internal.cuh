@@ -412,9 +412,9 @@ struct fg_fluid {
     int* count = nullptr;      // device: live particles
     uint8_t* keep = nullptr;   // device: survivor flags (cap rounded up to whole blocks)
     int* block_keep = nullptr;
+    uint32_t* stage = nullptr;  // pinned staging of small calls
   } parts;
   uint32_t* image = nullptr;
-  void* image_pinned = nullptr;  // pinned staging of fg_render's frames for pageable targets
   // Non-null when this handle is a batch of scenes (fg_batch_create).
   fg::BatchGeom* batch = nullptr;
   // Asynchronous smoke download (fg_download_async): a copy stream, the event
@@ -552,8 +552,8 @@ cudaError_t launch_particles_advect(fg_fluid* f, float dt, int n_upper, const fl
 cudaError_t launch_render(fg_fluid* f, const float* field, const float* dev_minmax, int diverging,
                           uint32_t* img);
 // Device-to-device copy of an NX x NY field between two row pitches.
-// One copy between rows x width floats stored linearly and the same rows at a
-// pitch (both 16-byte aligned; rows * width < 2^31); a launch takes a list.
+// One copy between rows x width floats stored linearly (16-byte aligned) and
+// the same rows at a pitch (rows * width < 2^31); a launch takes a list.
 struct CopyItem {
   float* linear;
   float* pitched;

@@ -17,7 +17,8 @@ template <bool TO_LINEAR>
 __global__ void __launch_bounds__(256) k_copy_list(const __grid_constant__ CopyList l) {
   const CopyItem c = l.it[blockIdx.y];
   const unsigned W = c.width, n = c.rows * W, n4 = n / 4;
-  const bool vec = (W & 3) == 0 && (c.pitch & 3) == 0;
+  const bool vec = (W & 3) == 0 && (c.pitch & 3) == 0 &&
+                   (reinterpret_cast<uintptr_t>(c.pitched) & 15) == 0;
   for (unsigned k = blockIdx.x * 256 + threadIdx.x; k < n4; k += gridDim.x * 256) {
     unsigned i = 4 * k / W, j = 4 * k - i * W;
     float4* lin = reinterpret_cast<float4*>(c.linear) + k;

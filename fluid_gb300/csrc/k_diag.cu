@@ -143,17 +143,22 @@ __global__ void k_minmax_partials(const float* __restrict__ F, float* __restrict
 }
 
 // (max v, max -v) -> float (min, max), with the reference's initial values
-// (MaxFloat32, -MaxFloat32) when no cell was seen.
-__global__ void k_store_minmax(const float* __restrict__ r, float* __restrict__ out) {
-  float hi = r[0], nlo = r[2];
-  out[0] = nlo == -INFINITY ? FLT_MAX : -nlo;
-  out[1] = hi == -INFINITY ? -FLT_MAX : hi;
-}
+// (MaxFloat32, -MaxFloat32) when no cell was seen.  The results of the
+// reductions go to device or pinned host memory.
+struct StoreMinMax {
+  float* out;
+  __device__ void operator()(const float* r) const {
+    float hi = r[0], nlo = r[2];
+    out[0] = nlo == -INFINITY ? FLT_MAX : -nlo;
+    out[1] = hi == -INFINITY ? -FLT_MAX : hi;
+  }
+};
 
 // A max slot of a final row -> float, 0 when no cell was seen.
-__global__ void k_store_max0(const float* __restrict__ r, float* __restrict__ out) {
-  out[0] = r[0] < 0.0f ? 0.0f : r[0];
-}
+struct StoreMax0 {
+  float* out;
+  __device__ void operator()(const float* r) const { out[0] = r[0] < 0.0f ? 0.0f : r[0]; }
+};
 
 __global__ void k_sample_velocity(const float* __restrict__ U, const float* __restrict__ V,
                                   float x, float y, float* __restrict__ out, Grid g) {
@@ -198,12 +203,26 @@ cudaError_t launch_smoke_mass(fg_fluid* f) {
   return launch_store_mass(f, nb);
 }
 
-static cudaError_t finish_max0(fg_fluid* f, int nb, float* dev_out) {
-  float* out = nullptr;
-  count(f, combine_rows<1>(f->stream, f->partials, nb, 1u, &out));
+// The total row of nb block rows to `store`: one block while its threads take
+// at most 16 rows each, else after a first level of 2048 rows a block.
+template <int NS, typename Store>
+static cudaError_t finish_rows(fg_fluid* f, int nb, unsigned max_mask, Store store) {
+  const float* rows = f->partials;
+  if (nb > 16384) {
+    float* lvl = f->partials + (size_t)2 * NS * nb;
+    const int g = (nb + 2047) / 2048;
+    count(f);
+    k_combine_rows<NS><<<g, 1024, 0, f->stream>>>(rows, nb, 2048, max_mask, lvl);
+    rows = lvl;
+    nb = g;
+  }
   count(f);
-  k_store_max0<<<1, 1, 0, f->stream>>>(out, dev_out);
-  return cudaGetLastError();
+  return launch_pdl(k_combine_store<NS, Store>, dim3(1), dim3(1024), 0, f->stream, rows, nb,
+                    max_mask, store);
+}
+
+static cudaError_t finish_max0(fg_fluid* f, int nb, float* out) {
+  return finish_rows<1>(f, nb, 1u, StoreMax0{out});
 }
 
 cudaError_t launch_max_divergence(fg_fluid* f, float* dev_out) {
@@ -226,12 +245,8 @@ cudaError_t launch_max_speed(fg_fluid* f, float* dev_out) {
   return finish_max0(f, nb, dev_out);
 }
 
-static cudaError_t finish_minmax(fg_fluid* f, int nb, float* dev_minmax) {
-  float* out = nullptr;
-  count(f, combine_rows<2>(f->stream, f->partials, nb, 3u, &out));
-  count(f);
-  k_store_minmax<<<1, 1, 0, f->stream>>>(out, dev_minmax);
-  return cudaGetLastError();
+static cudaError_t finish_minmax(fg_fluid* f, int nb, float* minmax) {
+  return finish_rows<2>(f, nb, 3u, StoreMinMax{minmax});
 }
 
 cudaError_t launch_view(fg_fluid* f, int kind, float* dev_minmax) {

@@ -400,7 +400,7 @@ class Fluid:
 
     def tape_grad(self):
         """dL/d(initial U, V, M, newU, newV, newM) as numpy arrays."""
-        out = [np.zeros(self.numCells, np.float32) for _ in range(6)]
+        out = [np.empty(self.numCells, np.float32) for _ in range(6)]
         self._check(self._L.fg_tape_grad(self._h, *[o.ctypes.data for o in out]), "fg_tape_grad")
         return dict(zip(("U", "V", "M", "newU", "newV", "newM"), out))
 
@@ -424,8 +424,8 @@ class Fluid:
                 fu, fv = forces[t] if forces is not None else (None, None)
                 self.step_forward(dt, fu, fv)
             loss = self.tape_seed_smoke_l2(target)
-            gfu = [np.zeros(self.numCells, np.float32) for _ in range(steps)]
-            gfv = [np.zeros(self.numCells, np.float32) for _ in range(steps)]
+            gfu = [np.empty(self.numCells, np.float32) for _ in range(steps)]
+            gfv = [np.empty(self.numCells, np.float32) for _ in range(steps)]
             for t in reversed(range(steps)):
                 self.step_adjoint(gfu[t], gfv[t])
             out = self.tape_grad()
@@ -454,8 +454,8 @@ class Fluid:
     def particles(self):
         n = ctypes.c_int()
         self._check(self._L.fg_particles_count(self._h, ctypes.byref(n)), "fg_particles_count")
-        out = {k: np.zeros(n.value, np.float32) for k in ("X", "Y", "Age", "MaxAge")}
-        rgb = np.zeros((n.value, 3), np.uint8)
+        out = {k: np.empty(n.value, np.float32) for k in ("X", "Y", "Age", "MaxAge")}
+        rgb = np.empty((n.value, 3), np.uint8)
         self._check(self._L.fg_particles_get(self._h, out["X"].ctypes.data, out["Y"].ctypes.data,
                                              out["Age"].ctypes.data, out["MaxAge"].ctypes.data,
                                              rgb.ctypes.data), "fg_particles_get")
@@ -477,7 +477,7 @@ class Fluid:
         """The app's drawScalarField / drawVorticityField image (NumX * NumY *
         4 bytes RGBA, pixel (i, j) showing cell (i, NumY - 1 - j))."""
         self._before()
-        out = np.zeros(self.numCells * 4, np.uint8)
+        out = np.empty(self.numCells * 4, np.uint8)
         self._check(self._L.fg_render(self._h, int(kind), out.ctypes.data), "fg_render")
         self._after()
         return out
@@ -522,7 +522,7 @@ class Fluid:
 
     def _view(self, fn):
         self._before()
-        out = np.zeros(self.numCells, dtype=np.float32)
+        out = np.empty(self.numCells, dtype=np.float32)
         mn, mx = ctypes.c_float(), ctypes.c_float()
         self._check(fn(self._h, out.ctypes.data, ctypes.byref(mn), ctypes.byref(mx)))
         self._after()
@@ -665,7 +665,7 @@ class Batch:
     def grad(self, s):
         """dL_s/d(initial U, V, M) of scene s."""
         n = self.scenes[s].numCells
-        out = [np.zeros(n, np.float32) for _ in range(3)]
+        out = [np.empty(n, np.float32) for _ in range(3)]
         self._check(self._L.fg_batch_grad(self._h, int(s), *[o.ctypes.data for o in out]),
                     "fg_batch_grad")
         return dict(zip(("U", "V", "M"), out))

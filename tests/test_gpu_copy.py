@@ -47,3 +47,47 @@ def test_copies_keep_every_value(w, h):
 
 def test_copies_of_many_scenes():
     round_trip([(8 + 3 * k, 40 - k) for k in range(39)])
+
+
+@pytest.mark.parametrize("counts", [(1, 2, 3), (5, 16384, 7), (16385, 3), (3, 16383)])
+def test_particles_come_back_in_order(counts):
+    import fluid_gb300 as gpu
+
+    f = gpu.Fluid(1.0, 40, 30, 1.0, auto_sync=False)
+    rng = np.random.default_rng(7)
+    want = {k: np.zeros(0, np.float32) for k in ("X", "Y", "MaxAge")}
+    rgb = np.zeros((0, 3), np.uint8)
+    assert f.particles()["X"].size == 0
+    for n in counts:
+        x, y, age = (rng.uniform(1, 30, n).astype(np.float32) for _ in range(3))
+        c = rng.integers(0, 256, (n, 3)).astype(np.uint8)
+        f.particles_add(x, y, age, c)
+        for k, v in zip(("X", "Y", "MaxAge"), (x, y, age)):
+            want[k] = np.concatenate([want[k], v])
+        rgb = np.concatenate([rgb, c])
+        got = f.particles()
+        for k, v in want.items():
+            assert np.array_equal(got[k], v), (n, k)
+        assert not got["Age"].any() and np.array_equal(got["RGB"], rgb)
+    f.particles_clear()
+    assert f.particles()["X"].size == 0
+    f.particles_add(x[:3], y[:3], age[:3], c[:3])
+    assert np.array_equal(f.particles()["Y"], y[:3])
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 40), (510, 1030), (2100, 2046)])
+def test_view_ranges(w, h):
+    """The one-block and the two-level reductions of a view's range."""
+    import fluid_gb300 as gpu
+
+    f = gpu.Fluid(1.0, w, h, 1.0, auto_sync=False)
+    f.S[:] = 1
+    f.M[:] = np.random.default_rng(1).uniform(-3, 5, f.numCells).astype(np.float32)
+    f.U[:] = 2 * f.M
+    f.V[:] = 0.5 - f.M
+    f.mark_dirty()
+    v = f.Smoke()
+    assert (v.MinValue, v.MaxValue) == (f.M.min(), f.M.max())
+    for v in (f.Vorticity(), f.VelocityMagnitude()):
+        inner = v.values.reshape(f.NumX, f.NumY)[1:-1, 1:-1]
+        assert (v.MinValue, v.MaxValue) == (inner.min(), inner.max())
