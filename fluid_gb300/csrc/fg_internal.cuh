@@ -213,6 +213,7 @@ struct DevStats {  // device-side accumulation target (finalised per step)
   double last_maxdiv;
   int sweeps;
   int timeout;  // 1: a bounded device-side wait of the step gave up
+  int ticket;   // finished blocks of the reduction that is running (grid_row)
 };
 
 // ---------------------------------------------------------------- batches
@@ -532,9 +533,6 @@ cudaError_t launch_step_adjoint(fg_fluid* f, float dt, float* const* tape);
 cudaError_t launch_loss_seed(fg_fluid* f, const float* target, double* dev_loss);
 // k_diag.cu
 cudaError_t launch_div_stats(fg_fluid* f);
-cudaError_t launch_smoke_mass(fg_fluid* f);
-// Combines the smoke-mass block partials the final smoke pass wrote.
-cudaError_t launch_store_mass(fg_fluid* f, int nb);
 cudaError_t launch_clear_stats(fg_fluid* f);
 cudaError_t launch_max_divergence(fg_fluid* f, float* dev_out);
 cudaError_t launch_view(fg_fluid* f, int kind, float* dev_minmax);  // 0 vorticity, 1 magnitude

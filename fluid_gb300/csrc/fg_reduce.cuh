@@ -44,6 +44,14 @@ __host__ __device__ __forceinline__ FF ff_add(FF a, FF b) {
 }
 
 #ifdef __CUDACC__
+// Adds a float pair to a running pair; the errors gather in its low part.
+__device__ __forceinline__ void ff_acc(FF& a, FF q) {
+  float t, e;
+  two_sum(a.hi, q.hi, t, e);
+  a.hi = t;
+  a.lo = a.lo + (e + q.lo);
+}
+
 // x*x as an unevaluated float pair (exact).
 __device__ __forceinline__ FF ff_sq(float x) {
   float p = x * x;
@@ -189,48 +197,71 @@ inline int combine_rows(cudaStream_t st, float* part, int n, unsigned max_mask, 
   return 2;
 }
 
-// Combines all n rows of `in` in one block -- thread k merges rows k,
-// k + blockDim.x, ... in turn, then the block's fixed tree -- and hands the
-// total row to store(row) on thread 0: the per-step statistics in one
-// launch instead of a two-level combine and a store kernel.
-template <int NS, typename Store>
-__global__ void __launch_bounds__(1024)
-    k_combine_store(const float* __restrict__ in, int n, unsigned max_mask, Store store) {
-  __shared__ float sh[64 * NS];
-  __shared__ float row[2 * NS];
-  pdl_enter();
-  FF v[NS];
-  slots_identity<NS>(v, max_mask);
-  // U rows' loads are issued before their merges (in the same order), so
-  // a thread waits for one round trip per U rows instead of one per row.
-  constexpr int U = NS > 2 ? 4 : 8;
-  int k = threadIdx.x;
-  for (; k + (U - 1) * (int)blockDim.x < n; k += U * blockDim.x) {
-    FF w[U][NS];
-#pragma unroll
-    for (int q = 0; q < U; ++q) {
-      const size_t r = (size_t)(k + q * blockDim.x) * 2 * NS;
-#pragma unroll
-      for (int s = 0; s < NS; ++s) w[q][s] = FF{in[r + 2 * s], in[r + 2 * s + 1]};
-    }
-#pragma unroll
-    for (int q = 0; q < U; ++q) slots_merge<NS>(v, w[q], max_mask);
+// A grid's reduction in one launch: every block writes its row, and the block
+// that takes the last ticket combines all nblocks of them -- thread k merges
+// rows k, k + block size, ... in turn, then the block's fixed tree, so the
+// order does not depend on which block it is -- and hands the total row to
+// store(row) on thread 0.  *ticket is 0 before and after.  sh holds 64 * NS
+// floats.  Without a ticket the rows stay in `part`.  (A second launch for
+// the rows cost 5 us a reduction on small grids, most of it the launch.)
+template <int NS, unsigned EXACT = 0u, typename Store>
+__device__ __forceinline__ void grid_row(FF (&v)[NS], unsigned max_mask, float* sh, float* part,
+                                         int block, int nblocks, int* ticket, Store store) {
+  __shared__ int last;
+  __shared__ float total[2 * NS];
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x, nt = blockDim.x * blockDim.y;
+  block_row<NS, EXACT>(v, max_mask, sh, part + (size_t)2 * NS * block);  // (written by thread 0)
+  if (!ticket) return;
+  if (tid == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1) == nblocks - 1;
   }
-  for (; k < n; k += blockDim.x) {
-    FF w[NS];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const float2* rows = reinterpret_cast<const float2*>(part);
+  FF t[NS];
+  slots_identity<NS>(t, max_mask);
+  constexpr int U = NS > 2 ? 4 : 8;  // rows whose loads are in flight together
+  for (int k = tid; k < nblocks; k += U * nt) {
+    float2 w[U][NS];
 #pragma unroll
-    for (int s = 0; s < NS; ++s)
-      w[s] = FF{in[(size_t)k * 2 * NS + 2 * s], in[(size_t)k * 2 * NS + 2 * s + 1]};
-    slots_merge<NS>(v, w, max_mask);
+    for (int q = 0; q < U; ++q)
+#pragma unroll
+      for (int s = 0; s < NS; ++s)
+        if (k + q * nt < nblocks) w[q][s] = __ldcg(rows + (size_t)(k + q * nt) * NS + s);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (k + q * nt < nblocks) {
+        FF x[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) x[s] = FF{w[q][s].x, w[q][s].y};
+        slots_merge<NS>(t, x, max_mask);
+      }
   }
-  block_row<NS>(v, max_mask, sh, row);  // thread 0 writes the row
-  if (threadIdx.x == 0) store(row);
+  block_row<NS>(t, max_mask, sh, total);
+  if (tid == 0) {
+    store(total);
+    *ticket = 0;
+  }
 }
 
 // Total of a sum slot of a final row, in FP64.
 __device__ __forceinline__ double row_sum(const float* row, int s) {
   return (double)row[2 * s] + (double)row[2 * s + 1];
 }
+
+// Blocks of the per-cell passes that end in grid_row: each walks several tiles,
+// five blocks an SM.  A block holds its SM until its ticket is back (a fence
+// and an atomic, 2 us), which one tile a block in many waves does not hide:
+// the smoke pass of 2048 x 2048 took 54 us with 16,705 such blocks.
+constexpr int kStatBlocks = 5 * 152;
+
+// The smoke mass (sum over interior cells) to the step's statistics.
+struct StoreMass {
+  DevStats* st;
+  __device__ void operator()(const float* r) const { st->smoke_mass = row_sum(r, 0); }
+};
 #endif
 
 }  // namespace

@@ -10,6 +10,8 @@
 // staging value.  The result is written to the rotation partner of the state
 // field and to the staging buffer, after which state and partner swap.
 #include "fg_batch.cuh"
+#include <algorithm>
+
 #include "fg_internal.cuh"
 #include "fg_reduce.cuh"
 
@@ -337,27 +339,25 @@ __device__ __forceinline__ void sl_smoke_cell(int i, int j, const float* __restr
   sl_smoke_value(i, j, Ut, Vt, Ms, Mo, nM, flags, dt, smokeAdv, diffuse, smokeDiffusion, g);
 }
 
-__global__ void k_sl_smoke(const float* __restrict__ Ut, const float* __restrict__ Vt,
-                           const float* __restrict__ Ms, float* __restrict__ Mo, float* nM,
-                           const uint8_t* __restrict__ flags, float dt, float smokeAdv,
-                           int diffuse, float smokeDiffusion, float* __restrict__ mass_part,
-                           Grid g) {
+__global__ void __launch_bounds__(256) k_sl_smoke(
+    const float* __restrict__ Ut, const float* __restrict__ Vt, const float* __restrict__ Ms,
+    float* __restrict__ Mo, float* nM, const uint8_t* __restrict__ flags, float dt, float smokeAdv,
+    int diffuse, float smokeDiffusion, float* __restrict__ mass_part, Grid g, int* ticket,
+    StoreMass store) {
   __shared__ float sh[64];
   pdl_enter();
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF mass{0.0f, 0.0f};
-  if (i < g.NX && j < g.NY) {
-    float m = sl_smoke_value(i, j, Ut, Vt, Ms, Mo, nM, flags, dt, smokeAdv, diffuse,
-                             smokeDiffusion, g);
-    if (!on_ring(i, j, g)) mass.hi = m;
-  }
   // Smoke mass of the result over interior cells (float pairs within the
   // block, FP64 across blocks).
-  if (mass_part) {
-    FF v[1] = {mass};
-    block_row<1>(v, 0u, sh, mass_part + 2 * (size_t)(blockIdx.y * gridDim.x + blockIdx.x));
+  FF v[1] = {{0.0f, 0.0f}};
+  const int tx = (g.NY + BX - 1) / BX, tiles = tx * ((g.NX + BY - 1) / BY);
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int y = t / tx, j = (t - y * tx) * BX + threadIdx.x, i = y * BY + threadIdx.y;
+    if (i >= g.NX || j >= g.NY) continue;
+    const float m = sl_smoke_value(i, j, Ut, Vt, Ms, Mo, nM, flags, dt, smokeAdv, diffuse,
+                                   smokeDiffusion, g);
+    if (!on_ring(i, j, g)) ff_acc(v[0], FF{m, 0.0f});
   }
+  grid_row<1>(v, 0u, sh, mass_part, blockIdx.x, gridDim.x, ticket, store);
 }
 
 // BFECC smoke pass 1 (fluid.go:1007): forward advection into Fm without
@@ -560,12 +560,14 @@ static cudaError_t smoke_pass(fg_fluid* f, const float* Ms, float dt) {
     swap_state(f, FG_M);
     return cudaGetLastError();
   }
-  dim3 gr = cell_grid(f);
-  if (!partials_fit(f, 1, gr.x * gr.y)) return cudaErrorInvalidValue;
-  launch_pdl(k_sl_smoke, gr, dim3(BX, BY), 0, f->stream, f->d[FG_U], f->d[FG_V], Ms,
-             f->partner[FG_M], f->d[FG_NEWM], f->flags, dt, sa, diffuse, sd, f->partials, f->g);
+  const dim3 gr = cell_grid(f);
+  const int nb = (int)std::min<long long>((long long)gr.x * gr.y, kStatBlocks);
+  if (!partials_fit(f, 1, nb)) return cudaErrorInvalidValue;
+  launch_pdl(k_sl_smoke, dim3(nb), dim3(BX, BY), 0, f->stream, f->d[FG_U], f->d[FG_V], Ms,
+             f->partner[FG_M], f->d[FG_NEWM], f->flags, dt, sa, diffuse, sd, f->partials, f->g,
+             &f->dstats->ticket, StoreMass{f->dstats});
   swap_state(f, FG_M);
-  return launch_store_mass(f, gr.x * gr.y);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_advect_smoke(fg_fluid* f, float dt) { return smoke_pass(f, f->d[FG_M], dt); }

@@ -1,6 +1,7 @@
 // Diagnostics and field views (pkg/fluid/fluid.go:529-557, 798-891;
 // pressure.go, smoke.go): reductions accumulate in FP64 through fixed-slot
 // block partials, so repeated runs give identical numbers.
+#include <algorithm>
 #include <cfloat>
 
 #include "fg_internal.cuh"
@@ -13,138 +14,23 @@ constexpr int BX = 32, BY = 8;
 inline dim3 cell_grid(const fg_fluid* f) {
   return dim3((f->NY + BX - 1) / BX, (f->NX + BY - 1) / BY);
 }
-__device__ __forceinline__ int block_id() { return blockIdx.y * gridDim.x + blockIdx.x; }
 __device__ __forceinline__ bool fluid_interior(uint8_t fl) {
   return (fl & (F_FLUID | F_INTERIOR)) == (F_FLUID | F_INTERIOR);
 }
 
-// Post-projection divergence statistics: rows {sum div^2, max |div|, count}
-// over fluid interior cells.
-__global__ void k_div_partials(const float* __restrict__ U, const float* __restrict__ V,
-                               const uint8_t* __restrict__ flags, float* __restrict__ part,
-                               Grid g) {
-  __shared__ float sh[64 * 3];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-  if (j < g.NY && i < g.NX) {
-    int c = i * g.P + j;
-    if (fluid_interior(flags[c])) {
-      float div = U[c + g.P] - U[c] + V[c + 1] - V[c];
-      v[0] = ff_sq(div);
-      v[1].hi = fabsf(div);
-      v[2].hi = 1.0f;
-    }
-  }
-  block_row<3>(v, 2u, sh, part + 6 * (size_t)block_id());
-}
-
-__global__ void k_store_div(const float* __restrict__ r, DevStats* st) {
-  st->div_l2_sq = row_sum(r, 0);
-  st->div_max = (double)r[2];
-  st->div_count = row_sum(r, 2);
-}
-
-// sum of M over interior cells.
-__global__ void k_mass_partials(const float* __restrict__ M, float* __restrict__ part, Grid g) {
-  __shared__ float sh[64];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[1] = {{0.0f, 0.0f}};
-  if (i >= 1 && i <= g.NX - 2 && j >= 1 && j <= g.NY - 2) v[0].hi = M[i * g.P + j];
-  block_row<1>(v, 0u, sh, part + 2 * (size_t)block_id());
-}
-
-struct StoreMass {
+// Where the reductions' total rows go.
+struct StoreDiv {
   DevStats* st;
-  __device__ void operator()(const float* r) const { st->smoke_mass = row_sum(r, 0); }
+  __device__ void operator()(const float* r) const {
+    st->div_l2_sq = row_sum(r, 0);
+    st->div_max = (double)r[2];
+    st->div_count = row_sum(r, 2);
+  }
 };
 
-// MaxDivergence (fluid.go:876-891): float32 |div|, NaN ignored (fmaxf).
-__global__ void k_maxdiv_partials(const float* __restrict__ U, const float* __restrict__ V,
-                                  const uint8_t* __restrict__ flags, float* __restrict__ part,
-                                  Grid g) {
-  __shared__ float sh[64];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[1] = {{0.0f, 0.0f}};
-  if (i < g.NX && j < g.NY) {
-    int c = i * g.P + j;
-    if (fluid_interior(flags[c])) {
-      float div = U[c + g.P] - U[c] + V[c + 1] - V[c];
-      v[0].hi = fabsf(div);
-    }
-  }
-  block_row<1>(v, 1u, sh, part + 2 * (size_t)block_id());
-}
-
-// |U| + |V| on fluid interior cells (GetAdaptiveTimeStep fluid.go:534-543).
-__global__ void k_speed_partials(const float* __restrict__ U, const float* __restrict__ V,
-                                 const uint8_t* __restrict__ flags, float* __restrict__ part,
-                                 Grid g) {
-  __shared__ float sh[64];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[1] = {{0.0f, 0.0f}};
-  if (i < g.NX && j < g.NY) {
-    int c = i * g.P + j;
-    if (fluid_interior(flags[c])) v[0].hi = fabsf(U[c]) + fabsf(V[c]);
-  }
-  block_row<1>(v, 1u, sh, part + 2 * (size_t)block_id());
-}
-
-// Vorticity (fluid.go:806-838, kind 0) and VelocityMagnitude (fluid.go:841-873,
-// kind 1) on fluid interior cells, 0 elsewhere; rows {max v, max -v} over
-// the computed cells (-inf when a block saw none).
-__global__ void k_view(const float* __restrict__ U, const float* __restrict__ V,
-                       const uint8_t* __restrict__ flags, float* __restrict__ out, int kind,
-                       float* __restrict__ part, Grid g) {
-  __shared__ float sh[128];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[2] = {{-INFINITY, 0.0f}, {-INFINITY, 0.0f}};
-  if (i < g.NX && j < g.NY) {
-    int c = i * g.P + j;
-    float x = 0.0f;
-    if (fluid_interior(flags[c])) {
-      if (kind == 0) {
-        float dvdx = (V[c + g.P] - V[c - g.P]) * 0.5f / g.h;
-        float dudy = (U[c + 1] - U[c - 1]) * 0.5f / g.h;
-        x = dvdx - dudy;
-      } else {
-        float u = (U[c] + U[c + g.P]) * 0.5f;
-        float w = (V[c] + V[c + 1]) * 0.5f;
-        x = sqrtf(u * u + w * w);
-      }
-      if (!isnan(x)) {
-        v[0].hi = x;
-        v[1].hi = -x;
-      }
-    }
-    out[c] = x;
-  }
-  block_row<2>(v, 3u, sh, part + 4 * (size_t)block_id());
-}
-
-// min / max over all cells of a field (Pressure(), Smoke()).
-__global__ void k_minmax_partials(const float* __restrict__ F, float* __restrict__ part, Grid g) {
-  __shared__ float sh[128];
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  int i = blockIdx.y * blockDim.y + threadIdx.y;
-  FF v[2] = {{-INFINITY, 0.0f}, {-INFINITY, 0.0f}};
-  if (i < g.NX && j < g.NY) {
-    float x = F[i * g.P + j];
-    if (!isnan(x)) {
-      v[0].hi = x;
-      v[1].hi = -x;
-    }
-  }
-  block_row<2>(v, 3u, sh, part + 4 * (size_t)block_id());
-}
-
 // (max v, max -v) -> float (min, max), with the reference's initial values
-// (MaxFloat32, -MaxFloat32) when no cell was seen.  The results of the
-// reductions go to device or pinned host memory.
+// (MaxFloat32, -MaxFloat32) when no cell was seen. To device or pinned host
+// memory.
 struct StoreMinMax {
   float* out;
   __device__ void operator()(const float* r) const {
@@ -160,6 +46,107 @@ struct StoreMax0 {
   __device__ void operator()(const float* r) const { out[0] = r[0] < 0.0f ? 0.0f : r[0]; }
 };
 
+// body(c) for the cells of a block's tiles.
+template <typename Body>
+__device__ __forceinline__ void each_cell(const Grid& g, Body body) {
+  const int tx = (g.NY + BX - 1) / BX, tiles = tx * ((g.NX + BY - 1) / BY);
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const int y = t / tx, j = (t - y * tx) * BX + threadIdx.x, i = y * BY + threadIdx.y;
+    if (i < g.NX && j < g.NY) body(i * g.P + j);
+  }
+}
+
+// Post-projection divergence statistics: rows {sum div^2, max |div|, count}
+// over fluid interior cells.
+__global__ void __launch_bounds__(256)
+    k_div_stats(const float* __restrict__ U, const float* __restrict__ V,
+                const uint8_t* __restrict__ flags, float* __restrict__ part, Grid g, int* ticket,
+                StoreDiv store) {
+  __shared__ float sh[64 * 3];
+  pdl_enter();
+  FF v[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+  each_cell(g, [&](int c) {
+    if (!fluid_interior(flags[c])) return;
+    float div = U[c + g.P] - U[c] + V[c + 1] - V[c];
+    ff_acc(v[0], ff_sq(div));
+    v[1].hi = fmaxf(v[1].hi, fabsf(div));
+    v[2].hi += 1.0f;
+  });
+  grid_row<3>(v, 2u, sh, part, blockIdx.x, gridDim.x, ticket, store);
+}
+
+// MaxDivergence (fluid.go:876-891): float32 |div|, NaN ignored (fmaxf).
+__global__ void __launch_bounds__(256)
+    k_max_divergence(const float* __restrict__ U, const float* __restrict__ V,
+                     const uint8_t* __restrict__ flags, float* __restrict__ part, Grid g,
+                     int* ticket, StoreMax0 store) {
+  __shared__ float sh[64];
+  FF v[1] = {{0.0f, 0.0f}};
+  each_cell(g, [&](int c) {
+    if (fluid_interior(flags[c]))
+      v[0].hi = fmaxf(v[0].hi, fabsf(U[c + g.P] - U[c] + V[c + 1] - V[c]));
+  });
+  grid_row<1>(v, 1u, sh, part, blockIdx.x, gridDim.x, ticket, store);
+}
+
+// |U| + |V| on fluid interior cells (GetAdaptiveTimeStep fluid.go:534-543).
+__global__ void __launch_bounds__(256)
+    k_max_speed(const float* __restrict__ U, const float* __restrict__ V,
+                const uint8_t* __restrict__ flags, float* __restrict__ part, Grid g, int* ticket,
+                StoreMax0 store) {
+  __shared__ float sh[64];
+  FF v[1] = {{0.0f, 0.0f}};
+  each_cell(g, [&](int c) {
+    if (fluid_interior(flags[c])) v[0].hi = fmaxf(v[0].hi, fabsf(U[c]) + fabsf(V[c]));
+  });
+  grid_row<1>(v, 1u, sh, part, blockIdx.x, gridDim.x, ticket, store);
+}
+
+// A value's part in a range {max v, max -v}: NaN is left out.
+__device__ __forceinline__ void range_of(FF (&v)[2], float x) {
+  if (isnan(x)) return;
+  v[0].hi = fmaxf(v[0].hi, x);
+  v[1].hi = fmaxf(v[1].hi, -x);
+}
+
+// Vorticity (fluid.go:806-838, kind 0) and VelocityMagnitude (fluid.go:841-873,
+// kind 1) on fluid interior cells, 0 elsewhere; rows {max v, max -v} over
+// the computed cells (-inf when a block saw none).
+__global__ void __launch_bounds__(256)
+    k_view(const float* __restrict__ U, const float* __restrict__ V,
+           const uint8_t* __restrict__ flags, float* __restrict__ out, int kind,
+           float* __restrict__ part, Grid g, int* ticket, StoreMinMax store) {
+  __shared__ float sh[128];
+  FF v[2] = {{-INFINITY, 0.0f}, {-INFINITY, 0.0f}};
+  each_cell(g, [&](int c) {
+    float x = 0.0f;
+    if (fluid_interior(flags[c])) {
+      if (kind == 0) {
+        float dvdx = (V[c + g.P] - V[c - g.P]) * 0.5f / g.h;
+        float dudy = (U[c + 1] - U[c - 1]) * 0.5f / g.h;
+        x = dvdx - dudy;
+      } else {
+        float u = (U[c] + U[c + g.P]) * 0.5f;
+        float w = (V[c] + V[c + 1]) * 0.5f;
+        x = sqrtf(u * u + w * w);
+      }
+      range_of(v, x);
+    }
+    out[c] = x;
+  });
+  grid_row<2>(v, 3u, sh, part, blockIdx.x, gridDim.x, ticket, store);
+}
+
+// min / max over all cells of a field (Pressure(), Smoke()).
+__global__ void __launch_bounds__(256)
+    k_field_minmax(const float* __restrict__ F, float* __restrict__ part, Grid g, int* ticket,
+                   StoreMinMax store) {
+  __shared__ float sh[128];
+  FF v[2] = {{-INFINITY, 0.0f}, {-INFINITY, 0.0f}};
+  each_cell(g, [&](int c) { range_of(v, F[c]); });
+  grid_row<2>(v, 3u, sh, part, blockIdx.x, gridDim.x, ticket, store);
+}
+
 __global__ void k_sample_velocity(const float* __restrict__ U, const float* __restrict__ V,
                                   float x, float y, float* __restrict__ out, Grid g) {
   out[0] = sample_field(U, x, y, 0.0f, g.hh, g);
@@ -172,100 +159,57 @@ cudaError_t launch_clear_stats(fg_fluid* f) {
   return cudaMemsetAsync(f->dstats, 0, sizeof(DevStats), f->stream);
 }
 
+// Blocks of a reduction over the cells' tiles, 0 when their rows do not fit.
+static int stat_blocks(const fg_fluid* f, int ns) {
+  const dim3 gr = cell_grid(f);
+  const int nb = (int)std::min<long long>((long long)gr.x * gr.y, kStatBlocks);
+  return partials_fit(f, ns, nb) ? nb : 0;
+}
+
 cudaError_t launch_div_stats(fg_fluid* f) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 3, nb)) return cudaErrorInvalidValue;
+  const int nb = stat_blocks(f, 3);
+  if (!nb) return cudaErrorInvalidValue;
   count(f);
-  k_div_partials<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags,
-                                                     f->partials, f->g);
-  float* out = nullptr;
-  count(f, combine_rows<3>(f->stream, f->partials, nb, 2u, &out));
+  return launch_pdl(k_div_stats, dim3(nb), dim3(BX, BY), 0, f->stream, f->d[FG_U], f->d[FG_V],
+                    f->flags, f->partials, f->g, &f->dstats->ticket, StoreDiv{f->dstats});
+}
+
+cudaError_t launch_max_divergence(fg_fluid* f, float* out) {
+  const int nb = stat_blocks(f, 1);
+  if (!nb) return cudaErrorInvalidValue;
   count(f);
-  k_store_div<<<1, 1, 0, f->stream>>>(out, f->dstats);
+  k_max_divergence<<<nb, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags,
+                                                       f->partials, f->g, &f->dstats->ticket,
+                                                       StoreMax0{out});
   return cudaGetLastError();
 }
 
-cudaError_t launch_store_mass(fg_fluid* f, int nb) {
-  if (!partials_fit(f, 1, nb)) return cudaErrorInvalidValue;
+cudaError_t launch_max_speed(fg_fluid* f, float* out) {
+  const int nb = stat_blocks(f, 1);
+  if (!nb) return cudaErrorInvalidValue;
   count(f);
-  launch_pdl(k_combine_store<1, StoreMass>, dim3(1), dim3(1024), 0, f->stream, f->partials, nb,
-             0u, StoreMass{f->dstats});
+  k_max_speed<<<nb, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags, f->partials,
+                                                  f->g, &f->dstats->ticket, StoreMax0{out});
   return cudaGetLastError();
 }
 
-cudaError_t launch_smoke_mass(fg_fluid* f) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 1, nb)) return cudaErrorInvalidValue;
+cudaError_t launch_view(fg_fluid* f, int kind, float* minmax) {
+  const int nb = stat_blocks(f, 2);
+  if (!nb) return cudaErrorInvalidValue;
   count(f);
-  k_mass_partials<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[FG_M], f->partials, f->g);
-  return launch_store_mass(f, nb);
+  k_view<<<nb, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags, f->view, kind,
+                                             f->partials, f->g, &f->dstats->ticket,
+                                             StoreMinMax{minmax});
+  return cudaGetLastError();
 }
 
-// The total row of nb block rows to `store`: one block while its threads take
-// at most 16 rows each, else after a first level of 2048 rows a block.
-template <int NS, typename Store>
-static cudaError_t finish_rows(fg_fluid* f, int nb, unsigned max_mask, Store store) {
-  const float* rows = f->partials;
-  if (nb > 16384) {
-    float* lvl = f->partials + (size_t)2 * NS * nb;
-    const int g = (nb + 2047) / 2048;
-    count(f);
-    k_combine_rows<NS><<<g, 1024, 0, f->stream>>>(rows, nb, 2048, max_mask, lvl);
-    rows = lvl;
-    nb = g;
-  }
+cudaError_t launch_field_minmax(fg_fluid* f, int field, float* minmax) {
+  const int nb = stat_blocks(f, 2);
+  if (!nb) return cudaErrorInvalidValue;
   count(f);
-  return launch_pdl(k_combine_store<NS, Store>, dim3(1), dim3(1024), 0, f->stream, rows, nb,
-                    max_mask, store);
-}
-
-static cudaError_t finish_max0(fg_fluid* f, int nb, float* out) {
-  return finish_rows<1>(f, nb, 1u, StoreMax0{out});
-}
-
-cudaError_t launch_max_divergence(fg_fluid* f, float* dev_out) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 1, nb)) return cudaErrorInvalidValue;
-  count(f);
-  k_maxdiv_partials<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags,
-                                                        f->partials, f->g);
-  return finish_max0(f, nb, dev_out);
-}
-
-cudaError_t launch_max_speed(fg_fluid* f, float* dev_out) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 1, nb)) return cudaErrorInvalidValue;
-  count(f);
-  k_speed_partials<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags,
-                                                       f->partials, f->g);
-  return finish_max0(f, nb, dev_out);
-}
-
-static cudaError_t finish_minmax(fg_fluid* f, int nb, float* minmax) {
-  return finish_rows<2>(f, nb, 3u, StoreMinMax{minmax});
-}
-
-cudaError_t launch_view(fg_fluid* f, int kind, float* dev_minmax) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 2, nb)) return cudaErrorInvalidValue;
-  count(f);
-  k_view<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[FG_U], f->d[FG_V], f->flags, f->view, kind,
-                                             f->partials, f->g);
-  return finish_minmax(f, nb, dev_minmax);
-}
-
-cudaError_t launch_field_minmax(fg_fluid* f, int field, float* dev_minmax) {
-  dim3 gr = cell_grid(f);
-  int nb = gr.x * gr.y;
-  if (!partials_fit(f, 2, nb)) return cudaErrorInvalidValue;
-  count(f);
-  k_minmax_partials<<<gr, dim3(BX, BY), 0, f->stream>>>(f->d[field], f->partials, f->g);
-  return finish_minmax(f, nb, dev_minmax);
+  k_field_minmax<<<nb, dim3(BX, BY), 0, f->stream>>>(f->d[field], f->partials, f->g,
+                                                     &f->dstats->ticket, StoreMinMax{minmax});
+  return cudaGetLastError();
 }
 
 cudaError_t launch_sample_velocity(fg_fluid* f, float x, float y, float* dev_uv) {

@@ -1363,9 +1363,7 @@ __global__ void k_grad(float* __restrict__ U, float* __restrict__ V, float* __re
 // potential (resid_ff per cell, sum r^2 and max |r|) and, when confinement
 // is off, addTurbulence (fluid.go:496-526), which only touches a cell's own
 // U, V.  Reads U, V and writes the rotated buffers Uo, Vo, so the divergence
-// can recompute a neighbour's projected face from its original value.  A
-// thread handles GR consecutive cells of one column (k_grad_fused below).
-constexpr int GR = 8;
+// can recompute a neighbour's projected face from its original value.
 struct GradAcc {
   FF d2, r2;
   float dmax, rmax, n;
@@ -1382,15 +1380,29 @@ struct GradIn {
   float2 nz;
 };
 
+// Its results: the faces, p, and the faces before turbulence (which a recorded
+// step keeps).
+struct GradOut {
+  float u, v, p, u2, v2;
+};
+
+// addTurbulence (fluid.go:496-526) on a fluid cell's own faces.
+__device__ __forceinline__ void turbulence(float& u, float& v, float2 nz, float turbStrength) {
+  float noiseU = nz.x * turbStrength;
+  float noiseV = nz.y * turbStrength;
+  float localVel = sqrtf(u * u + v * v);
+  if (localVel > 0.1f) {
+    float turbulenceFactor = go_min(localVel * 0.5f, 1.0f);
+    u += noiseU * turbulenceFactor;
+    v += noiseV * turbulenceFactor;
+  }
+}
+
 // The cell's update from its inputs: the projected faces, p, the residual
-// and divergence statistics, turbulence; writes Uo, Vo, p (and the
-// pre-turbulence faces U2o, V2o of a recorded step).
-__device__ __forceinline__ void grad_apply(int c, bool hasL, bool hasR, bool hasB, bool hasT,
-                                           const GradIn& in, float* __restrict__ Uo,
-                                           float* __restrict__ Vo, float* __restrict__ p,
-                                           float cp, float turbStrength, int do_turb,
-                                           GradAcc& acc, float* __restrict__ U2o,
-                                           float* __restrict__ V2o) {
+// and divergence statistics, turbulence.
+__device__ __forceinline__ GradOut grad_apply(bool hasL, bool hasR, bool hasB, bool hasT,
+                                              const GradIn& in, float cp, float turbStrength,
+                                              int do_turb, GradAcc& acc) {
   const uint8_t fl = in.fl, fR = in.fR, fT = in.fT;
   const bool act = flag_active(fl), aL = flag_active(in.fL), aR = flag_active(fR);
   const bool aB = flag_active(in.fB), aT = flag_active(fT);
@@ -1398,12 +1410,15 @@ __device__ __forceinline__ void grad_apply(int c, bool hasL, bool hasR, bool has
   float u = in.u, v = in.v;
   if (hasL && hasB && hasT && (act || aL)) u = u + (fbit(fl, F_FLUID) * pL - fbit(fl, F_W) * pc);
   if (hasB && hasL && hasR && (act || aB)) v = v + (fbit(fl, F_FLUID) * pB - fbit(fl, F_S) * pc);
-  p[c] = act ? cp * pc : 0.0f;
+  GradOut out;
+  out.p = act ? cp * pc : 0.0f;
+  out.u2 = u;
+  out.v2 = v;
   if (act) {
     FF r = resid_ff(in.bc, pL, pR, pB, pT, (float)flag_count(fl), pc);
     FF q = ff_sq(r.hi);
     q.lo = q.lo + 2.0f * r.hi * r.lo;
-    acc.r2 = ff_add(acc.r2, q);
+    ff_acc(acc.r2, q);
     acc.rmax = fmaxf(acc.rmax, fabsf(r.hi));
   }
   if ((fl & (F_FLUID | F_INTERIOR)) == (F_FLUID | F_INTERIOR)) {
@@ -1413,31 +1428,41 @@ __device__ __forceinline__ void grad_apply(int c, bool hasL, bool hasR, bool has
     float vT = in.vT0;
     if (act || aT) vT = vT + (fbit(fT, F_FLUID) * pc - fbit(fT, F_S) * pT);
     float div = uR - u + vT - v;
-    acc.d2 = ff_add(acc.d2, ff_sq(div));
+    ff_acc(acc.d2, ff_sq(div));
     acc.dmax = fmaxf(acc.dmax, fabsf(div));
     acc.n = acc.n + 1.0f;
-    if (U2o) {
-      // The projected field before turbulence (a recorded step keeps it).
-      U2o[c] = u;
-      V2o[c] = v;
-    }
-    if (do_turb) {
-      float noiseU = in.nz.x * turbStrength;
-      float noiseV = in.nz.y * turbStrength;
-      float localVel = sqrtf(u * u + v * v);
-      if (localVel > 0.1f) {
-        float turbulenceFactor = go_min(localVel * 0.5f, 1.0f);
-        u += noiseU * turbulenceFactor;
-        v += noiseV * turbulenceFactor;
-      }
-    }
+    if (do_turb) turbulence(u, v, in.nz, turbStrength);
   }
-  if (U2o && (fl & (F_FLUID | F_INTERIOR)) != (F_FLUID | F_INTERIOR)) {
-    U2o[c] = u;
-    V2o[c] = v;
-  }
-  Uo[c] = u;
-  Vo[c] = v;
+  out.u = u;
+  out.v = v;
+  return out;
+}
+
+// grad_apply of a plain cell: an interior fluid cell with four fluid
+// neighbours (flags kPlain), whose bits are all 1 and whose neighbours' flags
+// say nothing more.  The same operations without the factors of 1.
+constexpr uint8_t kPlain = F_W | F_E | F_S | F_N | F_FLUID | F_INTERIOR;
+__device__ __forceinline__ GradOut grad_plain(const GradIn& in, float cp, float turbStrength,
+                                              int do_turb, GradAcc& acc) {
+  GradOut out;
+  float u = in.u + (in.pL - in.pc), v = in.v + (in.pB - in.pc);
+  out.p = cp * in.pc;
+  const FF r = resid_ff(in.bc, in.pL, in.pR, in.pB, in.pT, 4.0f, in.pc);
+  FF q = ff_sq(r.hi);
+  q.lo = q.lo + 2.0f * r.hi * r.lo;
+  ff_acc(acc.r2, q);
+  acc.rmax = fmaxf(acc.rmax, fabsf(r.hi));
+  const float uR = in.uR0 + (in.pc - in.pR), vT = in.vT0 + (in.pc - in.pT);
+  const float div = uR - u + vT - v;
+  ff_acc(acc.d2, ff_sq(div));
+  acc.dmax = fmaxf(acc.dmax, fabsf(div));
+  acc.n = acc.n + 1.0f;
+  out.u2 = u;
+  out.v2 = v;
+  if (do_turb) turbulence(u, v, in.nz, turbStrength);
+  out.u = u;
+  out.v = v;
+  return out;
 }
 
 __device__ __forceinline__ void grad_cell(int i, int j, const float* __restrict__ U,
@@ -1492,22 +1517,49 @@ __device__ __forceinline__ void grad_cell(int i, int j, const float* __restrict_
   in.vT0 = with_force(V, Fv, cT);
   in.bc = rhs[c];
   in.nz = do_turb ? noise[c] : make_float2(0.0f, 0.0f);
-  grad_apply(c, hasL, hasR, hasB, hasT, in, Uo, Vo, p, cp, turbStrength, do_turb, acc, U2o, V2o);
+  const GradOut o = grad_apply(hasL, hasR, hasB, hasT, in, cp, turbStrength, do_turb, acc);
+  Uo[c] = o.u;
+  Vo[c] = o.v;
+  p[c] = o.p;
+  if (U2o) {
+    U2o[c] = o.u2;
+    V2o[c] = o.v2;
+  }
 }
 
-// The gradient subtract and its fused statistics over GR consecutive rows
-// per thread (a block of 32 x 8 threads covers 32 columns x 8 GR rows): on
-// interior strips the flags, the final potential and U of rows i-1, i, i+1
-// roll from row to row instead of being loaded again (about 14 loads per
-// cell instead of 19); each cell's inputs and update are grad_cell's.
-// Strips at the domain edge run grad_cell row by row.
-__device__ __forceinline__ float phi_fin(const float* __restrict__ phi,
-                                         const float* __restrict__ e, int c) {
-  float x = phi[c];
-  if (e) x = x + e[c];
-  return x;
-}
-__global__ void __launch_bounds__(256)
+// The step's statistics from the combined row of k_grad_fused's partials
+// (sum div^2, max |div|, fluid cells, sum r^2, max |r|) and, after a solve,
+// its sweep count and last checked max |r| from the control block.
+struct StoreDivP {
+  DevStats* st;
+  const PCtl* ctl;
+  __device__ void operator()(const float* r) const {
+    st->div_l2_sq = row_sum(r, 0);
+    st->div_max = (double)r[2];
+    st->div_count = row_sum(r, 2);
+    st->resid_l2_sq = row_sum(r, 3);
+    st->resid_max = (double)r[8];
+    if (ctl) {
+      st->sweeps = ctl->sweeps;
+      st->last_maxdiv = (double)__uint_as_float(ctl->slots[ctl->last_launch]);
+    }
+  }
+};
+
+// The gradient subtract and its fused statistics, 4 columns of a row a thread
+// at a time: fields move in 16-byte pieces (rows start on 128 bytes; a piece
+// past the last column reads pitch padding, which nothing uses).  At most
+// kGradBlocks blocks walk the grid, three an SM (76 registers a thread), so
+// the reduction at the end of a block is paid once per block and its rows are
+// few enough to combine in the same launch.  Plain cells take 150 operations
+// of the 240 the flag-by-flag form takes.  With the combining (us; before:
+// one column of 8 rows a thread and a second launch): 128 x 128 9.5 (11.7 +
+// 4.9), 512 x 256 9.4 (11.4 + 5.3), 1500 x 1100 25 (27.7 + 5.9), 2048 x 2048
+// 41.6 (56 + 7.1).  One piece a thread in 4109 blocks: 66; two rows a piece 82.
+constexpr int kGradBlocks = 3 * 152;
+// REC: a recorded step (force fields, the faces before turbulence kept).
+template <bool REC>
+__global__ void __launch_bounds__(256, 3)
     k_grad_fused(const float* __restrict__ U, const float* __restrict__ V,
                  float* __restrict__ Uo, float* __restrict__ Vo, float* __restrict__ p,
                  const float* __restrict__ phi0, const float* __restrict__ phi1,
@@ -1517,61 +1569,101 @@ __global__ void __launch_bounds__(256)
                  const float2* __restrict__ noise, float turbStrength, int do_turb,
                  float* __restrict__ part, Grid g, const float* __restrict__ Fu,
                  const float* __restrict__ Fv, float* __restrict__ U2o,
-                 float* __restrict__ V2o) {
+                 float* __restrict__ V2o, int* ticket, StoreDivP store) {
   __shared__ float shr[64 * 5];
   pdl_enter();
+  const float *fu = REC ? Fu : nullptr, *fv = REC ? Fv : nullptr;
   const float* phi = ctl->sel ? phi1 : phi0;
   const float* e = ectl ? (ectl->sel ? e1 : e0) : nullptr;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i0 = (blockIdx.y * blockDim.y + threadIdx.y) * GR;
+  const int nq = (g.NY + 3) / 4, total = nq * g.NX, P = g.P;
   GradAcc acc{{0.0f, 0.0f}, {0.0f, 0.0f}, 0.0f, 0.0f, 0.0f};
-  if (j < g.NY && i0 < g.NX) {
-    if (j >= 1 && j <= g.NY - 2 && i0 >= 1 && i0 + GR - 1 <= g.NX - 2) {
-      const int P = g.P;
-      int c = i0 * P + j;
-      uint8_t fprev = flags[c - P], fcur = flags[c];
-      float pprev = phi_fin(phi, e, c - P), pcur = phi_fin(phi, e, c);
-      float ucur = with_force(U, Fu, c);
-#pragma unroll
-      for (int r = 0; r < GR; ++r) {
-        const uint8_t fnext = flags[c + P];
-        const float pnext = phi_fin(phi, e, c + P);
-        const float unext = with_force(U, Fu, c + P);
-        GradIn in;
-        in.fl = fcur;
-        in.fL = fprev;
-        in.fR = fnext;
-        in.fB = flags[c - 1];
-        in.fT = flags[c + 1];
-        in.pc = pcur;
-        in.pL = pprev;
-        in.pR = pnext;
-        in.pB = phi_fin(phi, e, c - 1);
-        in.pT = phi_fin(phi, e, c + 1);
-        in.u = ucur;
-        in.v = with_force(V, Fv, c);
-        in.uR0 = unext;
-        in.vT0 = with_force(V, Fv, c + 1);
-        in.bc = rhs[c];
-        in.nz = do_turb ? noise[c] : make_float2(0.0f, 0.0f);
-        grad_apply(c, true, true, true, true, in, Uo, Vo, p, cp, turbStrength, do_turb, acc, U2o,
-                   V2o);
-        fprev = fcur;
-        fcur = fnext;
-        pprev = pcur;
-        pcur = pnext;
-        ucur = unext;
-        c += P;
+  for (int idx = blockIdx.x * 256 + threadIdx.x; idx < total; idx += gridDim.x * 256) {
+    const int i = idx / nq, j = 4 * (idx - i * nq);
+    auto ld4 = [](const float* x, int c) { return *reinterpret_cast<const float4*>(x + c); };
+    auto sum4 = [&](const float* x, const float* y, int c) {
+      float4 a = ld4(x, c);
+      if (y) {
+        const float4 b = ld4(y, c);
+        a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
       }
+      return a;
+    };
+    auto sum1 = [](const float* x, const float* y, int c) { return y ? x[c] + y[c] : x[c]; };
+    auto fl4 = [&](int c) { return *reinterpret_cast<const uint32_t*>(flags + c); };
+    auto at = [](const float4& x, int k) { return k == 0 ? x.x : k == 1 ? x.y : k == 2 ? x.z : x.w; };
+    auto fat = [](uint32_t x, int k) { return (uint8_t)(x >> 8 * k); };
+    const bool more = j + 4 < g.NY;  // the column right of the piece is a cell
+    const int c = i * P + j;
+    const bool hasL = i >= 1, hasR = i <= g.NX - 2;
+    // (Off the grid: the row itself, masked below.)
+    const int cl = hasL ? c - P : c, cn = hasR ? c + P : c;
+    const float4 pprev = sum4(phi, e, cl), pcur = sum4(phi, e, c), pnext = sum4(phi, e, cn);
+    const float4 ucur = sum4(U, fu, c), unext = sum4(U, fu, cn);
+    const uint32_t f = fl4(c);
+    const float4 v = sum4(V, fv, c), b = ld4(rhs, c);
+    const float pl = j >= 1 ? sum1(phi, e, c - 1) : 0.0f;
+    const float pr = more ? sum1(phi, e, c + 4) : 0.0f;
+    const float vr = more ? sum1(V, fv, c + 4) : 0.0f;
+    float4 n0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), n1 = n0;
+    if (do_turb) {
+      n0 = ld4(reinterpret_cast<const float*>(noise + c), 0);
+      n1 = ld4(reinterpret_cast<const float*>(noise + c), 4);
+    }
+    GradIn in[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool hasT = j + k <= g.NY - 2;
+      in[k].pc = at(pcur, k);
+      in[k].pL = hasL ? at(pprev, k) : 0.0f;
+      in[k].pR = hasR ? at(pnext, k) : 0.0f;
+      in[k].pB = k ? at(pcur, k - 1) : pl;
+      in[k].pT = !hasT ? 0.0f : k < 3 ? at(pcur, k + 1) : pr;
+      in[k].u = at(ucur, k);
+      in[k].v = at(v, k);
+      in[k].uR0 = at(unext, k);
+      in[k].vT0 = k < 3 ? at(v, k + 1) : vr;
+      in[k].bc = at(b, k);
+      in[k].nz = k == 0 ? make_float2(n0.x, n0.y) : k == 1 ? make_float2(n0.z, n0.w)
+                 : k == 2 ? make_float2(n1.x, n1.y) : make_float2(n1.z, n1.w);
+    }
+    float o[5][4];
+    auto out = [&](int k, const GradOut& x) {
+      o[0][k] = x.u; o[1][k] = x.v; o[2][k] = x.p; o[3][k] = x.u2; o[4][k] = x.v2;
+    };
+    if (more && f == kPlain * 0x01010101u) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) out(k, grad_plain(in[k], cp, turbStrength, do_turb, acc));
     } else {
-      for (int r = 0; r < GR && i0 + r < g.NX; ++r)
-        grad_cell(i0 + r, j, U, V, Uo, Vo, p, phi, e, rhs, flags, cp, noise, turbStrength,
-                  do_turb, g, acc, Fu, Fv, U2o, V2o);
+      const uint32_t fp = hasL ? fl4(c - P) : 0, fn = hasR ? fl4(cn) : 0;
+      const uint8_t fb = j >= 1 ? flags[c - 1] : 0, ft = more ? flags[c + 4] : 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool hasB = j + k >= 1, hasT = j + k <= g.NY - 2;
+        if (j + k >= g.NY) continue;
+        in[k].fl = fat(f, k);
+        in[k].fL = fat(fp, k);
+        in[k].fR = fat(fn, k);
+        in[k].fB = k ? fat(f, k - 1) : fb;
+        in[k].fT = !hasT ? 0 : k < 3 ? fat(f, k + 1) : ft;
+        out(k, grad_apply(hasL, hasR, hasB, hasT, in[k], cp, turbStrength, do_turb, acc));
+      }
+    }
+    float* dst[5] = {Uo, Vo, p, U2o, V2o};
+#pragma unroll
+    for (int q = 0; q < 5; ++q) {
+      if (q >= 3 && !(REC && U2o)) break;
+      if (j + 4 <= g.NY) {
+        *reinterpret_cast<float4*>(dst[q] + c) = make_float4(o[q][0], o[q][1], o[q][2], o[q][3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (j + k < g.NY) dst[q][c + k] = o[q][k];
+      }
     }
   }
   // Row slots: sum div^2, max |div|, fluid cells (exact), sum r^2, max |r|.
   FF row[5] = {acc.d2, {acc.dmax, 0.0f}, {acc.n, 0.0f}, acc.r2, {acc.rmax, 0.0f}};
-  block_row<5, 0x4u>(row, 0x12u, shr, part + 10 * (size_t)(blockIdx.y * gridDim.x + blockIdx.x));
+  grid_row<5, 0x4u>(row, 0x12u, shr, part, blockIdx.x, gridDim.x, ticket, store);
 }
 
 // Copies the solve's final potential (the buffer the control block names),
@@ -1605,26 +1697,6 @@ __device__ __forceinline__ void grad_batch_cell(int i, int j, const float* __res
   grad_cell(i, j, U, V, Uo, Vo, p, ctl->sel ? phi1 : phi0, nullptr, rhs, flags, cp, noise,
             turbStrength, do_turb, g, acc, nullptr, nullptr, U2o, V2o);
 }
-
-// The step's statistics from the combined row of k_grad_fused's partials
-// (sum div^2, max |div|, fluid cells, sum r^2, max |r|) and, after a solve,
-// its sweep count and last checked max |r| from the control block.
-struct StoreDivP {
-  DevStats* st;
-  const PCtl* ctl;
-  __device__ void operator()(const float* r) const {
-    st->div_l2_sq = row_sum(r, 0);
-    st->div_max = (double)r[2];
-    st->div_count = row_sum(r, 2);
-    st->resid_l2_sq = row_sum(r, 3);
-    st->resid_max = (double)r[8];
-    if (ctl) {
-      st->sweeps = ctl->sweeps;
-      st->last_maxdiv = (double)__uint_as_float(ctl->slots[ctl->last_launch]);
-    }
-  }
-};
-
 
 }  // namespace
 
@@ -2564,6 +2636,25 @@ cudaError_t launch_mg_rebuild(fg_fluid* f) {
   return cudaGetLastError();
 }
 
+// The gradient subtract; swaps in the projected U, V.  `ticket`: where the
+// statistics are combined (null: they are not).
+static cudaError_t launch_grad_fused(fg_fluid* f, PCtl* ctl, PCtl* ectl, const float* phi0,
+                                     const float* phi1, float cp, float dt, bool fuse_turb,
+                                     int* ticket, StoreDivP store) {
+  const long long pieces = (long long)((f->NY + 3) / 4) * f->NX;
+  const int nb = (int)std::min<long long>((pieces + 255) / 256, kGradBlocks);
+  if (!partials_fit(f, 5, nb)) return cudaErrorInvalidValue;
+  count(f);
+  cudaError_t e = launch_pdl(
+      f->step_fu || f->step_u2 ? k_grad_fused<true> : k_grad_fused<false>, dim3(nb), dim3(256), 0, f->stream, f->d[FG_U], f->d[FG_V], f->partner[FG_U],
+      f->partner[FG_V], f->d[FG_P], phi0, phi1, ctl, f->err, f->err2, ectl, f->rhs, f->flags, cp,
+      f->noise, f->prm.turbulence_strength * dt, fuse_turb ? 1 : 0, f->partials, f->g, f->step_fu,
+      f->step_fv, f->step_u2, f->step_v2, ticket, store);
+  swap_state(f, FG_U);
+  swap_state(f, FG_V);
+  return e;
+}
+
 cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb) {
   float cp = f->density * f->h / dt;  // fluid.go:158
   cudaError_t e;
@@ -2613,21 +2704,8 @@ cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb
       return e;
     mark(f, "outer correction");
   }
-  dim3 rg((f->NY + BX - 1) / BX, (f->NX + BY * GR - 1) / (BY * GR));
-  int nb = rg.x * rg.y;
-  if (!partials_fit(f, 5, nb)) return cudaErrorInvalidValue;
-  count(f);
-  launch_pdl(k_grad_fused, rg, bl, 0, f->stream, f->d[FG_U], f->d[FG_V], f->partner[FG_U],
-             f->partner[FG_V], f->d[FG_P], f->phi, f->phi2, ctl, f->err, f->err2,
-             refine ? ectl : nullptr, f->rhs, f->flags, cp, f->noise,
-             f->prm.turbulence_strength * dt, fuse_turb ? 1 : 0, f->partials, f->g, f->step_fu,
-             f->step_fv, f->step_u2, f->step_v2);
-  swap_state(f, FG_U);
-  swap_state(f, FG_V);
-  count(f);
-  launch_pdl(k_combine_store<5, StoreDivP>, dim3(1), dim3(1024), 0, f->stream, f->partials, nb,
-             0x12u, StoreDivP{f->dstats, num_iters > 0 ? ctl : nullptr});
-  return cudaGetLastError();
+  return launch_grad_fused(f, ctl, refine ? ectl : nullptr, f->phi, f->phi2, cp, dt, fuse_turb,
+                           &f->dstats->ticket, StoreDivP{f->dstats, num_iters > 0 ? ctl : nullptr});
 }
 
 cudaError_t launch_store_phi(fg_fluid* f, float* dst) {
@@ -2654,19 +2732,10 @@ cudaError_t launch_grad_replay(fg_fluid* f, float dt, const float* phi, bool fus
     swap_state(f, FG_V);
     return cudaGetLastError();
   }
-  dim3 rg((f->NY + BX - 1) / BX, (f->NX + BY * GR - 1) / (BY * GR)), bl(BX, BY);
-  if (!partials_fit(f, 5, rg.x * rg.y)) return cudaErrorInvalidValue;
-  count(f);
   // The potential is the same buffer whichever one the control block names;
   // the statistics partials it writes are not combined.
-  k_grad_fused<<<rg, bl, 0, f->stream>>>(
-      f->d[FG_U], f->d[FG_V], f->partner[FG_U], f->partner[FG_V], f->d[FG_P], phi, phi,
-      (const PCtl*)f->pctl, nullptr, nullptr, nullptr, f->rhs, f->flags, cp, f->noise,
-      f->prm.turbulence_strength * dt, fuse_turb ? 1 : 0, f->partials, f->g, f->step_fu,
-      f->step_fv, f->step_u2, f->step_v2);
-  swap_state(f, FG_U);
-  swap_state(f, FG_V);
-  return cudaGetLastError();
+  return launch_grad_fused(f, (PCtl*)f->pctl, nullptr, phi, phi, cp, dt, fuse_turb, nullptr,
+                           StoreDivP{});
 }
 
 }  // namespace fg
