@@ -2007,59 +2007,69 @@ int batch_pack(fg_fluid* f) {
   return FG_OK;
 }
 
-// Plans the batch's resident Jacobi solves: for each form, groups of whole
-// scenes (in the order jord: more sweeps first) whose regions fit the GPU at
-// once, evenly filled; the form whose groups' phases take least (measured per
-// phase, 3 us a launch), if that is less than the launches of 8 sweeps over
-// all started regions (2.4 us each and 6.2 us per 304 regions; 21 scenes of
-// 64^2-512^2: 8.7 us each).
+// Plans the batch's resident Jacobi solves: for either height of a region, the
+// scenes (in the order jord: more sweeps first) split into groups that fit the
+// GPU at once so that the groups' phases take least -- each group at the time
+// per phase of the fastest form that holds it, and 3 us a launch -- if that is
+// less than the launches of 8 sweeps over all started regions (2.4 us each and
+// 6.2 us per 304 regions).  21 scenes of 64^2-512^2 with 309 regions: 8.7 us
+// per 8 sweeps and 252 us a step by launches, 295 in two equal groups of
+// 8-warp regions, 224 as planned here (two unequal ones of 12 warps).
 int batch_resident(fg_fluid* f, const std::vector<int>& jord) {
   BatchGeom* b = f->batch;
   JresForm forms[3];
   jres_batch_forms(forms);
+  auto phases = [&](size_t s) { return (b->jac_iters[s] + kJacHalo - 1) / kJacHalo; };
+  const size_t n = jord.size();
   double best = 0.0;
   for (int k = 0; k < (b->max_iters + kJacHalo - 1) / kJacHalo; ++k) {
     int started = 0;
-    for (size_t s = 0; s < jord.size(); ++s)
-      if ((b->jac_iters[s] + kJacHalo - 1) / kJacHalo > k) started += b->jac_regions[s];
+    for (size_t s = 0; s < n; ++s)
+      if (phases(s) > k) started += b->jac_regions[s];
     best += 2.4 + 6.2 * started / 304.0;
   }
-  for (const JresForm& fm : forms) {
-    if (fm.cap <= 0) continue;
+  int rows = 0;
+  for (int r : {64, 96}) {
     std::vector<int> size;
-    int total = 0, largest = 0;
     for (int s : jord) {
       const Grid& g = b->scenes[s].g;
-      size.push_back(span_count(g.NX, fm.rows) * span_count(g.NY, kJacRegionCols));
-      total += size.back();
-      largest = std::max(largest, size.back());
+      size.push_back(span_count(g.NX, r) * span_count(g.NY, kJacRegionCols));
     }
-    if (largest > fm.cap) continue;
-    const int n_groups = (total + fm.cap - 1) / fm.cap, want = (total + n_groups - 1) / n_groups;
-    std::vector<std::pair<int, int>> groups;
-    double us = 0.0;
-    int first = 0, held = 0;
-    for (size_t s = 0; s <= size.size(); ++s) {
-      if (s == size.size() || (held > 0 && (held + size[s] > fm.cap || held >= want))) {
-        groups.push_back({first, held});
-        first += held;
-        held = 0;
-        if (s == size.size()) break;
+    // us[e]: the least time of the first e scenes, their last group from[e]..e.
+    std::vector<double> us(n + 1, 1e30);
+    std::vector<size_t> from(n + 1, 0);
+    std::vector<int> form(n + 1, 0);
+    us[0] = 0.0;
+    for (size_t s = 0; s < n; ++s) {
+      int held = 0;
+      for (size_t e = s + 1; e <= n; ++e) {
+        held += size[e - 1];
+        const JresForm* fit = nullptr;
+        for (const JresForm& fm : forms)
+          if (fm.rows == r && held <= fm.cap && (!fit || fm.us < fit->us)) fit = &fm;
+        if (!fit) break;
+        const double t = us[s] + 3.0 + fit->us * phases(s);
+        if (t < us[e]) {
+          us[e] = t;
+          from[e] = s;
+          form[e] = fit->form;
+        }
       }
-      if (held == 0) us += 3.0 + fm.us * ((b->jac_iters[s] + kJacHalo - 1) / kJacHalo);
-      held += size[s];
     }
-    if (us >= best) continue;
-    best = us;
-    b->res_form = fm.form;
-    b->res_groups = groups;
+    if (us[n] >= best) continue;
+    best = us[n];
+    rows = r;
+    b->res_groups.clear();
     b->res_cap = 0;
-    for (const auto& gp : groups) b->res_cap = std::max(b->res_cap, gp.second);
+    std::vector<int> first(n + 1, 0);
+    for (size_t s = 0; s < n; ++s) first[s + 1] = first[s] + size[s];
+    for (size_t e = n; e > 0; e = from[e]) {
+      b->res_groups.push_back({first[from[e]], first[e] - first[from[e]], form[e]});
+      b->res_cap = std::max(b->res_cap, b->res_groups.back().count);
+    }
+    std::reverse(b->res_groups.begin(), b->res_groups.end());
   }
   if (!b->res_cap) return FG_OK;
-  int rows = 0;
-  for (const JresForm& fm : forms)
-    if (fm.form == b->res_form) rows = fm.rows;
   std::vector<JRegion> rg;
   for (int s : jord) {
     const BScene& sc = b->scenes[s];

@@ -277,6 +277,11 @@ struct JRegion {
 // Regions a resident Jacobi solve's buffers are made for at most.
 constexpr int JRES_MAX_REGIONS = 512;
 
+// A group of a batch's resident solve: its regions in the table and the form
+// (regions of 8 or 12 warps, one or two an SM) it runs in.
+struct ResGroup {
+  int first, count, form;
+};
 struct BatchGeom {
   int n = 0;
   std::vector<BScene> scenes;
@@ -295,11 +300,11 @@ struct BatchGeom {
   // launch runs only the table's prefix of scenes that have started.
   std::vector<int> jac_iters, jac_regions;
   int max_iters = 0;
-  // Resident solves: every region, and groups (first region, regions) of
-  // whole scenes that are solved one after the other; res_cap the largest.
+  // Resident solves: every region, and groups of whole scenes that are solved
+  // one after the other; res_cap the largest group's regions.
   JRegion* res_regions = nullptr;
-  std::vector<std::pair<int, int>> res_groups;
-  int res_cap = 0, res_form = 0;
+  std::vector<ResGroup> res_groups;
+  int res_cap = 0;
   int* src_scene = nullptr;  // device: scene of each source group
   double* losses = nullptr;  // device: per-scene loss of the last seed, then n floats 1 / L
 };

@@ -1084,7 +1084,7 @@ struct JResArgs {
   int iters;
   unsigned* epoch;             // per block: the tag its last solve ended on (all alike)
   unsigned inc;                // the launch's phases (a batch: of its longest solve)
-  int count;                   // regions; the blocks past them only keep their epoch
+  int cap;                     // a batch: the regions of its largest group
   uint4* pkt;                  // [region][parity][JSlot::N]
   PCtl* ctl;
   const JRegion* regions;      // batch: the launch's regions (nullptr: one grid)
@@ -1124,10 +1124,6 @@ __global__ void __launch_bounds__(32 * NW, MB) k_jacobi_res(JResArgs a) {
   __shared__ JRegion rg;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, id = blockIdx.x;
   const unsigned epoch = a.epoch[id];
-  if (BATCH && id >= a.count) {
-    if (tid == 0) a.epoch[id] = epoch + a.inc;
-    return;
-  }
   if (BATCH) {
     if (tid == 0) rg = a.regions[id];
   } else if (tid == 0) {
@@ -1285,6 +1281,9 @@ __global__ void __launch_bounds__(32 * NW, MB) k_jacobi_res(JResArgs a) {
   }
   if (tid == 0) {
     a.epoch[id] = epoch + a.inc;
+    // (A batch's groups share the slots: those this one does not use keep step.)
+    if (BATCH)
+      for (int k = id + gridDim.x; k < a.cap; k += gridDim.x) a.epoch[k] = epoch + a.inc;
     if (fail) atomicExch(a.err, 1);
     if (id == 0) {
       a.ctl->sweeps = iters;
@@ -2079,7 +2078,7 @@ void jres_batch_forms(JresForm (&out)[3]) {
   const TmaDevice* d = tma_device();
   const bool ok = d && d->ready.load();
   const int form[3] = {JRES_8, JRES_12, JRES_8X2};
-  const float us[3] = {3.0f, 4.1f, 6.2f};
+  const float us[3] = {3.0f, 4.1f, 6.0f};
   for (int k = 0; k < 3; ++k) {
     int cap = !ok ? 0 : form[k] == JRES_8X2 ? d->res_blocks[JRES_8X2]
                                             : std::min(d->sms, d->res_blocks[form[k]]);
@@ -2160,7 +2159,7 @@ static cudaError_t jacobi_solve_batch(fg_fluid* f, PCtl* ctl, const float* bw, f
   const int pf_blocks = dv && dv->sms > 0 ? dv->batch_pf_per_sm * dv->sms : 0;
   // Groups of scenes whose regions fit the GPU at once, each group's whole
   // solve one resident launch.
-  if (f->jres && dv && bt->res_regions && bt->res_cap > 0 && dv->res_blocks[bt->res_form] >= bt->res_cap) {
+  if (f->jres && dv && bt->res_regions && bt->res_cap > 0) {
     JResArgs a = {};
     a.x = x0;
     a.W = f->wgt;
@@ -2173,13 +2172,14 @@ static cudaError_t jacobi_solve_batch(fg_fluid* f, PCtl* ctl, const float* bw, f
     unsigned* epochs = static_cast<unsigned*>(f->jres);
     uint4* pkts = reinterpret_cast<uint4*>(epochs + JRES_MAX_REGIONS);
     bool ok = true;
-    for (const auto& gp : bt->res_groups) {  // (groups run in turn: they share the buffers)
+    for (const ResGroup& gp : bt->res_groups) {  // (groups run in turn: they share the buffers)
       a.regions = bt->res_regions + gp.first;
-      a.count = gp.second;
+      a.cap = bt->res_cap;
       a.inc = (unsigned)((bt->max_iters + TMAX - 1) / TMAX);
       a.epoch = epochs;
       a.pkt = pkts;
-      ok = launch_res(f->stream, a, om1 == 0.0f, true, bt->res_form, bt->res_cap) == cudaSuccess;
+      ok = dv->res_blocks[gp.form] >= gp.count &&
+           launch_res(f->stream, a, om1 == 0.0f, true, gp.form, gp.count) == cudaSuccess;
       if (!ok) break;
       count(f);
     }
