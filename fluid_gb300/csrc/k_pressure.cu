@@ -2343,6 +2343,7 @@ __global__ void k_mg_restrict(const float* __restrict__ xf, const float* __restr
                               const uint8_t* __restrict__ flf, Grid gf,
                               const uint8_t* __restrict__ flc, const float* __restrict__ wc,
                               float* __restrict__ bc, float* __restrict__ bwc, Grid gc) {
+  pdl_enter();
   int J = blockIdx.x * blockDim.x + threadIdx.x;
   int I = blockIdx.y * blockDim.y + threadIdx.y;
   if (I < 1 || J < 1 || I > gc.NX - 2 || J > gc.NY - 2) return;
@@ -2374,6 +2375,7 @@ __device__ __forceinline__ void mg_prolong_cell(int i, int j, const float* __res
 }
 __global__ void k_mg_prolong(const float* __restrict__ xc, const uint8_t* __restrict__ flc, Grid gc,
                              float* __restrict__ xf, const uint8_t* __restrict__ flf, Grid gf) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i < 1 || j < 1 || i > gf.NX - 2 || j > gf.NY - 2) return;
@@ -2447,6 +2449,7 @@ __global__ void __launch_bounds__(kMgFuseThreads)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kMgFuseThreads / 32;
   uint8_t* bsm = reinterpret_cast<uint8_t*>(mg_smem);
   const int last = m.n - 1;
+  pdl_enter();
   for (int l = 0; l <= last; ++l) {
     const MgSm a = mg_sm(m, l, mg_smem, bsm);
     const Grid& gg = m.gg[l];
@@ -2499,10 +2502,9 @@ void mg_sweeps(cudaStream_t st, const MgLevelDev& v, const float* src, float* ds
   const TmaDevice* dv = tma_ready(st);
   const bool narrow = dv && dv->sms > 0 && (long long)gr.x * gr.y < dv->sms;
 #define FG_MGJ(F, NW)                                                                           \
-  k_jacobi_rb<false, F, false, false, NW>                                                       \
-      <<<dim3(gr.x, span_count(v.g.NX, RT * NW)), 32 * NW, 0, st>>>(                            \
-          src, dst, v.w, v.bw, nullptr, v.flags, om1, ctl, 0, t0, ns, 0.0f, sel, zero, v.g,     \
-          nullptr, nullptr, nullptr, nullptr, nullptr)
+  launch_pdl(k_jacobi_rb<false, F, false, false, NW>, dim3(gr.x, span_count(v.g.NX, RT * NW)),  \
+             dim3(32 * NW), 0, st, src, dst, v.w, v.bw, nullptr, v.flags, om1, ctl, 0, t0, ns,  \
+             0.0f, sel, zero, v.g, nullptr, nullptr, nullptr, nullptr, nullptr)
   if (narrow) {
     if (ns == TMAX) FG_MGJ(true, NWARP / 2); else FG_MGJ(false, NWARP / 2);
   } else {
@@ -2569,7 +2571,7 @@ struct MgRun {
       m.b0 = h->lv[l].b;
       m.bw0 = h->lv[l].bw;
       m.x0 = h->lv[l].x[0];
-      k_mg_bottom<<<1, kMgFuseThreads, bo, f->stream>>>(m, om1);
+      launch_pdl(k_mg_bottom, dim3(1), dim3(kMgFuseThreads), bo, f->stream, m, om1);
       cur[l] = 0;
       ++launches;
       return;
@@ -2581,12 +2583,12 @@ struct MgRun {
     MgLevelDev& v = h->lv[l];
     MgLevelDev& c = h->lv[l + 1];
     smooth(l, kMgPre, zero, false);
-    k_mg_restrict<<<level_grid(c.g), dim3(BX, BY), 0, f->stream>>>(v.x[cur[l]], v.b, v.flags, v.g,
-                                                                   c.flags, c.w, c.b, c.bw, c.g);
+    launch_pdl(k_mg_restrict, level_grid(c.g), dim3(BX, BY), 0, f->stream, v.x[cur[l]], v.b,
+               v.flags, v.g, c.flags, c.w, c.b, c.bw, c.g);
     ++launches;
     cycle(l + 1, true, false);
-    k_mg_prolong<<<level_grid(v.g), dim3(BX, BY), 0, f->stream>>>(c.x[cur[l + 1]], c.flags, c.g,
-                                                                  v.x[cur[l]], v.flags, v.g);
+    launch_pdl(k_mg_prolong, level_grid(v.g), dim3(BX, BY), 0, f->stream, c.x[cur[l + 1]], c.flags,
+               c.g, v.x[cur[l]], v.flags, v.g);
     ++launches;
     smooth(l, kMgPost, false, last && l == 0);
   }
