@@ -107,6 +107,8 @@ __device__ __forceinline__ void setup_cell(int i, int j, const float* __restrict
                                            int zero_phi, const Grid& g) {
   setup_cell_p(i, j, U, V, phi, rhs, W, BW, flags, om, zero_phi, g, g.P);
 }
+// The flags of an interior fluid cell with four fluid neighbours.
+constexpr uint8_t kPlain = F_W | F_E | F_S | F_N | F_FLUID | F_INTERIOR;
 __global__ void k_setup_system(const float* __restrict__ U, const float* __restrict__ V,
                                float* __restrict__ phi, float* __restrict__ rhs,
                                float* __restrict__ W, float* __restrict__ BW,
@@ -117,6 +119,73 @@ __global__ void k_setup_system(const float* __restrict__ U, const float* __restr
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
   setup_cell_p(i, j, U, V, phi, rhs, W, BW, flags, om, zero_phi, g, Ps, Fu, Fv);
+}
+
+// The same for a handle's own fields (g.P the pitch of all of them), 4 columns
+// a thread in 16-byte pieces; a piece of plain cells has one weight.  Bound by
+// memory traffic from 1500 x 1100 on; one cell a thread, with a division each,
+// was bound by its instructions (2048 x 2048: 20.1 us, 14.1 this way; the
+// traffic takes 12).
+__global__ void __launch_bounds__(256)
+    k_setup_pieces(const float* __restrict__ U, const float* __restrict__ V,
+                   float* __restrict__ phi, float* __restrict__ rhs, float* __restrict__ W,
+                   float* __restrict__ BW, const uint8_t* __restrict__ flags, float om,
+                   int zero_phi, Grid g, const float* __restrict__ Fu,
+                   const float* __restrict__ Fv) {
+  pdl_enter();
+  const int nq = (g.NY + 3) / 4, idx = blockIdx.x * 256 + threadIdx.x;
+  const int i = idx / nq, j = 4 * (idx - i * nq);
+  if (i >= g.NX) return;
+  const int c = i * g.P + j, cn = i <= g.NX - 2 ? c + g.P : c;
+  auto sum4 = [](const float* x, const float* y, int k, float (&o)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(x + k);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    if (y) {
+      const float4 b = *reinterpret_cast<const float4*>(y + k);
+      o[0] = o[0] + b.x; o[1] = o[1] + b.y; o[2] = o[2] + b.z; o[3] = o[3] + b.w;
+    }
+  };
+  const bool more = j + 4 < g.NY;  // the column right of the piece is a cell
+  const uint32_t f = *reinterpret_cast<const uint32_t*>(flags + c);
+  float u[4], un[4], v[4];
+  sum4(U, Fu, c, u);
+  sum4(U, Fu, cn, un);
+  sum4(V, Fv, c, v);
+  const float vr = more ? with_force(V, Fv, c + 4) : 0.0f;
+  const bool plain = more && f == kPlain * 0x01010101u;
+  float b[4], w[4], bw[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    b[k] = w[k] = bw[k] = 0.0f;
+    const uint8_t fl = (uint8_t)(f >> 8 * k);
+    if (plain) {
+      b[k] = -(un[k] - u[k] + (k < 3 ? v[k + 1] : vr) - v[k]);
+      w[k] = om * 0.25f;
+      bw[k] = w[k] * b[k];
+    } else if (i <= g.NX - 2 && j + k <= g.NY - 2) {
+      const bool act = flag_active(fl);
+      const float div = un[k] - u[k] + (k < 3 ? v[k + 1] : vr) - v[k];
+      b[k] = act ? -div : 0.0f;
+      w[k] = act ? om / (float)flag_count(fl) : 0.0f;
+      bw[k] = w[k] * b[k];
+    }
+  }
+  auto put = [&](float* d, const float (&x)[4]) {
+    if (j + 4 <= g.NY) {
+      *reinterpret_cast<float4*>(d + c) = make_float4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (j + k < g.NY) d[c + k] = x[k];
+    }
+  };
+  put(rhs, b);
+  put(W, w);
+  put(BW, bw);
+  if (zero_phi) {
+    const float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    put(phi, z);
+  }
 }
 
 // Register-blocked, temporally blocked Jacobi.  A CTA of 8 warps holds a
@@ -1440,7 +1509,6 @@ __device__ __forceinline__ GradOut grad_apply(bool hasL, bool hasR, bool hasB, b
 // grad_apply of a plain cell: an interior fluid cell with four fluid
 // neighbours (flags kPlain), whose bits are all 1 and whose neighbours' flags
 // say nothing more.  The same operations without the factors of 1.
-constexpr uint8_t kPlain = F_W | F_E | F_S | F_N | F_FLUID | F_INTERIOR;
 __device__ __forceinline__ GradOut grad_plain(const GradIn& in, float cp, float turbStrength,
                                               int do_turb, GradAcc& acc) {
   GradOut out;
@@ -2688,9 +2756,19 @@ cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb
   // sel = 0 (phi) until a launch runs.
   if ((e = cudaMemsetAsync(ctl, 0, sizeof(PCtl), f->stream)) != cudaSuccess) return e;
   count(f);
-  launch_pdl(k_setup_system, gr, bl, 0, f->stream, f->d[FG_U], f->d[FG_V], f->phi, f->rhs,
-             f->wgt, f->bw, f->flags, om, num_iters == 0 ? 1 : 0, f->g, f->P, f->step_fu,
-             f->step_fv);
+  // Pieces of four cells leave too few threads to hide the loads on small
+  // grids (us, cells against pieces: 128 x 128 2.3, 3.5; 512 x 256 2.6, 3.5;
+  // 1500 x 1100 9.1, 7.2; 2048 x 2048 20.1, 14.1).
+  if ((long long)f->NX * f->NY < (1 << 20)) {
+    launch_pdl(k_setup_system, gr, bl, 0, f->stream, f->d[FG_U], f->d[FG_V], f->phi, f->rhs,
+               f->wgt, f->bw, f->flags, om, num_iters == 0 ? 1 : 0, f->g, f->P, f->step_fu,
+               f->step_fv);
+  } else {
+    const long long pieces = (long long)((f->NY + 3) / 4) * f->NX;
+    launch_pdl(k_setup_pieces, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, f->stream,
+               f->d[FG_U], f->d[FG_V], f->phi, f->rhs, f->wgt, f->bw, f->flags, om,
+               num_iters == 0 ? 1 : 0, f->g, f->step_fu, f->step_fv);
+  }
   mark(f, "pressure setup");
   if (num_iters > 0) {
     e = mgs ? mg_solve(f, num_iters, om)
