@@ -2388,22 +2388,24 @@ __device__ __forceinline__ void mg_restrict_cell(int I, int J, const float* __re
                                                  const float* __restrict__ wc,
                                                  float* __restrict__ bc, float* __restrict__ bwc,
                                                  const Grid& gc) {
+  // (Interior cells: the children are rows 2I-1, 2I and columns 2J-1, 2J, the
+  // last without its pair on odd sides.  Every load is issued before the flags
+  // select.)
   const int cc = I * gc.P + J;
   float rs = 0.0f;
-  if (flag_active(flc[cc])) {
-    int a0, a1, b0, b1;
-    mg_children(I, gc.NX, gf.NX, a0, a1);
-    mg_children(J, gc.NY, gf.NY, b0, b1);
-    for (int a = a0; a <= a1; ++a)
-      for (int b = b0; b <= b1; ++b) {
-        const int cf = a * gf.P + b;
-        const uint8_t fl = flf[cf];
-        if (!flag_active(fl)) continue;
-        float nb = xf[cf - gf.P] + xf[cf + gf.P] + xf[cf - 1] + xf[cf + 1];
-        float ax = (float)flag_count(fl) * xf[cf] - nb;
-        rs = rs + (bf[cf] - ax);
-      }
-  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int i = 2 * I - 1 + a, j = 2 * J - 1 + b;
+      const int cf = min(i, gf.NX - 2) * gf.P + min(j, gf.NY - 2);
+      const uint8_t fl = flf[cf];
+      float nb = xf[cf - gf.P] + xf[cf + gf.P] + xf[cf - 1] + xf[cf + 1];
+      float ax = (float)flag_count(fl) * xf[cf] - nb;
+      const float sum = rs + (bf[cf] - ax);
+      rs = flag_active(fl) && i <= gf.NX - 2 && j <= gf.NY - 2 ? sum : rs;
+    }
+  rs = flag_active(flc[cc]) ? rs : 0.0f;
   bc[cc] = rs;
   bwc[cc] = wc[cc] * rs;
 }
@@ -2425,21 +2427,25 @@ __device__ __forceinline__ void mg_prolong_cell(int i, int j, const float* __res
                                                 float* __restrict__ xf,
                                                 const uint8_t* __restrict__ flf, const Grid& gf) {
   const int cf = i * gf.P + j;
-  if (!flag_active(flf[cf])) return;
   const int I = (i - 1) / 2 + 1, J = (j - 1) / 2 + 1;
   const int di = ((i - 1) & 1) ? 1 : -1, dj = ((j - 1) & 1) ? 1 : -1;
   const int ci[4] = {I, I + di, I, I + di}, cj[4] = {J, J, J + dj, J + dj};
   const float wt[4] = {9.0f, 3.0f, 3.0f, 1.0f};
+  const float x = xf[cf];
+  const bool act = flag_active(flf[cf]);
   float num = 0.0f, den = 0.0f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int cc = ci[k] * gc.P + cj[k];
-    if (!flag_active(flc[cc])) continue;
-    num = num + wt[k] * xc[cc];
-    den = den + wt[k];
+    const bool on = flag_active(flc[cc]);
+    const float sum = num + wt[k] * xc[cc];
+    num = on ? sum : num;
+    den = on ? den + wt[k] : den;
   }
-  const float e = den > 0.0f ? num / den : 0.0f;
-  xf[cf] = xf[cf] + e;
+  // (All four: den = 16, whose quotient the product with 1/16 is.)
+  float e = num * 0.0625f;
+  if (den != 16.0f) e = den > 0.0f ? num / den : 0.0f;
+  if (act) xf[cf] = x + e;
 }
 __global__ void k_mg_prolong(const float* __restrict__ xc, const uint8_t* __restrict__ flc, Grid gc,
                              float* __restrict__ xf, const uint8_t* __restrict__ flf, Grid gf) {
@@ -2453,19 +2459,22 @@ __global__ void k_mg_prolong(const float* __restrict__ xc, const uint8_t* __rest
 // The bottom of the V-cycle in one block, in shared memory: levels l0 ..
 // n-1 (a launch per operation would cost more than their work, and their
 // arrays fit on one SM).  The block copies the levels' weights and flags
-// and level l0's right-hand side into shared memory (rows of NY, no pitch
-// padding), zeroes the iterates, runs the same per-cell operations as the
+// and level l0's right-hand side into shared memory (rows of mg_pitch
+// cells), zeroes the iterates, runs the same per-cell operations as the
 // launches above and the Jacobi sweep kernel -- zero-started pre-smoothing
 // and restriction down to the coarsest level, its sweeps, then
 // prolongation and post-smoothing back up -- and writes level l0's iterate
 // back to its buffer 0.  Every level starts in buffer 0 and makes an even
 // number of sweeps, so its iterate ends in buffer 0; only interior cells
 // are written and the ghost rings stay 0 as the sweep kernel leaves them.
+// Latency bound (one block): 33 us for levels of 94 x 69 down to 6 x 5 cells
+// against 41 with synchronous loads (7.6 us of it), rows of warps at every
+// level and a block barrier in each of the 32 coarsest sweeps (7.5 us).
 constexpr int kMgFuseLevels = 12, kMgFuseThreads = 1024;
 constexpr int kMgSmemBytes = 200 * 1024;  // dynamic shared memory of k_mg_bottom
 struct MgFused {
   Grid gg[kMgFuseLevels];               // the levels in global memory (pitched)
-  Grid gs[kMgFuseLevels];               // the same in shared memory (pitch NY)
+  Grid gs[kMgFuseLevels];               // the same in shared memory (pitch mg_pitch)
   const uint8_t* flags[kMgFuseLevels];  // global
   const float* w[kMgFuseLevels];        // global
   const float* b0;                      // level l0's right-hand side and w * b (global)
@@ -2475,73 +2484,101 @@ struct MgFused {
   int boff[kMgFuseLevels];              // first byte of each level's flags in shared memory
   int n;                                // levels held (the first is l0)
 };
-// A level's arrays in shared memory: five float arrays of NX * NY, then flags.
+// A level's arrays in shared memory: five float arrays of NX * pitch, then flags.
 struct MgSm {
   float *x0, *x1, *b, *bw, *w;
   uint8_t* fl;
 };
 __device__ __forceinline__ MgSm mg_sm(const MgFused& m, int l, float* fs, uint8_t* bs) {
-  const int n = m.gs[l].NX * m.gs[l].NY;
+  const int n = m.gs[l].NX * m.gs[l].P;
   float* p = fs + m.foff[l];
   return MgSm{p, p + n, p + 2 * n, p + 3 * n, p + 4 * n, bs + m.boff[l]};
 }
 
 __device__ __forceinline__ void mg_fused_sweeps(const MgSm& a, const Grid& g, int ns, bool zero,
                                                 float om1) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kMgFuseThreads / 32;
+  const int tid = threadIdx.x, cols = g.NY - 2, n = (g.NX - 2) * cols;
+  auto cell = [&](const float* xs, int c, float w, float bw, float xc, bool z) {
+    float nb = z ? 0.0f : xs[c - g.P] + xs[c + g.P] + xs[c - 1] + xs[c + 1];
+    float y = __fmaf_rn(w, nb, bw);
+    return __fmaf_rn(om1, xc, y);
+  };
+  if (n <= kMgFuseThreads) {
+    // One cell a thread, its weights and value in registers; a level of one
+    // warp's cells needs no barrier between its sweeps.
+    const int i = tid / cols, c = (1 + i) * g.P + 1 + tid - i * cols;
+    const bool mine = tid < n, one = n <= 32;
+    const float w = mine ? a.w[c] : 0.0f, bw = mine ? a.bw[c] : 0.0f;
+    float xc = mine && !zero ? a.x0[c] : 0.0f;
+    if (!one || tid < 32)
+      for (int s = 0; s < ns; ++s) {
+        if (mine) {
+          xc = cell((s & 1) ? a.x1 : a.x0, c, w, bw, xc, zero && s == 0);
+          ((s & 1) ? a.x0 : a.x1)[c] = xc;
+        }
+        if (one) __syncwarp();
+        else __syncthreads();
+      }
+    if (one) __syncthreads();
+    return;
+  }
+  const int lane = tid & 31, warp = tid >> 5, nw = kMgFuseThreads / 32;
   for (int s = 0; s < ns; ++s) {
-    const float* xs = (s & 1) ? a.x1 : a.x0;
-    float* xd = (s & 1) ? a.x0 : a.x1;
+    const float* __restrict__ xs = (s & 1) ? a.x1 : a.x0;
+    float* __restrict__ xd = (s & 1) ? a.x0 : a.x1;
     const bool z = zero && s == 0;
     for (int i = 1 + warp; i < g.NX - 1; i += nw)
+#pragma unroll 3
       for (int j = 1 + lane; j < g.NY - 1; j += 32) {
         const int c = i * g.P + j;
-        float xc = 0.0f, nb;
-        if (!z) {
-          xc = xs[c];
-          nb = xs[c - g.P] + xs[c + g.P] + xs[c - 1] + xs[c + 1];
-        } else {
-          nb = 0.0f + 0.0f + 0.0f + 0.0f;
-        }
-        float y = __fmaf_rn(a.w[c], nb, a.bw[c]);
-        y = __fmaf_rn(om1, xc, y);
-        xd[c] = y;
+        xd[c] = cell(xs, c, a.w[c], a.bw[c], z ? 0.0f : xs[c], z);
       }
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(kMgFuseThreads)
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kMgFuseThreads, 1)
     k_mg_bottom(const __grid_constant__ MgFused m, float om1) {
   extern __shared__ __align__(16) float mg_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kMgFuseThreads / 32;
   uint8_t* bsm = reinterpret_cast<uint8_t*>(mg_smem);
   const int last = m.n - 1;
   pdl_enter();
+  // Every level's arrays in pieces of four cells, all copies in flight
+  // together (pitches are multiples of 4; the pieces' last cells may be pitch
+  // padding, which nothing reads).
   for (int l = 0; l <= last; ++l) {
     const MgSm a = mg_sm(m, l, mg_smem, bsm);
-    const Grid& gg = m.gg[l];
-    const Grid& gs = m.gs[l];
-    for (int i = warp; i < gs.NX; i += nw)
-      for (int j = lane; j < gs.NY; j += 32) {
-        const int cs = i * gs.P + j, cg = i * gg.P + j;
-        a.w[cs] = m.w[l][cg];
-        a.fl[cs] = m.flags[l][cg];
-        a.b[cs] = l == 0 ? m.b0[cg] : 0.0f;
-        a.bw[cs] = l == 0 ? m.bw0[cg] : 0.0f;
-        a.x0[cs] = 0.0f;
-        a.x1[cs] = 0.0f;
+    const int q4 = m.gs[l].P / 4;
+    for (int k = threadIdx.x; k < m.gs[l].NX * q4; k += kMgFuseThreads) {
+      const int i = k / q4, cs = 4 * k, cg = i * m.gg[l].P + 4 * (k - i * q4);
+      cp_async16(a.w + cs, m.w[l] + cg, 16);
+      cp_async4(a.fl + cs, m.flags[l] + cg);
+      if (l == 0) {
+        cp_async16(a.b + cs, m.b0 + cg, 16);
+        cp_async16(a.bw + cs, m.bw0 + cg, 16);
       }
+      *reinterpret_cast<float4*>(a.x0 + cs) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(a.x1 + cs) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   for (int l = 0; l < last; ++l) {
     const MgSm f = mg_sm(m, l, mg_smem, bsm), c = mg_sm(m, l + 1, mg_smem, bsm);
     mg_fused_sweeps(f, m.gs[l], kMgPre, true, om1);
     const Grid& gf = m.gs[l];
     const Grid& gc = m.gs[l + 1];
-    for (int I = 1 + warp; I < gc.NX - 1; I += nw)
-      for (int J = 1 + lane; J < gc.NY - 1; J += 32)
-        mg_restrict_cell(I, J, f.x0, f.b, f.fl, gf, c.fl, c.w, c.b, c.bw, gc);
+    for (int k = threadIdx.x; k < (gc.NX - 2) * (gc.NY - 2); k += kMgFuseThreads) {
+      const int I = k / (gc.NY - 2);
+      mg_restrict_cell(1 + I, 1 + k - I * (gc.NY - 2), f.x0, f.b, f.fl, gf, c.fl, c.w, c.b, c.bw,
+                       gc);
+    }
     __syncthreads();
   }
   mg_fused_sweeps(mg_sm(m, last, mg_smem, bsm), m.gs[last], kMgCoarse, true, om1);
@@ -2584,6 +2621,9 @@ void mg_sweeps(cudaStream_t st, const MgLevelDev& v, const float* src, float* ds
 // The V-cycles of one solve.  cur[l] names the buffer of level l holding
 // its iterate; the last smoothing of level 0 reports to the main control
 // block (sweeps = cycles, sel = the buffer of the result).
+// A level's pitch in shared memory: whole pieces of four cells.
+inline int mg_pitch(int NY) { return (NY + 3) / 4 * 4; }
+
 // The first coarse level from which all levels down fit k_mg_bottom's
 // shared memory (at most kMgFuseLevels of them); the level count when none
 // does.
@@ -2592,7 +2632,7 @@ int mg_bottom_level(const MgHier* h) {
   long long bytes = 0;
   int bottom = L;
   for (int l = L - 1; l >= 1 && L - l <= kMgFuseLevels; --l) {
-    bytes += (5 * (long long)sizeof(float) + 1) * h->lv[l].g.NX * h->lv[l].g.NY;
+    bytes += (5 * (long long)sizeof(float) + 1) * h->lv[l].g.NX * mg_pitch(h->lv[l].g.NY);
     if (bytes > kMgSmemBytes - 64) break;
     bottom = l;
   }
@@ -2625,16 +2665,16 @@ struct MgRun {
       for (int k = 0; k < m.n; ++k) {
         const MgLevelDev& v = h->lv[l + k];
         m.gg[k] = v.g;
-        m.gs[k] = make_grid(v.g.NX, v.g.NY, v.g.NY, v.g.h);
+        m.gs[k] = make_grid(v.g.NX, v.g.NY, mg_pitch(v.g.NY), v.g.h);
         m.flags[k] = v.flags;
         m.w[k] = v.w;
         m.foff[k] = fo;
-        fo += 5 * v.g.NX * v.g.NY;
+        fo += 5 * v.g.NX * mg_pitch(v.g.NY);
       }
       int bo = fo * (int)sizeof(float);
       for (int k = 0; k < m.n; ++k) {
         m.boff[k] = bo;
-        bo += h->lv[l + k].g.NX * h->lv[l + k].g.NY;
+        bo += h->lv[l + k].g.NX * mg_pitch(h->lv[l + k].g.NY);
       }
       m.b0 = h->lv[l].b;
       m.bw0 = h->lv[l].bw;
