@@ -54,7 +54,14 @@ template <auto Body, class... A>
 __global__ void kb_border(const BTile* __restrict__ tiles, const BScene* __restrict__ sc, A... a) {
   const BTile t = tiles[blockIdx.x];
   const Grid g = sc[t.s].g;
+  pdl_enter();
   Body(t.x * blockDim.x + threadIdx.x, bshift(a, sc[t.s].off)..., g);
+}
+template <auto Body, class... A>
+inline cudaError_t launch_border(const fg_fluid* f, A... a) {
+  const BatchGeom* b = f->batch;
+  return launch_pdl(kb_border<Body, A...>, dim3(b->n_border_tiles), dim3(128), 0, f->stream,
+                    b->border_tiles, b->scenes_dev, a...);
 }
 
 // Launches a per-cell stage: the single-scene kernel K over the handle's
@@ -64,8 +71,8 @@ __global__ void kb_border(const BTile* __restrict__ tiles, const BScene* __restr
     if ((f)->batch) {                                                                        \
       launch_cells<BODY>((f), __VA_ARGS__);                                                  \
     } else {                                                                                 \
-      K<<<dim3(((f)->NY + 31) / 32, ((f)->NX + 7) / 8), dim3(32, 8), 0, (f)->stream>>>(      \
-          __VA_ARGS__, (f)->g);                                                              \
+      launch_pdl(K, dim3(((f)->NY + 31) / 32, ((f)->NX + 7) / 8), dim3(32, 8), 0,            \
+                 (f)->stream, __VA_ARGS__, (f)->g);                                          \
     }                                                                                        \
   } while (0)
 
@@ -76,13 +83,10 @@ __global__ void kb_border(const BTile* __restrict__ tiles, const BScene* __restr
 #define FG_BORDER(f, K, BODY, ...)                                                           \
   do {                                                                                       \
     if ((f)->batch) {                                                                        \
-      const BatchGeom* b_ = (f)->batch;                                                      \
-      kb_border<BODY><<<b_->n_border_tiles, 128, 0, (f)->stream>>>(b_->border_tiles,         \
-                                                                   b_->scenes_dev,           \
-                                                                   __VA_ARGS__);             \
+      launch_border<BODY>((f), __VA_ARGS__);                                                 \
     } else {                                                                                 \
       int n_ = (f)->NX > (f)->NY ? (f)->NX : (f)->NY;                                        \
-      K<<<(n_ + 127) / 128, 128, 0, (f)->stream>>>(__VA_ARGS__, (f)->g);                     \
+      launch_pdl(K, dim3((n_ + 127) / 128), dim3(128), 0, (f)->stream, __VA_ARGS__, (f)->g); \
     }                                                                                        \
   } while (0)
 

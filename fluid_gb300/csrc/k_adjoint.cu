@@ -62,6 +62,7 @@ __device__ __forceinline__ void add_forces_cell(int i, int j, float* __restrict_
 }
 __global__ void k_add_forces(float* __restrict__ U, float* __restrict__ V,
                              const float* __restrict__ Fu, const float* __restrict__ Fv, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -154,6 +155,7 @@ __global__ void k_adj_sl_velocity(const float* __restrict__ lamU, const float* _
                                   float* dUt, float* dVt, float* dFu, float* dFv, float* dRu,
                                   float* dRv, float* dNu, float* dNv,
                                   const uint8_t* __restrict__ flags, float sdt, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -272,6 +274,7 @@ __global__ void k_adj_bfecc_vel(const float* __restrict__ lamCu, const float* __
                                 const float* __restrict__ Fu, const float* __restrict__ Fv,
                                 float* dOu, float* dOv, float* dFu, float* dFv,
                                 const uint8_t* __restrict__ flags, float dt, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -328,6 +331,7 @@ __global__ void k_adj_sl_smoke(const float* __restrict__ lamM, const float* __re
                                float* dU, float* dV, float* dMs, float* dN,
                                const uint8_t* __restrict__ flags, float sdt, float smokeAdv,
                                int bwd, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -393,6 +397,7 @@ __global__ void k_adj_bfecc_smoke(const float* __restrict__ lamC, const float* _
                                   const float* __restrict__ Fm, float* dO, float* dF, float* dU,
                                   float* dV, const uint8_t* __restrict__ flags, float dt,
                                   float smokeAdv, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -460,6 +465,7 @@ __device__ __forceinline__ void adj_borders_border(int t, float* __restrict__ dU
 }
 __global__ void k_adj_borders(float* __restrict__ dU, float* __restrict__ dV,
                               const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   adj_borders_border(t, dU, dV, flags, g);
 }
@@ -492,6 +498,7 @@ __global__ void k_adj_turbulence(float* __restrict__ dU, float* __restrict__ dV,
                                  const float* __restrict__ U2, const float* __restrict__ V2,
                                  const float2* __restrict__ noise,
                                  const uint8_t* __restrict__ flags, float turbStrength, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -587,6 +594,7 @@ __global__ void k_adj_conf_local(float* __restrict__ dU, float* __restrict__ dV,
                                  const uint8_t* __restrict__ flags, float conf, float dt,
                                  float turbStrength, int do_turb, float* __restrict__ lw,
                                  float* __restrict__ lgx, float* __restrict__ lgy, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -618,6 +626,7 @@ __global__ void k_adj_conf_curl(const float* __restrict__ U2, const float* __res
                                 const float* __restrict__ lwd, const float* __restrict__ lgx,
                                 const float* __restrict__ lgy, float* __restrict__ lw,
                                 const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -639,6 +648,7 @@ __device__ __forceinline__ void adj_conf_apply_cell(int i, int j, float* __restr
 }
 __global__ void k_adj_conf_apply(float* __restrict__ dU, float* __restrict__ dV,
                                  const float* __restrict__ lw, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -667,6 +677,7 @@ __device__ __forceinline__ void adj_grad_t_cell(int i, int j, const float* __res
 __global__ void k_adj_grad_t(const float* __restrict__ dU, const float* __restrict__ dV,
                              const float* __restrict__ W, float* __restrict__ rhs,
                              float* __restrict__ BW, const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -699,6 +710,7 @@ __global__ void k_adj_resid(const float* __restrict__ lam, const float* __restri
                             const float* __restrict__ e1, const void* __restrict__ esel,
                             const float* __restrict__ W, float* __restrict__ rhs,
                             float* __restrict__ BW, const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -737,6 +749,7 @@ __global__ void k_adj_div_t(float* __restrict__ dU, float* __restrict__ dV,
                             const void* __restrict__ ctl_sel, const float* __restrict__ e0,
                             const float* __restrict__ e1, const void* __restrict__ esel,
                             const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -770,6 +783,7 @@ __global__ void k_adj_sources(float* __restrict__ dU, float* __restrict__ dV,
                               float* __restrict__ dM, const SourceRec* __restrict__ recs,
                               const uint32_t* __restrict__ off, int n_groups,
                               const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_groups) return;
   adj_sources_group(dU, dV, dM, recs, off[k], off[k + 1], flags, g);
@@ -779,6 +793,7 @@ __global__ void kb_adj_sources(float* __restrict__ dU, float* __restrict__ dV,
                                const uint32_t* __restrict__ off, const int* __restrict__ gs,
                                int n_groups, const uint8_t* __restrict__ flags,
                                const BScene* __restrict__ sc) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_groups) return;
   const BScene& s = sc[gs[k]];
@@ -792,6 +807,7 @@ __global__ void k_mask_forces(float* __restrict__ Fu, float* __restrict__ Fv,
                               const SourceRec* __restrict__ recs,
                               const uint32_t* __restrict__ off, int n_groups,
                               const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_groups) return;
   uint32_t cell = recs[off[k]].cell;
@@ -908,6 +924,7 @@ __global__ void k_adj_begin(float* __restrict__ aU, float* __restrict__ aV, floa
                             float* __restrict__ w1, float* __restrict__ w2,
                             float* __restrict__ w3, float* __restrict__ w4,
                             float* __restrict__ w5, int n) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   aU[k] = aU[k] + aNU[k];
@@ -982,7 +999,7 @@ cudaError_t launch_step_adjoint(fg_fluid* f, float dt, float* const* tape) {
   cudaError_t e;
   const int n = f->NX * f->P;
   count(f);
-  k_adj_begin<<<(n + 255) / 256, 256, 0, st>>>(A[F::A_U], A[F::A_V], A[F::A_M], A[F::A_NU],
+  launch_pdl(k_adj_begin, dim3((n + 255) / 256), dim3(256), 0, st, A[F::A_U], A[F::A_V], A[F::A_M], A[F::A_NU],
                                                A[F::A_NV], A[F::A_NM], A[F::A_CU], A[F::A_CV],
                                                A[F::A_FU], A[F::A_FV], A[F::A_CM], A[F::A_FM], n);
   float sa = p.smoke_advection;
@@ -1096,12 +1113,12 @@ cudaError_t launch_step_adjoint(fg_fluid* f, float dt, float* const* tape) {
   if (f->n_src_groups > 0) {
     count(f);
     if (f->batch)
-      kb_adj_sources<<<(f->n_src_groups + 255) / 256, 256, 0, st>>>(
-          A[F::A_U], A[F::A_V], A[F::A_M], f->src_dev, f->src_off_dev, f->batch->src_scene,
+      launch_pdl(
+          kb_adj_sources, dim3((f->n_src_groups + 255) / 256), dim3(256), 0, st, A[F::A_U], A[F::A_V], A[F::A_M], f->src_dev, f->src_off_dev, f->batch->src_scene,
           f->n_src_groups, f->flags, f->batch->scenes_dev);
     else
-      k_adj_sources<<<(f->n_src_groups + 255) / 256, 256, 0, st>>>(
-          A[F::A_U], A[F::A_V], A[F::A_M], f->src_dev, f->src_off_dev, f->n_src_groups, f->flags,
+      launch_pdl(
+          k_adj_sources, dim3((f->n_src_groups + 255) / 256), dim3(256), 0, st, A[F::A_U], A[F::A_V], A[F::A_M], f->src_dev, f->src_off_dev, f->n_src_groups, f->flags,
           g);
   }
   return cudaGetLastError();
@@ -1110,7 +1127,7 @@ cudaError_t launch_step_adjoint(fg_fluid* f, float dt, float* const* tape) {
 cudaError_t launch_mask_forces(fg_fluid* f, float* fu, float* fv) {
   if (f->n_src_groups <= 0 || f->batch) return cudaSuccess;
   count(f);
-  k_mask_forces<<<(f->n_src_groups + 255) / 256, 256, 0, f->stream>>>(
+  launch_pdl(k_mask_forces, dim3((f->n_src_groups + 255) / 256), dim3(256), 0, f->stream,
       fu, fv, f->src_dev, f->src_off_dev, f->n_src_groups, f->flags, f->g);
   return cudaGetLastError();
 }

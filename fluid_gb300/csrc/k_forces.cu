@@ -94,6 +94,7 @@ __device__ __forceinline__ void apply_sources_group(const SourceRec* __restrict_
 __global__ void k_apply_sources(const SourceRec* __restrict__ recs,
                                 const uint32_t* __restrict__ off, int n_groups, float* U,
                                 float* V, float* M, const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_groups) return;
   apply_sources_group(recs, off[k], off[k + 1], U, V, M, flags, g);
@@ -105,6 +106,7 @@ __global__ void kb_apply_sources(const SourceRec* __restrict__ recs,
                                  int n_groups, float* U, float* V, float* M,
                                  const uint8_t* __restrict__ flags,
                                  const BScene* __restrict__ sc) {
+  pdl_enter();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_groups) return;
   const BScene& s = sc[gs[k]];
@@ -154,6 +156,7 @@ __device__ __forceinline__ void curl_cell(int i, int j, const float* __restrict_
 }
 __global__ void k_curl(const float* __restrict__ U, const float* __restrict__ V,
                        float* __restrict__ curl, const uint8_t* __restrict__ flags, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -205,6 +208,7 @@ __global__ void k_conf_turb(float* __restrict__ U, float* __restrict__ V,
                             const float* __restrict__ curl, const float2* __restrict__ noise,
                             const uint8_t* __restrict__ flags, float conf, float dt,
                             float turbStrength, int do_conf, int do_turb, Grid g) {
+  pdl_enter();
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int i = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.NX || j >= g.NY) return;
@@ -303,11 +307,11 @@ cudaError_t launch_apply_sources(fg_fluid* f) {
   if (f->n_src_groups <= 0) return cudaSuccess;
   count(f);
   if (f->batch)
-    kb_apply_sources<<<(f->n_src_groups + 255) / 256, 256, 0, f->stream>>>(
+    launch_pdl(kb_apply_sources, dim3((f->n_src_groups + 255) / 256), dim3(256), 0, f->stream,
         f->src_dev, f->src_off_dev, f->batch->src_scene, f->n_src_groups, f->d[FG_U],
         f->d[FG_V], f->d[FG_M], f->flags, f->batch->scenes_dev);
   else
-    k_apply_sources<<<(f->n_src_groups + 255) / 256, 256, 0, f->stream>>>(
+    launch_pdl(k_apply_sources, dim3((f->n_src_groups + 255) / 256), dim3(256), 0, f->stream,
         f->src_dev, f->src_off_dev, f->n_src_groups, f->d[FG_U], f->d[FG_V], f->d[FG_M],
         f->flags, f->g);
   return cudaGetLastError();
