@@ -824,7 +824,7 @@ def app_rows(fluid_gb300):
     rows = {}
     # The CPU baseline's own workload on the GPU: the 2048^2 cavity with the
     # reference's serial SOR (200 sweeps, no early exit), bit for bit, as the
-    # cluster wavefront -- the drop-in path for a caller who keeps the
+    # pipeline of warps -- the drop-in path for a caller who keeps the
     # reference's scheme.
     f = fluid_gb300.Fluid(1.0, W, H, 1.0, auto_sync=False, UseBFECC=True, num_iters=ITERS,
                           early_exit=False)
@@ -841,10 +841,10 @@ def app_rows(fluid_gb300):
     rows["reference_sor_2048"] = {
         "value": W * H / ms / 1e3, "unit": "Mcell-steps/s", "ms_per_step": ms,
         "config": "the CPU baseline's workload (2048^2 cavity, BFECC, the reference's serial SOR "
-                  "with 200 sweeps) bit for bit on the GPU (cluster wavefront on diagonal-major "
-                  "copies); device-timed steps; its CPU baseline is the line's cpu_baseline"}
+                  "with 200 sweeps) bit for bit on the GPU (sweeps pipelined over warps and "
+                  "strips); device-timed steps; its CPU baseline is the line's cpu_baseline"}
     del f
-    # The reference scheme (serial SOR, bit for bit) as the wavefront kernel:
+    # The reference scheme (serial SOR, bit for bit) as the pipeline of warps:
     # the 512^2 cavity, the reference's 8 iterations per step.
     f = fluid_gb300.Fluid(1.0, MG_SIDE, MG_SIDE, 1.0, auto_sync=False, UseBFECC=True, num_iters=8)
     S = f.S.reshape(f.NumX, f.NumY)
@@ -860,8 +860,8 @@ def app_rows(fluid_gb300):
     rows["reference_sor"] = {"value": MG_SIDE * MG_SIDE / ms / 1e3, "unit": "Mcell-steps/s",
                              "ms_per_step": ms,
                              "config": "%dx%d cavity, the reference's lexicographic SOR bit for bit "
-                                       "(8 sweeps with the reference's early exit, wavefront on an "
-                                       "8-block cluster), BFECC; device-timed steps"
+                                       "(8 sweeps with the reference's early exit, pipelined over "
+                                       "warps and strips), BFECC; device-timed steps"
                                        % (MG_SIDE, MG_SIDE)}
     del f
     # Multigrid: a lid-driven cavity stepped with UseMultigrid (8 V-cycles).

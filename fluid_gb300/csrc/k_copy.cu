@@ -12,7 +12,10 @@ namespace {
 // rows at a pitch on the other (a batch's slices: width = pitch).  Linear
 // storage is walked in 16-byte pieces, so writes to a host mirror leave the
 // chip as whole lines whatever the width; the pitched side is addressed in
-// 16-byte pieces where the width allows it.
+// 16-byte pieces where the width allows it.  Bound by the host link for mirrors
+// (185 GB/s; small ones by the launch: 4 fields of 130 x 130 in 10 us with the
+// synchronisation, 17 by four copies) and by HBM for a batch's slices (147
+// slices of 21 scenes in 33 us with both synchronisations, 640 by copies).
 template <bool TO_LINEAR>
 __global__ void __launch_bounds__(256) k_copy_list(const __grid_constant__ CopyList l) {
   const CopyItem c = l.it[blockIdx.y];
