@@ -34,15 +34,6 @@ __host__ __device__ __forceinline__ void two_sum(float a, float b, float& s, flo
   e = (a - (s - bb)) + (b - bb);
 }
 
-__host__ __device__ __forceinline__ FF ff_add(FF a, FF b) {
-  float s, e;
-  two_sum(a.hi, b.hi, s, e);
-  e = e + (a.lo + b.lo);
-  float h, l;
-  two_sum(s, e, h, l);
-  return FF{h, l};
-}
-
 #ifdef __CUDACC__
 // Adds a float pair to a running pair; the errors gather in its low part.
 __device__ __forceinline__ void ff_acc(FF& a, FF q) {
