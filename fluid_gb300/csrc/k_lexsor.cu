@@ -431,7 +431,9 @@ __device__ __forceinline__ void wv_sweep(const WaveArgs& a, WaveShared* sh, cons
         add_if(pn, cp * pp, c2.y);
         max_if(mx, div, c2.y);
         F(at0) = un;
-        F(at0 + RB) = en;  // (the lane above stores its own value there one step later)
+        // (A lower lane's east face is the next lane's `un` one step later; no
+        // two lanes store the same word between two barriers of the warp.)
+        if (lane == 31) F(at0 + RB) = en;
         F(at0 + 4 * R::O1) = vn;
         F(at0 + 4 * R::O2) = pn;
         v0 = tn;
