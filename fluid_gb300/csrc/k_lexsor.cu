@@ -508,7 +508,10 @@ __device__ void wv_loader(const WaveArgs& a, WaveShared* sh, float* ring, int b,
       const unsigned long long v = ld_gpu(fin);
       r = (unsigned)(v >> 32) == tag - 1 && (int)(v & 0xffffffffu) >= min(c + 32, a.NY);
     }
-    return __all_sync(0xffffffffu, r) != 0;
+    const bool all = __all_sync(0xffffffffu, r) != 0;
+    // (A vote orders no memory: what the two lanes acquired, before every lane's copies.)
+    __syncwarp();
+    return all;
   };
   auto publish = [&](int cols) {
     __syncwarp();

@@ -903,6 +903,7 @@ __device__ __forceinline__ bool flow_ready_warp(const int* done, int ph, int t, 
   }
   if (!__all_sync(0xffffffffu, ok)) return false;
   asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  __syncwarp();  // (a vote orders no memory: the lanes' flags before lane 0's copy)
   return true;
 }
 
