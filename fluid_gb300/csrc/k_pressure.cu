@@ -954,7 +954,8 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
   // full: an item's boxes have landed (and s_item names it); empty: the
   // sweeping warps hold it in registers; stored: they have stored it.
   __shared__ __align__(8) uint64_t full, empty, stored;
-  __shared__ int s_item, s_lost;
+  __shared__ int s_item;
+  __shared__ unsigned s_lost;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntiles = ntx * nty, total = ntiles * nphase;
   int* counter = done + ntiles;
@@ -963,7 +964,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
     mbar_init(&empty, FW);
     mbar_init(&stored, FW);
     s_item = 0;
-    s_lost = 0;
+    s_lost = UINT_MAX;
   }
   __syncthreads();
   bool fail = false;
@@ -1052,11 +1053,20 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
     const bool own_col = lane * JT >= TMAX && lane * JT < RJ - TMAX;
     for (unsigned n = 0;; ++n) {
       const bool landed = mbar_wait_bounded(&full, n & 1);
-      const int item = s_item;
-      // (A wait that gave up: every warp leaves after this item's sweeps, whose
-      // barriers show it to all; the item named is then an earlier one.)
-      if (!landed) s_lost = 1;
-      if (item >= total) break;
+      // A warp whose wait gave up sweeps whatever the buffer holds, as item 0,
+      // and a warp that has seen the end meets the same barriers before it
+      // leaves: whatever each warp saw, all of them pass TMAX barriers here, so
+      // none is left waiting in one.  s_lost names the item given up: set
+      // before the first barrier, it is seen by all after the last, and a
+      // faster warp that gives up the next item does not make a slower one
+      // leave before that item's barriers.
+      const int item = landed ? s_item : 0;
+      if (!landed) s_lost = n;
+      if (item >= total) {
+#pragma unroll 1
+        for (int sw = 0; sw < TMAX; ++sw) tile_barrier<FW, true>();
+        break;
+      }
       const int ph = item / ntiles, t = item - ph * ntiles;
       const int ty = t / ntx, tx = t - ty * ntx;
       const int gi0 = ty * FO - TMAX + warp * RT;
@@ -1083,7 +1093,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty);
       tile_sweeps<OMEGA1, NoHook, FW, true>(x, w, bw, om1, xch, warp, lane);
-      if (*(volatile int*)&s_lost) {
+      if (*(volatile unsigned*)&s_lost <= n) {
         fail = true;
         break;
       }
