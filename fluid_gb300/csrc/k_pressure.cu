@@ -937,6 +937,11 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
+// The same for a whole warp: its lanes test one by one and may not see the same,
+// but what follows (a claim's shuffle, the next vote) needs all of them.
+__device__ __forceinline__ bool warp_test(uint64_t* bar, unsigned parity) {
+  return __all_sync(0xffffffffu, mbar_test(bar, parity)) != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -997,7 +1002,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
       bool taken = false;
       unsigned long long t0 = 0;
       for (int it = 0;; ++it) {
-        if (!taken && (unused || mbar_test(&empty, (n - 1) & 1))) {
+        if (!taken && (unused || warp_test(&empty, (n - 1) & 1))) {
           taken = true;
           flight = have;
           if (lane == 0) {
@@ -1022,7 +1027,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
           }
           copied = true;
         }
-        if (taken && !told && mbar_test(&stored, (n - 1) & 1)) {
+        if (taken && !told && warp_test(&stored, (n - 1) & 1)) {
           if (deep) after = claim();
           if (lane == 0 && cur_t != stall_tile) {  // (a stalled tile: fault injection)
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
@@ -1035,7 +1040,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
         if ((it & 63) == 63) {  // (the timer is slow to read)
           const unsigned long long now = global_ns();
           if (t0 == 0) t0 = now;
-          if (it >= MBAR_MAX_TRIES || now - t0 > MBAR_WAIT_NS) {
+          if (__any_sync(0xffffffffu, it >= MBAR_MAX_TRIES || now - t0 > MBAR_WAIT_NS)) {
             fail = true;
             break;
           }
@@ -1052,7 +1057,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
     const bool own_col = lane * JT >= TMAX && lane * JT < RJ - TMAX;
     for (unsigned n = 0;; ++n) {
-      const bool landed = mbar_wait_bounded(&full, n & 1);
+      const bool landed = __all_sync(0xffffffffu, mbar_wait_bounded(&full, n & 1));
       // A warp whose wait gave up sweeps whatever the buffer holds, as item 0,
       // and a warp that has seen the end meets the same barriers before it
       // leaves: whatever each warp saw, all of them pass TMAX barriers here, so

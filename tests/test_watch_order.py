@@ -30,6 +30,16 @@ def test_copies_follow_every_watched_publisher(watchers, copiers):
     assert not all(need <= seen[l] for l in copiers)
 
 
+def test_lanes_that_wait_agree_before_they_go_on():
+    """A lane's own test of a barrier, or its own reading of the timer, may
+    differ from the next lane's: every branch that leads to a shuffle, a vote
+    or a block barrier is taken by the whole warp or not at all."""
+    code = body("k_pressure.cu", "auto claim = [&]", "if (fail && lane == 0) {\n    atomicExch")
+    assert "mbar_test(" not in code.replace("warp_test(", "")
+    waits = [x for x in code.splitlines() if "mbar_wait_bounded(" in x or "MBAR_WAIT_NS" in x]
+    assert len(waits) == 2 and all("_sync(0xffffffffu" in x for x in waits)
+
+
 def body(path, start, end):
     import os
 
