@@ -510,6 +510,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
                "r"(bytes)
                : "memory");
 }
+// The same without the arrival: the phase stays open.
+__device__ __forceinline__ void mbar_expect_more(uint64_t* bar, unsigned bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
   uint32_t ok;
   asm volatile(
@@ -988,7 +994,10 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
     // and it goes first (1300 x 1300, 204 tiles: 8.5 us against 9.3).
     const bool deep = ntiles >= 2 * (int)gridDim.x;
     int cur_ph = 0, cur_t = -1, next = claim();
-    bool flight = false;
+    // The item whose boxes may be landing (its phase of `full`), and whether
+    // its last box has been sent for.
+    bool flight = false, whole = true;
+    unsigned flight_n = 0;
     for (unsigned n = 0;; ++n) {
       // Item `next` goes into the buffer when it is free; the item before it
       // is swept meanwhile.  Everything about it that needs no buffer (its
@@ -1005,12 +1014,14 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
         if (!taken && (unused || warp_test(&empty, (n - 1) & 1))) {
           taken = true;
           flight = have;
+          flight_n = n;
+          whole = !have;
           if (lane == 0) {
             s_item = next;
             if (have) {
               // The warps' earlier shared-memory reads before the copies' writes.
               asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-              mbar_expect_tx(&full, (zi ? 2u : 3u) * FLOW_FLOATS * 4u);
+              mbar_expect_more(&full, 2u * FLOW_FLOATS * 4u);
               tma_load_2d(tbuf + 2 * FLOW_FLOATS, &tmb, x, y, &full);
               tma_load_2d(tbuf + FLOW_FLOATS, &tmw, x, y, &full);
             } else {
@@ -1020,12 +1031,17 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
         }
         if (!ready) ready = flow_ready_warp(done, ph, t, ntx, nty, lane);
         if (!copied && ready && taken) {
-          if (lane == 0 && !zi) {
-            // The neighbours' (generic) stores, acquired above, before the copy's reads.
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            tma_load_2d(tbuf, (ph & 1) ? &tm1 : &tm0, x, y, &full);
+          if (lane == 0) {
+            if (zi) {
+              mbar_arrive(&full);
+            } else {
+              // The neighbours' (generic) stores, acquired above, before the copy's reads.
+              asm volatile("fence.proxy.async.global;" ::: "memory");
+              mbar_expect_tx(&full, FLOW_FLOATS * 4u);
+              tma_load_2d(tbuf, (ph & 1) ? &tm1 : &tm0, x, y, &full);
+            }
           }
-          copied = true;
+          copied = whole = true;
         }
         if (taken && !told && warp_test(&stored, (n - 1) & 1)) {
           if (deep) after = claim();
@@ -1051,8 +1067,16 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
       cur_ph = ph;
       cur_t = t;
     }
-    // A copy still landing when a wait gave up.
-    if (fail && flight && lane == 0) mbar_drain(&full, 0), mbar_drain(&full, 1);
+    if (fail && flight && lane == 0) {
+      // A wait gave up.  An item without its phi is ended here, marked lost, so
+      // that the warps that wait for it leave too; then the copies still
+      // landing.  (Left incomplete, the phase held the block for 9 s more.)
+      if (!whole) {
+        s_lost = flight_n;
+        mbar_arrive(&full);
+      }
+      mbar_drain(&full, flight_n & 1);
+    }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
     const bool own_col = lane * JT >= TMAX && lane * JT < RJ - TMAX;
