@@ -1229,7 +1229,8 @@ def run_ours(args):
             "stage_ms": stage_ms,
             "step_stats": {"div_l2_post": st["div_l2_post"], "resid_l2": st["resid_l2"],
                            "smoke_mass": st["smoke_mass"], "sweeps": st["sweeps"],
-                           "jacobi_kernel": {0: "none", 1: "sweep", 2: "tma",
+                           "jacobi_kernel": "resident" if st["jacobi_resident"] else
+                                            {0: "none", 1: "sweep", 2: "tma",
                                              3: "dataflow"}[st["jacobi_kernel"]]},
         }
         print(json.dumps(line), flush=True)

@@ -915,6 +915,7 @@ int fg_get_stats(fg_fluid* f, fg_stats* out) {
   out->last_maxdiv = s.last_maxdiv;
   out->sweeps = s.sweeps;
   out->jacobi_kernel = f->jacobi_kernel;
+  out->jacobi_resident = f->jacobi_resident;
   if (s.timeout) return fail(f, FG_ERR_TIMEOUT, "a device-side wait of the last step gave up");
   for (double v : {s.div_l2_sq, s.div_max, s.resid_l2_sq, s.resid_max, s.smoke_mass, s.last_maxdiv})
     if (!std::isfinite(v)) return fail(f, FG_ERR_NONFINITE, "the last step produced non-finite values");

@@ -365,6 +365,7 @@ struct fg_fluid {
   int* tile_done = nullptr;  // dataflow Jacobi kernel: per-tile phase flags + item counter
   int stall_tile = -1;       // fault injection: a tile the dataflow kernel never publishes
   int jacobi_kernel = 0;     // FG_JACOBI_KERNEL_* of the last main solve (fg_stats)
+  int jacobi_resident = 0;   // its resident form (warps a region, 16: two of 8 an SM) or 0
   // The serial schemes' pipeline (k_lexsor.cu): control words, packets and
   // the speculative pass's fields in one block (or none), and the blocks the
   // device holds at once.

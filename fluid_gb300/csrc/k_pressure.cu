@@ -2208,13 +2208,14 @@ static cudaError_t launch_res(cudaStream_t st, const JResArgs& a, bool o1, bool 
   return cudaLaunchKernelEx(&cfg, res_kernel(o1, batch, form), a);
 }
 
-// A fixed-count solve of one grid from x = 0 into x as one resident launch;
-// false (nothing launched) where its regions do not fit the GPU at once.
-static bool launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, const float* BW,
-                              float om1, int iters, int T, int stall) {
-  if (!f->jres) return false;
+// A fixed-count solve of one grid from x = 0 into x as one resident launch.
+// What fg_stats.jacobi_resident reports of it, or 0 (nothing launched) where
+// the grid's regions do not fit the GPU at once.
+static int launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, const float* BW,
+                             float om1, int iters, int T, int stall) {
+  if (!f->jres) return 0;
   const TmaDevice* dv = tma_ready(f->stream);
-  if (!dv) return false;
+  if (!dv) return 0;
   int n[4];
   for (int k = 0; k < 4; ++k) n[k] = res_regions(f->NX, f->NY, res_warps(k));
   // 4 warps a region while each gets an SM of its own, else 8, one or two to
@@ -2230,7 +2231,7 @@ static bool launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, 
          !(n[form] > 0 && n[form] <= (form == JRES_8X2 ? dv->res_blocks[form]
                                                        : std::min(dv->sms, dv->res_blocks[form]))))
     ++form;
-  if (form > JRES_8X2) return false;
+  if (form > JRES_8X2) return 0;
   const int nw = res_warps(form);
   JResArgs a = {};
   a.x = x;
@@ -2248,9 +2249,11 @@ static bool launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, 
   a.last_launch = (iters + T - 1) / T - 1;
   a.err = &f->dstats->timeout;
   a.stall = stall;
-  const bool ok = launch_res(f->stream, a, om1 == 0.0f, false, form, n[form]) == cudaSuccess;
-  if (!ok) cudaGetLastError();
-  return ok;
+  if (launch_res(f->stream, a, om1 == 0.0f, false, form, n[form]) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return form == JRES_8X2 ? 16 : nw;
 }
 
 // A batch's solves: every scene runs its own sweep count, no early exit.
@@ -2332,11 +2335,14 @@ static cudaError_t jacobi_solve(fg_fluid* f, PCtl* ctl, const float* b, const fl
   if (prof && (e = cudaEventRecord(f->prof_ev[0], f->stream)) != cudaSuccess) return e;
   int n = 0;
   const TmaDevice* dv = tma_ready(f->stream);
-  if (!rinit && !check && iters > 0 &&
-      launch_jacobi_res(f, ctl, x0, f->wgt, bw,
-                        1.0f - f->prm.jacobi_omega * f->prm.pressure_damping, iters, T,
-                        f->stall_tile)) {
-    // (Reported as the kernel that runs such a solve without the buffers.)
+  const int resident = rinit || check || iters <= 0
+                           ? 0
+                           : launch_jacobi_res(f, ctl, x0, f->wgt, bw,
+                                               1.0f - f->prm.jacobi_omega * f->prm.pressure_damping,
+                                               iters, T, f->stall_tile);
+  if (kind) f->jacobi_resident = resident;
+  if (resident) {
+    // (kind: the kernel that such a solve takes without the resident launch.)
     n = 1;
     if (kind)
       *kind = T < TMAX || iters < TMAX ? FG_JACOBI_KERNEL_SWEEP
@@ -2809,6 +2815,7 @@ cudaError_t launch_pressure(fg_fluid* f, int num_iters, float dt, bool fuse_turb
   float cp = f->density * f->h / dt;  // fluid.go:158
   cudaError_t e;
   f->jacobi_kernel = FG_JACOBI_KERNEL_NONE;
+  f->jacobi_resident = 0;
   if (f->prm.scheme == FG_SCHEME_LEXSOR) return launch_lexsor(f, num_iters, dt);
   PCtl* ctl = (PCtl*)f->pctl;
   PCtl* ectl = (PCtl*)f->ectl;

@@ -108,19 +108,25 @@ typedef struct fg_stats {
   double last_maxdiv;    /* max |div| seen by the last pressure sweep                     */
   int sweeps;            /* pressure sweeps executed (early exit included)                */
   int jacobi_kernel;     /* FG_JACOBI_KERNEL_*: the kernel of the last JACOBI-scheme solve */
-  int reserved[6];
+  int jacobi_resident;   /* nonzero: that solve ran as one resident launch instead (below) */
+  int reserved[5];
 } fg_stats;
 
-/* fg_stats.jacobi_kernel: which kernel ran the sweeps of the last step's main
+/* fg_stats.jacobi_kernel: the kernel for the sweeps of the last step's main
  * JACOBI-scheme solve (host-side record of what was enqueued or captured).
  * NONE for the other schemes and for batches; SWEEP is the per-launch kernel
  * that loads its tiles itself (early exit, depths below 8, grids without a
  * tensor map); TMA the per-launch kernel fed by the tensor memory
  * accelerator; DATAFLOW the one cooperative launch that runs every full
  * 8-sweep phase (fixed sweep counts of at least 16 on grids of at least one
- * tile per SM).  A fixed-count solve whose regions all fit the GPU at once
- * runs as one launch that keeps them in registers, with the same result; it
- * reports the value of its sweep count, depth and grid by the rules above. */
+ * tile per SM).
+ *
+ * fg_stats.jacobi_resident: a fixed-count solve whose regions all fit the GPU
+ * at once runs as one launch that keeps them in registers, with the same
+ * result.  jacobi_resident then says in which form: 4, 8 or 12 warps a region,
+ * one region an SM, or 16 for two regions of 8 warps an SM; jacobi_kernel names
+ * the kernel that the same solve takes without that launch, which did not run.
+ * With jacobi_resident 0 the kernel named by jacobi_kernel ran. */
 #define FG_JACOBI_KERNEL_NONE 0
 #define FG_JACOBI_KERNEL_SWEEP 1
 #define FG_JACOBI_KERNEL_TMA 2
