@@ -107,11 +107,16 @@ int alloc_dev(fg_fluid* f, float** p) {
 }
 
 // The resident Jacobi solves' buffers (zeroed: no packet carries a live tag).
-int alloc_jres(fg_fluid* f, size_t n) {
-  if (!n) return FG_OK;
-  if (dev_malloc(&f->jres, n) != cudaSuccess) return FG_ERR_NOMEM;
-  CK(f, cudaMemsetAsync(f->jres, 0, n, f->stream), "jres");
-  return FG_OK;
+// Without them the solves run in the other kernels.
+bool alloc_jres(fg_fluid* f, size_t n) {
+  if (!n) return false;
+  if (dev_malloc(&f->jres, n) == cudaSuccess &&
+      cudaMemsetAsync(f->jres, 0, n, f->stream) == cudaSuccess)
+    return true;
+  cudaFree(f->jres);
+  f->jres = nullptr;
+  cudaGetLastError();
+  return false;
 }
 
 // Copies the fields of `mask` between the device and their pinned mirrors.
@@ -522,7 +527,6 @@ int fg_create(int width, int height, float density, float h, const fg_params* pa
   if (dev_malloc((void**)&f->tile_done, sizeof(int) * ((size_t)jacobi_tile_count(f->NX, f->NY) + 1)) !=
       cudaSuccess)
     return bail(FG_ERR_NOMEM);
-  if ((rc = alloc_jres(f, jres_bytes_grid(f->NX, f->NY)))) return bail(rc);
   cudaMemsetAsync(f->pctl, 0, pctl_bytes(f->n_slots), f->stream);
   cudaMemsetAsync(f->ectl, 0, pctl_bytes(f->n_slots), f->stream);
   cudaMemsetAsync(f->dstats, 0, sizeof(DevStats), f->stream);
@@ -537,6 +541,8 @@ int fg_create(int width, int height, float density, float h, const fg_params* pa
     return bail(FG_ERR_NOMEM);
   if (host_malloc((void**)&f->stats_pinned, sizeof(DevStats)) != cudaSuccess)
     return bail(FG_ERR_NOMEM);
+  f->jres_form = jres_grid_form(f->NX, f->NY);
+  alloc_jres(f, jres_bytes_grid(f->NX, f->NY, f->jres_form));
   if (launch_noise_table(f) != cudaSuccess) return bail(FG_ERR_CUDA);
   f->masks_stale = true;
   if (flush(f) || cudaStreamSynchronize(f->stream) != cudaSuccess) return bail(FG_ERR_CUDA);
@@ -2016,7 +2022,7 @@ int batch_pack(fg_fluid* f) {
 // 6.2 us per 304 regions).  21 scenes of 64^2-512^2 with 309 regions: 8.7 us
 // per 8 sweeps and 252 us a step by launches, 295 in two equal groups of
 // 8-warp regions, 224 as planned here (two unequal ones of 12 warps).
-int batch_resident(fg_fluid* f, const std::vector<int>& jord) {
+void batch_resident(fg_fluid* f, const std::vector<int>& jord) {
   BatchGeom* b = f->batch;
   JresForm forms[3];
   jres_batch_forms(forms);
@@ -2070,7 +2076,7 @@ int batch_resident(fg_fluid* f, const std::vector<int>& jord) {
     }
     std::reverse(b->res_groups.begin(), b->res_groups.end());
   }
-  if (!b->res_cap) return FG_OK;
+  if (!b->res_cap) return;
   std::vector<JRegion> rg;
   for (int s : jord) {
     const BScene& sc = b->scenes[s];
@@ -2082,8 +2088,13 @@ int batch_resident(fg_fluid* f, const std::vector<int>& jord) {
                              span_own(ti, sc.g.NX, rows) | span_own(tj, sc.g.NY, kJacRegionCols) << 16,
                              ntx, ti > 0, ti < nty - 1, tj > 0, tj < ntx - 1});
   }
-  int rc = upload_table(f, &b->res_regions, rg);
-  return rc ? rc : alloc_jres(f, jres_bytes(0, b->res_cap, rows == 96 ? b->res_cap : 0));
+  if (upload_table(f, &b->res_regions, rg) ||
+      !alloc_jres(f, jres_bytes(b->res_cap, rows / kJacWarpRows))) {
+    cudaGetLastError();
+    f->last_error.clear();
+    b->res_groups.clear();
+    b->res_cap = 0;
+  }
 }
 
 int batch_check_member(fg_fluid* f, const fg_fluid* m, const fg_fluid* m0) {
@@ -2220,7 +2231,7 @@ int fg_batch_create(fg_fluid* const* scenes, int n, fg_fluid** out) {
     return bail(rc);
   b->n_border_tiles = (int)bt.size();
   b->n_jac_tiles = (int)jt.size();
-  if ((rc = batch_resident(f, jord))) return bail(rc);
+  batch_resident(f, jord);
   // Partial rows of the per-scene loss: one float pair per cell tile for the
   // block shape with the most tiles, plus the reserve partials_fit keeps.
   long long max_tiles = 0;

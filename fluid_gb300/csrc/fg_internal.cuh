@@ -251,7 +251,7 @@ static_assert(sizeof(BCell) == 64, "one 64-byte entry per block");
 // grid's edge, the one that reaches n owns up to n, the others own [t S +
 // halo, t S + R - halo).  A batch's Jacobi BTile holds the region's first
 // column and row in x and y and the owned window in pad.
-constexpr int kJacRegionRows = 64, kJacRegionCols = 128, kJacHalo = 8;
+constexpr int kJacRegionRows = 64, kJacRegionCols = 128, kJacHalo = 8, kJacWarpRows = 8;
 __host__ __device__ inline int span_count(int n, int R) {
   const int S = R - 2 * kJacHalo;
   return n <= R ? 1 : (n - R + S - 1) / S + 1;
@@ -362,6 +362,7 @@ struct fg_fluid {
   fg::DevStats* dstats = nullptr;
   void* pctl = nullptr;   // control block of the main Jacobi solve (k_pressure.cu PCtl)
   void* jres = nullptr;  // resident Jacobi solves: epochs and packets (or none)
+  int jres_form = -1;    // their form (k_pressure.cu), -1: none takes the grid
   int* tile_done = nullptr;  // dataflow Jacobi kernel: per-tile phase flags + item counter
   int stall_tile = -1;       // fault injection: a tile the dataflow kernel never publishes
   int jacobi_kernel = 0;     // FG_JACOBI_KERNEL_* of the last main solve (fg_stats)
@@ -501,10 +502,11 @@ void mg_free(fg_fluid* f);
 // buffer holding x.
 void init_jacobi_tma();
 int jacobi_tile_count(int NX, int NY);
-// Bytes of the resident solves' buffers for a grid, or for so many regions of
-// 4, 8 and 12 warps at once (0: none).
-size_t jres_bytes_grid(int NX, int NY);
-size_t jres_bytes(int regions4, int regions8, int regions12);
+// The form of a grid's resident solves (-1: none), the bytes of their buffers,
+// and of the buffers for so many regions of 4, 8 or 12 warps at once.
+int jres_grid_form(int NX, int NY);
+size_t jres_bytes_grid(int NX, int NY, int form);
+size_t jres_bytes(int regions, int warps);
 struct JresForm {
   int form, rows, cap;
   float us;

@@ -209,7 +209,7 @@ constexpr int RI = NWARP * RT;     // 64 region rows
 constexpr int OJ = RJ - 2 * TMAX;  // 112 owned columns
 constexpr int OI = RI - 2 * TMAX;  // 48 owned rows
 constexpr int TB_THREADS = 32 * NWARP;
-static_assert(RI == kJacRegionRows && RJ == kJacRegionCols && TMAX == kJacHalo,
+static_assert(RI == kJacRegionRows && RJ == kJacRegionCols && TMAX == kJacHalo && RT == kJacWarpRows,
               "Jacobi region geometry");
 
 // RINIT (first launch of the outer correction): instead of loading bw, the
@@ -2162,20 +2162,38 @@ static cudaError_t enqueue_jacobi(cudaStream_t st, const Grid& g, PCtl* ctl, con
 }
 
 // ---------------------------------------------------------------- resident solves
-// Regions of a grid for the 4- and 8-warp forms.
+// Regions of NW warps that cover a grid; 0 above the buffers' limit.
 static int res_regions(int NX, int NY, int NW) {
   const long long n = (long long)span_count(NX, NW * RT) * span_count(NY, RJ);
   return n > JRES_MAX_REGIONS ? 0 : (int)n;
 }
-// Bytes of a handle's resident-solve buffers (epochs, then packets); 0 when
-// no form takes the grid.
-size_t jres_bytes(int regions4, int regions8, int regions12) {
-  const size_t n = 2 * std::max(std::max((size_t)regions4 * JSlot<4>::N, (size_t)regions8 * JSlot<8>::N),
-                                (size_t)regions12 * JSlot<12>::N);
-  return n ? JRES_MAX_REGIONS * sizeof(unsigned) + n * sizeof(uint4) : 0;
+// Regions the current device holds at once in a form.
+static int res_capacity(const TmaDevice* dv, int form) {
+  return form == JRES_8X2 ? dv->res_blocks[form] : std::min(dv->sms, dv->res_blocks[form]);
 }
-size_t jres_bytes_grid(int NX, int NY) {
-  return jres_bytes(res_regions(NX, NY, 4), res_regions(NX, NY, 8), res_regions(NX, NY, 12));
+size_t jres_bytes(int regions, int warps) {
+  const size_t n = warps == 4 ? JSlot<4>::N : warps == 8 ? JSlot<8>::N : JSlot<12>::N;
+  return JRES_MAX_REGIONS * sizeof(unsigned) + 2 * n * (size_t)regions * sizeof(uint4);
+}
+
+// The smallest regions that get an SM each; else two 8-warp regions an SM.
+// Measured per 8 sweeps (us), against the launches or the dataflow kernel
+// they replace: 4 warps 128^2 2.2 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
+// 2.9 (4.4), 800^2 3.0 (6.6); 12 warps 1024x768 4.2 (7.4), 1200x800 4.1
+// (9.4); 8 warps twice 1200^2 6.0 (11.0).  A larger form where a smaller
+// one fits is slower (512x256: 2.4, 3.1, 4.2, 3.9).  (Outside any capture.)
+int jres_grid_form(int NX, int NY) {
+  init_jacobi_tma();
+  const TmaDevice* dv = tma_device();
+  if (!dv || !dv->ready.load()) return -1;
+  for (int form = JRES_4; form <= JRES_8X2; ++form) {
+    const int n = res_regions(NX, NY, res_warps(form));
+    if (n > 0 && n <= res_capacity(dv, form)) return form;
+  }
+  return -1;
+}
+size_t jres_bytes_grid(int NX, int NY, int form) {
+  return form < 0 ? 0 : jres_bytes(res_regions(NX, NY, res_warps(form)), res_warps(form));
 }
 
 // The forms a batch may be solved in: rows of a region, regions at once, and
@@ -2188,8 +2206,7 @@ void jres_batch_forms(JresForm (&out)[3]) {
   const int form[3] = {JRES_8, JRES_12, JRES_8X2};
   const float us[3] = {3.0f, 4.1f, 6.0f};
   for (int k = 0; k < 3; ++k) {
-    int cap = !ok ? 0 : form[k] == JRES_8X2 ? d->res_blocks[JRES_8X2]
-                                            : std::min(d->sms, d->res_blocks[form[k]]);
+    const int cap = ok ? res_capacity(d, form[k]) : 0;
     out[k] = JresForm{form[k], res_warps(form[k]) * RT, std::min(cap, JRES_MAX_REGIONS), us[k]};
   }
 }
@@ -2210,29 +2227,14 @@ static cudaError_t launch_res(cudaStream_t st, const JResArgs& a, bool o1, bool 
 
 // A fixed-count solve of one grid from x = 0 into x as one resident launch.
 // What fg_stats.jacobi_resident reports of it, or 0 (nothing launched) where
-// the grid's regions do not fit the GPU at once.
+// the grid has no form or its buffers could not be had.
 static int launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, const float* BW,
                              float om1, int iters, int T, int stall) {
   if (!f->jres) return 0;
   const TmaDevice* dv = tma_ready(f->stream);
   if (!dv) return 0;
-  int n[4];
-  for (int k = 0; k < 4; ++k) n[k] = res_regions(f->NX, f->NY, res_warps(k));
-  // 4 warps a region while each gets an SM of its own, else 8, one or two to
-  // an SM.
-  // The smallest regions that get an SM each; else two 8-warp regions an SM.
-  // Measured per 8 sweeps (us), against the launches or the dataflow kernel
-  // they replace: 4 warps 128^2 2.2 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
-  // 2.9 (4.4), 800^2 3.0 (6.6); 12 warps 1024x768 4.2 (7.4), 1200x800 4.1
-  // (9.4); 8 warps twice 1200^2 6.0 (11.0).  A larger form where a smaller
-  // one fits is slower (512x256: 2.4, 3.1, 4.2, 3.9).
-  int form = JRES_4;
-  while (form <= JRES_8X2 &&
-         !(n[form] > 0 && n[form] <= (form == JRES_8X2 ? dv->res_blocks[form]
-                                                       : std::min(dv->sms, dv->res_blocks[form]))))
-    ++form;
-  if (form > JRES_8X2) return 0;
-  const int nw = res_warps(form);
+  const int form = f->jres_form, nw = res_warps(form), n = res_regions(f->NX, f->NY, nw);
+  if (n > res_capacity(dv, form)) return 0;  // (another context than the handle's first)
   JResArgs a = {};
   a.x = x;
   a.W = W;
@@ -2249,7 +2251,7 @@ static int launch_jacobi_res(fg_fluid* f, PCtl* ctl, float* x, const float* W, c
   a.last_launch = (iters + T - 1) / T - 1;
   a.err = &f->dstats->timeout;
   a.stall = stall;
-  if (launch_res(f->stream, a, om1 == 0.0f, false, form, n[form]) != cudaSuccess) {
+  if (launch_res(f->stream, a, om1 == 0.0f, false, form, n) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
