@@ -2176,19 +2176,28 @@ size_t jres_bytes(int regions, int warps) {
   return JRES_MAX_REGIONS * sizeof(unsigned) + 2 * n * (size_t)regions * sizeof(uint4);
 }
 
-// The smallest regions that get an SM each; else two 8-warp regions an SM.
-// Measured per 8 sweeps (us), against the launches or the dataflow kernel
-// they replace: 4 warps 128^2 2.2 (3.5), 512x256 2.4 (3.5); 8 warps 512^2
-// 2.9 (4.4), 800^2 3.0 (6.6); 12 warps 1024x768 4.2 (7.4), 1200x800 4.1
-// (9.4); 8 warps twice 1200^2 6.0 (11.0).  A larger form where a smaller
-// one fits is slower (512x256: 2.4, 3.1, 4.2, 3.9).  (Outside any capture.)
+// The smallest regions that get an SM each, but 4 warps only for up to 16
+// regions; else two 8-warp regions an SM.  Measured per 8 sweeps (us), against
+// the launches or the dataflow kernel they replace: 4 warps 128^2 2.2 (3.5);
+// 8 warps 512x256 3.1 (3.5), 512^2 2.9 (4.4), 800^2 3.0 (6.6); 12 warps
+// 1024x768 4.2 (7.4), 1200x800 4.1 (9.4); 8 warps twice 1200^2 6.0 (11.0).  A
+// larger form where a smaller one fits is slower.  4 warps take a solve alone
+// on the GPU further (512x256: 2.4), but own half of the cells they sweep and
+// hold more SMs while they wait, at the cost of every other stream's work:
+// a step of many handles in turn (us; 4 warps, 8 warps, the launches) 64 of
+// 256^2 673, 585, 648; 32 of 360^2 695, 570, 567; 32 of 512x256 836, 659, 694;
+// 64 of 192^2 439, 397, 432.  Up to 128^2 (16 regions) they cost nothing there:
+// 64 of 128^2 386, 403, 406; alone 58 us a step against 60 and 68.
+// (Outside any capture.)
+constexpr int kRes4Regions = 16;
 int jres_grid_form(int NX, int NY) {
   init_jacobi_tma();
   const TmaDevice* dv = tma_device();
   if (!dv || !dv->ready.load()) return -1;
   for (int form = JRES_4; form <= JRES_8X2; ++form) {
     const int n = res_regions(NX, NY, res_warps(form));
-    if (n > 0 && n <= res_capacity(dv, form)) return form;
+    const int most = form == JRES_4 ? kRes4Regions : JRES_MAX_REGIONS;
+    if (n > 0 && n <= std::min(most, res_capacity(dv, form))) return form;
   }
   return -1;
 }

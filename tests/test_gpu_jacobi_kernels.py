@@ -47,7 +47,8 @@ def solve(gpu, w, h, iters, **kw):
 
 
 @pytest.mark.parametrize("w,h,iters,tb,form", [
-    (62, 62, 24, 8, 4), (700, 500, 23, 8, 8), (1024, 768, 17, 5, 12), (400, 2700, 12, 4, 12),
+    (62, 62, 24, 8, 4), (128, 128, 24, 8, 4), (270, 126, 24, 8, 4),
+    (271, 126, 24, 8, 8), (192, 192, 24, 8, 8), (512, 256, 24, 8, 8), (700, 500, 23, 8, 8), (1024, 768, 17, 5, 12), (400, 2700, 12, 4, 12),
     (1200, 800, 24, 8, 12), (1200, 1250, 16, 8, 16),
 ])
 def test_resident_forms(gpu, w, h, iters, tb, form):
