@@ -96,6 +96,27 @@ int bind(fg_fluid* f) {
   return FG_OK;
 }
 
+// For batches and recorded rollouts, whose steps no fg_get_stats follows: the
+// mark of a bounded wait that gave up is read where a call waits for the
+// stream anyway.  timeout_fetch before that wait, timeout_check after it.
+int timeout_fetch(fg_fluid* f) {
+  if (!f->timeout_read)
+    CK(f, cudaMemcpyAsync(&f->stats_pinned->timeout, &f->dstats->timeout, sizeof(int),
+                          cudaMemcpyDeviceToHost, f->stream), "timeout");
+  return FG_OK;
+}
+int timeout_check(fg_fluid* f) {
+  f->timeout_read = true;
+  return f->stats_pinned->timeout
+             ? fail(f, FG_ERR_TIMEOUT, "a device-side wait of an earlier step gave up")
+             : FG_OK;
+}
+int timeout_clear(fg_fluid* f) {
+  f->timeout_read = false;
+  CK(f, cudaMemsetAsync(&f->dstats->timeout, 0, sizeof(int), f->stream), "timeout");
+  return FG_OK;
+}
+
 size_t field_bytes(const fg_fluid* f) { return sizeof(float) * (size_t)f->NX * f->P; }
 
 int alloc_dev(fg_fluid* f, float** p) {
@@ -377,7 +398,7 @@ int enqueue_step(fg_fluid* f, float dt) {
   f->n_marks = 0;
   mark(f, "start");
   CK(f, launch_apply_sources(f), "sources");
-  CK(f, launch_clear_stats(f), "clear stats");
+  CK(f, launch_clear_stats(f, f->batch != nullptr), "clear stats");
   if (p.scheme == FG_SCHEME_LEXSOR || multigrid(f))
     CK(f, cudaMemsetAsync(f->d[FG_P], 0, field_bytes(f), f->stream), "fill p");
   if (p.viscosity_diffusion > 0.0f) CK(f, launch_viscosity(f, dt), "viscosity");
@@ -814,6 +835,7 @@ static int simulate_enqueue(fg_fluid* f, float dt);
 
 int fg_simulate(fg_fluid* f, float dt) {
   if (!f) return FG_ERR_INVALID;
+  f->timeout_read = false;
   f->async_defer_ok = true;
   int rc = simulate_enqueue(f, dt);
   f->async_defer_ok = false;
@@ -1518,7 +1540,7 @@ int enqueue_step_record(fg_fluid* f, float dt, const float* fu, const float* fv,
   if (replay) {
     ep = launch_grad_replay(f, dt, phi, fuse);
   } else {
-    ep = launch_clear_stats(f);
+    ep = launch_clear_stats(f, true);
     if (ep == cudaSuccess) rc = enqueue_pressure(f, p.num_iters, dt, fuse);
     if (ep == cudaSuccess && !rc) ep = launch_store_phi(f, phi);
   }
@@ -1718,6 +1740,8 @@ int fg_tape_begin(fg_fluid* f, int max_steps, int every) {
     CK(f, cudaMemsetAsync(t->aux, 0, fb, f->stream), "tape");
   }
   if (t->version != f->params_version) tape_clear_graphs(t);
+  // (A batch whose state a wait spoiled stays marked until it is gathered.)
+  if (!f->batch && (rc = timeout_clear(f))) return rc;
   t->active = true;
   t->max_steps = max_steps;
   t->every = every;
@@ -1766,6 +1790,7 @@ int fg_step_forward(fg_fluid* f, float dt, const float* force_u, const float* fo
     CK(f, launch_mask_forces(f, force_at(f, k, 0), force_at(f, k, 1)), "forces");
   }
   invalidate(f, kStepFields);
+  f->timeout_read = false;
   {
     const float* fu = force_u ? force_at(f, k, 0) : nullptr;
     const float* fv = force_u ? force_at(f, k, 1) : nullptr;
@@ -1819,8 +1844,10 @@ int fg_tape_seed_smoke_l2(fg_fluid* f, const float* target, double* loss) {
   if (loss) {
     CK(f, cudaMemcpyAsync(f->scalar_pinned, slot, sizeof(double), cudaMemcpyDeviceToHost,
                           f->stream), "loss");
+    if ((rc = timeout_fetch(f))) return rc;
     CK(f, cudaStreamSynchronize(f->stream), "loss sync");
     memcpy(loss, f->scalar_pinned, sizeof(double));
+    return timeout_check(f);
   }
   return FG_OK;
 }
@@ -1844,6 +1871,7 @@ int fg_step_adjoint(fg_fluid* f, float* grad_force_u, float* grad_force_v) {
   float* rec[kTapeFields];
   for (int q = 0; q < kTapeFields; ++q)
     rec[q] = rec_at(f, k - s * t->every) + (size_t)q * field_elems(f);
+  f->timeout_read = false;
   const void* ptrs[4] = {rec[0], nullptr, nullptr, nullptr};
   rc = run_graphed(f, kGraphAdjoint, t->dts[k], ptrs, [&] {
     cudaError_t e = launch_step_adjoint(f, t->dts[k], rec);
@@ -1873,8 +1901,9 @@ int fg_tape_grad(fg_fluid* f, float* dU, float* dV, float* dM, float* dNU, float
                       fg_fluid::A_NU, fg_fluid::A_NV, fg_fluid::A_NM};
   for (int k = 0; k < 6; ++k)
     if (out[k] && (rc = get_field(f, out[k], f->adj[src[k]]))) return rc;
+  if ((rc = timeout_fetch(f))) return rc;
   CK(f, cudaStreamSynchronize(f->stream), "grad sync");
-  return FG_OK;
+  return timeout_check(f);
 }
 
 int fg_tape_steps(const fg_fluid* f, int* forward, int* reversed) {
@@ -2299,6 +2328,7 @@ int fg_batch_gather(fg_fluid* f) {
   int rc = bind(f);
   if (rc) return rc;
   if (f->tape && f->tape->active) return fail(f, FG_ERR_INVALID, "a recorded rollout is open");
+  if ((rc = timeout_clear(f))) return rc;
   return batch_pack(f);
 }
 
@@ -2307,7 +2337,10 @@ int fg_batch_scatter(fg_fluid* f) {
   int rc = bind(f);
   if (rc) return rc;
   const fg::BatchGeom* b = f->batch;
+  // (The members keep their state when the batch's is spoiled.)
+  if ((rc = timeout_fetch(f))) return rc;
   CK(f, cudaStreamSynchronize(f->stream), "batch sync");
+  if ((rc = timeout_check(f))) return rc;
   SliceCopies c = {f, true, {}};
   for (int s = 0; s < b->n; ++s) {
     fg_fluid* m = b->members[s];
@@ -2346,7 +2379,9 @@ int fg_batch_seed_smoke_l2(fg_fluid* f, const float* const* targets, double* los
   if (losses) {
     CK(f, cudaMemcpyAsync(losses, b->losses, sizeof(double) * b->n, cudaMemcpyDefault, f->stream),
        "losses");
+    if ((rc = timeout_fetch(f))) return rc;
     CK(f, cudaStreamSynchronize(f->stream), "losses");
+    return timeout_check(f);
   }
   return FG_OK;
 }
@@ -2369,8 +2404,9 @@ int fg_batch_grad(fg_fluid* f, int s, float* dU, float* dV, float* dM) {
     if (out[k])
       CK(f, cudaMemcpy2DAsync(out[k], hp, f->adj[src[k]] + sc.off, dp, hp, sc.g.NX,
                               cudaMemcpyDefault, f->stream), "grad");
+  if ((rc = timeout_fetch(f))) return rc;
   CK(f, cudaStreamSynchronize(f->stream), "grad sync");
-  return FG_OK;
+  return timeout_check(f);
 }
 
 // Picks the per-cell thread-block shape and the Jacobi sweeps per launch
@@ -2384,6 +2420,9 @@ int fg_batch_autotune(fg_fluid* f, float dt, int reps, int* tb_depth, int* block
   int rc = bind(f);
   if (rc) return rc;
   if (f->tape && f->tape->active) return fail(f, FG_ERR_INVALID, "a recorded rollout is open");
+  if ((rc = timeout_fetch(f))) return rc;
+  CK(f, cudaStreamSynchronize(f->stream), "autotune");
+  if ((rc = timeout_check(f))) return rc;
   const auto& shapes = kBatchShapes;
   static const int depths[] = {4, 6, 8};
   size_t fb = field_bytes(f);
@@ -2433,8 +2472,11 @@ int fg_batch_autotune(fg_fluid* f, float dt, int reps, int* tb_depth, int* block
   f->prm.tb_depth = depths[bd];
   f->params_version++;
   clear_graphs(f);
+  // (The state is restored: a wait that gave up spoiled the timed steps only.)
+  if (!rc) rc = timeout_fetch(f);
   cudaStreamSynchronize(f->stream);
   cudaFree(saved);
+  if (!rc && (rc = timeout_check(f))) timeout_clear(f);
   if (rc) return rc;
   if (tb_depth) *tb_depth = depths[bd];
   if (block_x) *block_x = shapes[bb][0];
@@ -2718,7 +2760,6 @@ int fg_debug_stall_tile(fg_fluid* f, int tile) {
     set_noalloc_stall(tile);
     return FG_OK;
   }
-  if (is_batch(f)) return batch_unsupported(f);
   int rc = flush(f);
   if (rc) return rc;
   f->stall_tile = tile < 0 ? -1 : tile;

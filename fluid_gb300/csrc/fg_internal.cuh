@@ -212,7 +212,8 @@ struct DevStats {  // device-side accumulation target (finalised per step)
   double smoke_mass;
   double last_maxdiv;
   int sweeps;
-  int timeout;  // 1: a bounded device-side wait of the step gave up
+  int timeout;  // 1: a bounded device-side wait gave up (of the step; of a
+                // batch's steps since its state was set, of a recorded rollout)
   int ticket;   // finished blocks of the reduction that is running (grid_row)
 };
 
@@ -454,6 +455,7 @@ struct fg_fluid {
   int n_marks = 0;
   float* scalar_pinned = nullptr;  // small D2H results
   fg::DevStats* stats_pinned = nullptr;
+  bool timeout_read = false;  // stats_pinned->timeout is the device's (nothing enqueued since)
   std::string last_error;
 
   // CUDA graphs of the step, keyed by the state pointers and dt.
@@ -541,7 +543,7 @@ cudaError_t launch_step_adjoint(fg_fluid* f, float dt, float* const* tape);
 cudaError_t launch_loss_seed(fg_fluid* f, const float* target, double* dev_loss);
 // k_diag.cu
 cudaError_t launch_div_stats(fg_fluid* f);
-cudaError_t launch_clear_stats(fg_fluid* f);
+cudaError_t launch_clear_stats(fg_fluid* f, bool keep_timeout = false);
 cudaError_t launch_max_divergence(fg_fluid* f, float* dev_out);
 cudaError_t launch_view(fg_fluid* f, int kind, float* dev_minmax);  // 0 vorticity, 1 magnitude
 cudaError_t launch_field_minmax(fg_fluid* f, int field, float* dev_minmax);

@@ -3,6 +3,7 @@
 // block partials, so repeated runs give identical numbers.
 #include <algorithm>
 #include <cfloat>
+#include <cstddef>
 
 #include "fg_internal.cuh"
 #include "fg_reduce.cuh"
@@ -155,8 +156,11 @@ __global__ void k_sample_velocity(const float* __restrict__ U, const float* __re
 
 }  // namespace
 
-cudaError_t launch_clear_stats(fg_fluid* f) {
-  return cudaMemsetAsync(f->dstats, 0, sizeof(DevStats), f->stream);
+cudaError_t launch_clear_stats(fg_fluid* f, bool keep_timeout) {
+  // (A batch's and a recorded rollout's mark of a wait that gave up outlives
+  // the step: it is read once for many steps.  The ticket is 0 at rest.)
+  return cudaMemsetAsync(f->dstats, 0, keep_timeout ? offsetof(DevStats, timeout) : sizeof(DevStats),
+                         f->stream);
 }
 
 // Blocks of a reduction over the cells' tiles, 0 when their rows do not fit.

@@ -2290,7 +2290,7 @@ static cudaError_t jacobi_solve_batch(fg_fluid* f, PCtl* ctl, const float* bw, f
     a.ctl = ctl;
     a.last_launch = L - 1;
     a.err = &f->dstats->timeout;
-    a.stall = -1;
+    a.stall = f->stall_tile;  // (that region of every group)
     unsigned* epochs = static_cast<unsigned*>(f->jres);
     uint4* pkts = reinterpret_cast<uint4*>(epochs + JRES_MAX_REGIONS);
     bool ok = true;

@@ -641,6 +641,12 @@ class Batch:
     def profile(self, on=True):
         self._check(self._L.fg_profile_enable(self._h, int(bool(on))), "fg_profile_enable")
 
+    def debug_stall_tile(self, tile):
+        """Fault injection: region `tile` of every resident launch sends nothing,
+        so bounded waits give up and scatter(), seed_smoke_l2() and grad() raise
+        FG_ERR_TIMEOUT (tile < 0 disarms)."""
+        self._check(self._L.fg_debug_stall_tile(self._h, int(tile)), "fg_debug_stall_tile")
+
     # ------------------------------------------------------------ recorded rollouts
     def tape_begin(self, max_steps, every=8):
         self._check(self._L.fg_tape_begin(self._h, int(max_steps), int(every)), "fg_tape_begin")

@@ -325,6 +325,10 @@ int fg_project_noalloc_status(void* stream);
  * fields and a potential; one interval of 13 recorded fields; 6 fields per
  * checkpoint) stay allocated for the next rollout until fg_destroy.
  *
+ * fg_tape_seed_smoke_l2 (with a loss), fg_tape_grad and, between them,
+ * fg_get_stats return FG_ERR_TIMEOUT when a bounded device-side wait of any
+ * step since fg_tape_begin gave up; what they wrote is then not to be used.
+ *
  * All fields (forces, seeds, target, gradients) use the mirrors' layout
  * (NumX * NumY floats, index i*NumY + j) in host or device memory.  Adjoint
  * advection scatters with FP32 atomics: gradients reproduce to about 1e-6
@@ -364,6 +368,11 @@ int fg_tape_end(fg_fluid* f);
  * kernels and Jacobi sweeps per launch (tb_depth) on `reps` steps of this
  * batch from its current state (restored afterwards), keeps the fastest and
  * reports it.  The choice changes no result bit.
+ *
+ * When a bounded device-side wait of a step gave up, fg_batch_seed_smoke_l2
+ * (with losses), fg_batch_grad and fg_batch_scatter return FG_ERR_TIMEOUT, and
+ * fg_batch_scatter leaves the members as they are, until fg_batch_gather sets
+ * the batch's state again.
  *
  * Entry points that address one scene's cells, mirrors or views return
  * FG_ERR_UNSUPPORTED on a batch handle. */
@@ -419,7 +428,9 @@ const char* fg_last_error(const fg_fluid* f);
  * t of the handle's solves, so the tiles that read it wait until their
  * bounded waits (about a second) give up; the step's fg_get_stats returns
  * FG_ERR_TIMEOUT; on smaller grids region t of the resident solve sends
- * nothing to its neighbours.  With the reference's serial scheme, strip t of 32 rows
+ * nothing to its neighbours, and on a batch region t of every launch of its
+ * resident solve (a solve that runs as launches of 8 sweeps has no such wait).
+ * With the reference's serial scheme, strip t of 32 rows
  * sends nothing to the next one, with the same result.  t < 0 disarms.
  * Changes the handle's captured graphs.
  * fg_debug_stall_tile(NULL, t): in later fg_project_noalloc calls, the
