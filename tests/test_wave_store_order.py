@@ -5,6 +5,7 @@ the stores of different lanes may become visible in any order, each lane's own
 in the order it made them.  The model makes one sweep over a strip of 32 rows
 chunk by chunk, applies a chunk's stores in random interleavings of the lanes
 and compares the ring's U with the serial loop."""
+import os
 import random
 
 import numpy as np
@@ -83,3 +84,10 @@ def test_the_model_sees_two_lanes_storing_one_word():
     want = serial(U, V, 1.7)
     got = sweep(U, V, 1.7, random.Random(0), set(range(LANES)))
     assert not np.array_equal(got[0], want[0])
+
+
+def test_the_kernel_stores_the_last_lanes_east_face_only():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    text = open(os.path.join(root, "fluid_gb300", "csrc", "k_lexsor.cu")).read()
+    stores = [x.strip() for x in text.splitlines() if "F(at0 + RB) = en" in x]
+    assert stores == ["if (lane == 31) F(at0 + RB) = en;"]
