@@ -559,7 +559,6 @@ cudaError_t launch_particles_advect(fg_fluid* f, float dt, int n_upper, const fl
 // red) colormap between dev_minmax[0..1] into an NX x NY RGBA8 image.
 cudaError_t launch_render(fg_fluid* f, const float* field, const float* dev_minmax, int diverging,
                           uint32_t* img);
-// Device-to-device copy of an NX x NY field between two row pitches.
 // One copy between rows x width floats stored linearly (16-byte aligned) and
 // the same rows at a pitch (rows * width < 2^31); a launch takes a list.
 struct CopyItem {
@@ -573,19 +572,8 @@ struct CopyList {
   bool full() const { return n == 120; }
 };
 cudaError_t launch_copy_list(fg_fluid* f, const CopyList& l, bool to_linear);
+// Device-to-device copy of an NX x NY field between two row pitches.
 cudaError_t launch_repitch(fg_fluid* f, float* dst, const float* src, int dpitch, int spitch);
-
-// Grid of the reduction kernels: 32 x 8 threads per block over (j, i), at
-// most about 1200 blocks; each block strides down the rows, so the single-
-// block combine of the block partials stays short.
-inline dim3 reduce_grid(const fg_fluid* f) {
-  int gx = (f->NY + 31) / 32;
-  int gy = (f->NX + 7) / 8;
-  int cap = 1216 / gx;
-  if (cap < 1) cap = 1;
-  if (gy > cap) gy = cap;
-  return dim3(gx, gy);
-}
 
 // True when a reduction with `ns` partials per block over `nb` blocks, plus
 // its two-level combine, fits the partials buffer without reaching the

@@ -33,9 +33,9 @@ inline dim3 cell_grid(const fg_fluid* f) {
 // below (smaller i), never back: a strip needs nothing of the strip above
 // within a group of G sweeps.  The strip's fields live in shared memory, a
 // ring of WV_W columns that a loader warp fills and a storer warp drains, so a
-// step costs the shuffle, the arithmetic and its own instructions (45 of them,
-// 50 ns), where a wavefront through L2 with a barrier per anti-diagonal paid
-// a memory round trip and the barrier (2.4 us, on one block or eight).
+// step costs the shuffle, the arithmetic and its own instructions, where a
+// wavefront through L2 with a barrier per anti-diagonal paid a memory round
+// trip and the barrier (2.4 us, on one block or eight).
 // Chunks of 16 columns: a chunk's waits, packets and report take about 240
 // cycles, so 8 columns measured slower in a strip (20x2046, one sweep: 163
 // against 147 us) and 8 columns with 16 sweeps a block, whose ring then has
@@ -49,12 +49,17 @@ inline dim3 cell_grid(const fg_fluid* f) {
 // unfinished task can always proceed.
 //
 // Bound by the serial chain: NX + NY steps and a packet's flight per strip.
-// Measured on a GB300 against the wavefront through L2 that it replaced (one
-// block, an 8-block cluster or a grid barrier per anti-diagonal), whole
-// passes from the host: the app's 300x251 jet with 8 sweeps and the early
-// exit 1382 -> 178 us, two steps of a 128x128 jet with 40 sweeps 2890 -> 380
-// us, a 1024x768 box with BFECC 4439 -> 423 us, a 512x512 box with 8
-// reference V-cycles 45.5 -> 3.3 ms; 200 sweeps alone at 2048^2 2.35 ms.
+// Measured on a GB300: one sweep takes 53 ns a column along a strip and 3.7 us
+// a strip of 32 rows (47 steps and 1.2 us of flight), a group of 8 sweeps 78 ns
+// and 4.5 us; every further group 26 us at 300x251, 20 at 30x30.  The chain
+// leaves most of the issue slots empty (32 % used on the SMs that have a
+// block; per issue 1.95 warps wait on a fixed latency, 0.95 on shared memory).
+// Against the wavefront through L2 that it replaced (one block, an 8-block
+// cluster or a grid barrier per anti-diagonal), whole passes from the host: the
+// app's 300x251 jet with 8 sweeps and the early exit 1386 -> 162 us, two steps
+// of a 128x128 jet with 40 sweeps 2893 -> 365 us, a 1024x768 box with BFECC
+// 4464 -> 413 us, a 512x512 box with 8 reference V-cycles 45.7 -> 3.3 ms; 200
+// sweeps alone at 2048^2 2.34 ms.
 constexpr int WV_G = 8;            // sweeps per group (compute warps of a block)
 constexpr int WV_C = 16;           // columns per chunk
 constexpr int WV_W = 256;          // ring columns
@@ -95,8 +100,10 @@ struct WaveCtl {
 // copies the scratch fields into the state, or, when the serial loop would
 // have stopped before the last sweep, runs exactly its sweeps on the state
 // (sweeps up to that one are the same in both passes, so the result and the
-// count are the serial loop's).
-enum { WV_WLAIN = 0, WV_SPECULATE = 1, WV_FINISH = 2 };
+// count are the serial loop's).  The copying launch takes 5.5 us at 128x128, 8
+// at 300x251, 10 at 1024x768, 61 at 2048^2, beside 61, 97, 254 and 528 us of a
+// makeIncompressible with 8 sweeps.
+enum { WV_PLAIN = 0, WV_SPECULATE = 1, WV_FINISH = 2 };
 
 struct WaveArgs {
   // SOR: U, V, p.  Coarse Gauss-Seidel: the solution (zero before group 0)
@@ -238,7 +245,7 @@ __device__ __forceinline__ void wv_fill_coef(WaveCoef* lut) {
 // Markstein's correction (IBM J. Res. Dev. 34, 1990), whose remainder is
 // exact for every float and these n; the remainder is taken as n q - x so
 // that a zero keeps its sign, and an infinity keeps its first quotient.
-// Equal to the division for all 2^32 floats and each n (checked on the host).
+// Equal to the division for all 2^32 floats and each n (tests/test_div_count.py).
 __device__ __forceinline__ float div_count(float x, float n, float r) {
   float q = x * r;
   const float e = __fmaf_rn(n, q, -x);
@@ -1293,7 +1300,7 @@ static void lexsor_solve(fg_fluid* f, int iters, float relax0, float relax1, flo
     pass(WV_SPECULATE);
     pass(WV_FINISH);
   } else {
-    pass(WV_WLAIN);
+    pass(WV_PLAIN);
   }
 }
 
@@ -1321,7 +1328,7 @@ static void launch_mg_coarse(fg_fluid* f, const int* stop, int cNX, int cNY, int
   a.P = cP;
   a.iters = 40;
   a.relax0 = 1.6f;
-  a.mode = WV_WLAIN;
+  a.mode = WV_PLAIN;
   a.stop = stop;
   a.stall = -1;
   wave_launch(f, a, true, 0, 40);

@@ -61,16 +61,16 @@ struct WTab {
   float w[5];  // w[s] = (omega * damping) / s
 };
 
-// Per cell: b = -div, w = om / s and bw = w * b on active cells, all 0
-// elsewhere (ring included); phi = 0 when `zero_phi` (a solve with no sweeps
-// reads it directly).
-// U, V use the grid pitch g.P, the solver arrays the pitch Ps.
 // U + Fu at face u (the force field of a recorded step, null otherwise).
 __device__ __forceinline__ float with_force(const float* __restrict__ U,
                                             const float* __restrict__ F, int u) {
   return F ? U[u] + F[u] : U[u];
 }
 
+// Per cell: b = -div, w = om / s and bw = w * b on active cells, all 0
+// elsewhere (ring included); phi = 0 when `zero_phi` (a solve with no sweeps
+// reads it directly).
+// U, V use the grid pitch g.P, the solver arrays the pitch Ps.
 __device__ __forceinline__ void setup_cell_p(int i, int j, const float* __restrict__ U,
                                              const float* __restrict__ V, float* __restrict__ phi,
                                              float* __restrict__ rhs, float* __restrict__ W,
@@ -562,9 +562,6 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, unsigned parity) {
     if (mbar_wait_bounded(bar, parity)) return;
 }
 
-// One sweep of a tile in registers, with the arithmetic of jacobi_tile;
-// buf alternates between consecutive sweeps (the row exchange is double
-// buffered, one barrier per sweep).
 // The barrier of a tile's NW warps: the block's, or (OWN) a named one of
 // theirs alone in a block with other warps.
 template <int NW, bool OWN>
@@ -574,6 +571,9 @@ __device__ __forceinline__ void tile_barrier() {
   else
     __syncthreads();
 }
+// One sweep of a tile in registers, with the arithmetic of jacobi_tile;
+// buf alternates between consecutive sweeps (the row exchange is double
+// buffered, one barrier per sweep).
 template <bool OMEGA1, int NW = NWARP, bool OWN = false>
 __device__ __forceinline__ void tile_sweep(float (&x)[RT][JT], const float (&w)[RT][JT],
                                            const float (&bw)[RT][JT], float om1,
@@ -923,10 +923,11 @@ __device__ __forceinline__ bool flow_ready_warp(const int* done, int ph, int t, 
 // other three: 12 x 32 x 152 + 4 x 32 x 40 = 63,488 of the 512 x 128 = 65,536
 // the block is launched with.)  Bound by the sweeps' instructions: of an item's
 // 8,000 cycles 5,430 are sweeps, 1,250 the fill from shared memory and 1,000
-// the stores; 48 MB of boxes a phase at 2048 x 2048 stay in L2.  Per 8 sweeps
-// (us), against two 8-warp blocks an SM whose own threads waited for boxes and
-// flags: 2048 x 2048 13.5 (16.9), 1300 x 1300 8.5 (10.7), 1500 x 1100 8.2
-// (10.5), 1700 x 1700 9.6 (12.5), 3000 x 2500 26.3 (32.2).  A fence in every
+// the stores; 48 MB of boxes a phase at 2048 x 2048 stay in L2.  Each further 8
+// sweeps (us), against two 8-warp blocks an SM whose own threads waited for
+// boxes and flags: 2048 x 2048 13.6 (16.9), 1300 x 1300 8.5 (10.7), 1500 x 1100
+// 8.2 (10.5), 1700 x 1700 9.7 (12.5), 3000 x 2500 26.9 (32.2); with the
+// launch's ends a phase of 25 at 2048 x 2048 takes 14.0.  A fence in every
 // poll of the flags and the timer read on every turn held the phi copy back
 // 5,000 cycles an item (15.0 at 2048 x 2048).
 constexpr int FW = 12, FI = FW * RT, FO = FI - 2 * TMAX, FLOW_FLOATS = FI * RJ;
@@ -1172,9 +1173,12 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
 // other kernels, the same bits.
 //
 // For grids whose regions fit the GPU at once.  Bound by the sweeps' own
-// latency (1.35 us per 8 sweeps for 4 warps, each alone on its scheduler:
-// 190 instructions a warp and sweep at half a one per cycle) and the packets'
-// flight (0.7 us).  With 8-warp regions the registers decide: 128 a thread
+// latency (1.35 us per 8 sweeps for 4 warps, each alone on its scheduler) and
+// the packets' flight (0.7 us): 196 warp instructions a warp and sweep, the
+// exchange included, in 30 % of the issue slots of the SMs that hold a region
+// of 4 warps (128^2, 40 sweeps), 189 in 46 % with 8 warps (512x256, 100
+// sweeps); per issue 0.8-0.9 warps wait on the packets, 0.2-0.4 on the sweeps'
+// barrier.  With 8-warp regions the registers decide: 128 a thread
 // (two blocks an SM) spill and take 3.9 us, 190 take 3.0.  Barriers split
 // into arrive and wait around the inner rows measured slower (2.2 against
 // 1.35 us without exchange), as did the boundary rows computed first (1.41).
@@ -1656,13 +1660,14 @@ struct StoreDivP {
 // The gradient subtract and its fused statistics, 4 columns of a row a thread
 // at a time: fields move in 16-byte pieces (rows start on 128 bytes; a piece
 // past the last column reads pitch padding, which nothing uses).  At most
-// kGradBlocks blocks walk the grid, three an SM (76 registers a thread), so
-// the reduction at the end of a block is paid once per block and its rows are
-// few enough to combine in the same launch.  Plain cells take 150 operations
-// of the 240 the flag-by-flag form takes.  With the combining (us; before:
-// one column of 8 rows a thread and a second launch): 128 x 128 9.5 (11.7 +
-// 4.9), 512 x 256 9.4 (11.4 + 5.3), 1500 x 1100 25 (27.7 + 5.9), 2048 x 2048
-// 41.6 (56 + 7.1).  One piece a thread in 4109 blocks: 66; two rows a piece 82.
+// kGradBlocks blocks walk the grid, three an SM (held to 80 registers a thread,
+// which spills 36 bytes, 104 when a step is recorded), so the reduction at the
+// end of a block is paid once per block and its rows are few enough to combine
+// in the same launch.  Plain cells take 150 operations of the 240 the
+// flag-by-flag form takes.  With the combining (us; before: one column of 8
+// rows a thread and a second launch): 128 x 128 9.1 (11.7 + 4.9), 512 x 256 9.3
+// (11.4 + 5.3), 1500 x 1100 24 (27.7 + 5.9), 2048 x 2048 42 (56 + 7.1).  One
+// piece a thread in 4109 blocks: 66; two rows a piece 82.
 constexpr int kGradBlocks = 3 * 152;
 // REC: a recorded step (force fields, the faces before turbulence kept).
 template <bool REC>
