@@ -57,6 +57,7 @@ def test_resident_forms(gpu, w, h, iters, tb, form):
 
 @pytest.mark.parametrize("w,h,iters,kw,kernel", [
     (9000, 260, 24, {}, "DATAFLOW"), (600, 4000, 40, {}, "DATAFLOW"),  # 339 and 288 tiles
+    (30000, 100, 16, {}, "DATAFLOW"),                 # one tile column
     (900, 2700, 12, dict(tb_depth=4), "SWEEP"),       # depths below 8
     (9000, 260, 8, {}, "TMA"),                        # one full launch
     (333, 222, 40, dict(early_exit=True, tolerance=0.0), "SWEEP"),
