@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
       // that the warps that wait for it leave too; then the copies still
       // landing.  (Left incomplete, the phase held the block for 9 s more.)
       if (!whole) {
-        s_lost = flight_n;
+        atomicMin(&s_lost, flight_n);
         mbar_arrive(&full);
       }
       mbar_drain(&full, flight_n & 1);
@@ -1086,12 +1086,13 @@ __global__ void __launch_bounds__(FLOW_THREADS, 1)
       // A warp whose wait gave up sweeps whatever the buffer holds, as item 0,
       // and a warp that has seen the end meets the same barriers before it
       // leaves: whatever each warp saw, all of them pass TMAX barriers here, so
-      // none is left waiting in one.  s_lost names the item given up: set
-      // before the first barrier, it is seen by all after the last, and a
-      // faster warp that gives up the next item does not make a slower one
-      // leave before that item's barriers.
+      // none is left waiting in one.  s_lost names the first item given up:
+      // set before the first barrier, it is seen by all after the last, and a
+      // faster warp (or the thirteenth) that gives up the next item neither
+      // makes a slower one leave before that item's barriers nor hides that
+      // this one is lost.
       const int item = landed ? s_item : 0;
-      if (!landed) s_lost = n;
+      if (!landed) atomicMin(&s_lost, n);
       if (item >= total) {
 #pragma unroll 1
         for (int sw = 0; sw < TMAX; ++sw) tile_barrier<FW, true>();

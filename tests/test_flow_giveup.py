@@ -12,10 +12,11 @@ WARPS, SWEEPS = 12, 8
 
 
 class Block:
-    def __init__(self, items, rng, agree=True, named=True):
+    def __init__(self, items, rng, agree=True, named=True, least=True):
         """agree: a warp that has seen the end passes the barriers too; named:
-        the mark of a warp that gave up says on which item."""
-        self.items, self.rng, self.agree, self.named = items, rng, agree, named
+        the mark of a wait that gave up says on which item; least: a later
+        item's mark does not replace an earlier one's."""
+        self.items, self.rng, self.agree, self.named, self.least = items, rng, agree, named, least
         self.full = self.empty = self.stored = 0  # completed phases
         self.n_empty = self.n_stored = 0          # arrivals of the present phase
         self.item, self.lost = 0, None
@@ -27,6 +28,10 @@ class Block:
 
     def gives_up(self):
         return self.impatient and self.clock >= self.when and self.rng.random() < 0.3
+
+    def lose(self, n):
+        n = n if self.named else -1
+        self.lost = n if self.lost is None or not self.least else min(self.lost, n)
 
     def wait(self, done):
         while not done():
@@ -50,6 +55,13 @@ class Block:
                 if not ok:
                     return
             self.item = n
+            if n < self.items:
+                ready = self.clock + self.rng.randrange(60)  # (the neighbours)
+                ok = yield from self.wait(lambda: self.clock >= ready)
+                if not ok:  # the item is closed without its last box
+                    self.lose(n)
+                    self.full += 1
+                    return
             yield
             self.full += 1  # (the copies land, or the end is told)
             if n:
@@ -65,7 +77,7 @@ class Block:
             if not self.agree and not landed:
                 item = self.item
             if not landed:
-                self.lost = n if self.named else -1
+                self.lose(n)
             if item >= self.items:
                 if self.agree:
                     for _ in range(SWEEPS):
@@ -112,14 +124,22 @@ class Block:
         return True
 
 
+def holds(items, seed, **kw):
+    try:
+        return Block(items, random.Random(seed), **kw).run()
+    except AssertionError:
+        return False
+
+
 @pytest.mark.parametrize("items", [1, 2, 5])
 def test_no_warp_is_left_in_a_barrier(items):
-    for seed in range(150):
+    for seed in range(300):
         assert Block(items, random.Random(seed)).run(), seed
 
 
 def test_the_model_sees_the_warps_disagree():
     """A warp that leaves without the barriers; a mark that a slower warp takes
-    for its own item's."""
-    assert not all(Block(2, random.Random(seed), agree=False).run() for seed in range(1000))
-    assert not all(Block(5, random.Random(seed), named=False).run() for seed in range(400))
+    for its own item's; a later item's mark in place of an earlier one's."""
+    assert not all(holds(1, seed, agree=False) for seed in range(1500))
+    assert not all(holds(5, seed, named=False) for seed in range(100))
+    assert not all(holds(3, seed, least=False) for seed in range(400))
